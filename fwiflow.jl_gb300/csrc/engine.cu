@@ -981,7 +981,7 @@ int plan_groups(fwigb_ctx* ctx, bool adj, std::vector<std::vector<int>>& groups)
   }
   const size_t ldz = ctx->geo.ldz;
   ctx->fields_stride = 18 * ldz * nx_max;
-  ctx->grads_stride = (ctx->illum ? 4 : 3) * ldz * nx_max;
+  ctx->grads_stride = (ctx->illum ? 6 : 5) * ldz * nx_max;
   ctx->store_stride = adj ? static_cast<size_t>(ctx->nSteps_max) * 5 * ring_max : 0;
   const size_t per_member = (ctx->fields_stride + ctx->grads_stride + ctx->store_stride) * sizeof(float);
   size_t budget = ctx->mem_budget;
@@ -995,6 +995,8 @@ int plan_groups(fwigb_ctx* ctx, bool adj, std::vector<std::vector<int>>& groups)
   int cap = static_cast<int>(std::min<size_t>(budget / std::max<size_t>(per_member, 1), 1u << 16));
   if (ctx->max_batch > 0) cap = std::min(cap, ctx->max_batch);
   cap = std::min(cap, static_cast<int>(ctx->plans.size()));
+  // A budget that holds one shot but for two of its five imaging sums is taken as one shot's.
+  if (cap < 1 && budget + 2 * ldz * nx_max * sizeof(float) >= per_member) cap = 1;
   if (cap < 1) {
     ctx->err = "one shot's wavefields and boundary store do not fit in device memory";
     return FWIGB_ERR_OOM;
@@ -1097,7 +1099,7 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
     sh.gstf = ctx->shot_gstf.as<float>(pl.gstf_off);
     sl.st = StoreD{ctx->store_stride ? ctx->g_store.as<float>(k * ctx->store_stride) : nullptr};
     float* gb = ctx->g_grads.as<float>(k * ctx->grads_stride);
-    sl.gr = Grads{gb, gb + n, gb + 2 * n, ctx->illum ? gb + 3 * n : nullptr};
+    sl.gr = Grads{gb, gb + n, gb + 2 * n, gb + 3 * n, gb + 4 * n, ctx->illum ? gb + 5 * n : nullptr};
     sl.nSteps = pl.nSteps;
     sl.x_off = pl.x_off;
     for (int t = 0; t < 3; ++t) {

@@ -140,10 +140,14 @@ struct StoreD {
   float* base;  // [step][5 fields: szz, sxz, sxx, vz, vx][ring_len]
 };
 
+// A shot's sums over time of the imaging terms ("Imaging" in kernels.cu), from
+// which k_reduce_grads forms its lambda, mu and rho gradients.
 struct Grads {
   float* lam;
   float* mu;
-  float* den;
+  float* tau;
+  float* va;
+  float* vb;
   float* illum;  // source illumination sum_t (vz^2 + vx^2), or null when not accumulated
 };
 
@@ -158,7 +162,7 @@ struct ShotSlot {
   CpmlD c;
   ShotD sh;
   StoreD st;
-  Grads gr;  // this shot's gradient on its sub-grid
+  Grads gr;  // this shot's imaging sums on its sub-grid
   int nSteps;
   int x_off;
 };

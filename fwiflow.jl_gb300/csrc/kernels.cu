@@ -12,11 +12,10 @@
 //                ring restore + velocity adjoint                 (step it)
 //            C : residual injection + stress adjoint + source gradient (it-1)
 //                + reverse velocity + rho imaging + velocity ring restore
-// The reference scatters the mu and rho kernels with atomicAdd
-// (el_stress.cu:113-124, el_velocity.cu:101-110); here every cell gathers the
-// contributions of its neighbours, recomputing their derivative terms from the
-// read-only fields of the same sweep, so there are no atomics and the sums are
-// deterministic.
+// The reference scatters the mu and rho kernels with atomicAdd in every step
+// (el_stress.cu:113-124, el_velocity.cu:101-110); here the sweeps sum each
+// cell's own time-dependent factor and one kernel per call gathers them (see
+// "Imaging" below), so there are no atomics and the sums are deterministic.
 #include "fwigb_kernels.h"
 
 #include <cudaTypedefs.h>
@@ -468,8 +467,22 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 }
 
 // ---------------------------------------------------------------------------
-// B: add_source(-) + el_stress(isFor=false) with the lambda / mu kernels +
-// to_bnd(stress) + el_velocity_adj. Staged: vz, vx, szz_a, sxx_a, sxz_a.
+// Imaging. The reference adds to the lambda, mu and rho kernels at every step
+// (el_stress.cu:110-124, el_velocity.cu:98-110), the mu kernel through the
+// chain rule of the 2x2 harmonic average and the rho kernel through that of
+// the two buoyancies. The chain rules do not depend on time, so the sweeps
+// sum over time only what does, at the cell itself,
+//   gr.lam += (szz_a + sxx_a)(dvz/dz + dvx/dx)     gr.tau += sxz_a (dvx/dz + dvz/dx)
+//   gr.mu  += szz_a dvz/dz + sxx_a dvx/dx          gr.va += vz_a (dszz/dz + dsxz/dx)
+//                                                  gr.vb += vx_a (dsxz/dz + dsxx/dx)
+// and k_reduce_grads applies them once per call. Gathering them in every step
+// took the neighbours' strains and divergences again, and the media values of
+// the chain rules; summing two values more per cell instead takes less: B 254
+// -> 234 us and C 257 -> 246 us a step of 24 aperture-windowed 608-row shots,
+// 16.5 -> 14.3 us and 15.4 -> 14.0 us on one 608 x 1600 shot.
+
+// B: add_source(-) + el_stress(isFor=false) with the sums of the lambda / mu
+// kernels + to_bnd(stress) + el_velocity_adj. Staged: vz, vx, szz_a, sxx_a, sxz_a.
 template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
@@ -477,20 +490,16 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
   SWEEP_EDGE_CELL(BOXZ, R)
   SWEEP_SMEM(BOXZ)
   const Grads& gr = S.gr;
-  float p_lam[R], p_l2m[R], p_amu[R], p_w[R], p_h[R];
-  float p_szz[R], p_sxx[R], p_sxz[R], p_gl[R], p_gm[R], p_vza[R], p_vxa[R];
+  float p_lam[R], p_l2m[R], p_amu[R];
+  float p_szz[R], p_sxx[R], p_sxz[R], p_vza[R], p_vxa[R];
   ldrows<R>(m.lam + i, rows_in, p_lam);
   ldrows<R>(m.l2m + i, rows_in, p_l2m);
   ldrows<R>(m.aveMu + i, rows_in, p_amu);
-  ldrows<R>(m.muw + i, rows_in, p_w);
-  ldrows<R>(m.hs + i, rows_in, p_h);
   pdl_wait();
   SWEEP_TMA(5, BOXZ)
   ldrows<R>(f.szz + i, rows_in, p_szz);
   ldrows<R>(f.sxx + i, rows_in, p_sxx);
   ldrows<R>(f.sxz + i, rows_in, p_sxz);
-  ldrows<R>(gr.lam + i, rows_in, p_gl);
-  ldrows<R>(gr.mu + i, rows_in, p_gm);
   ldrows<R>(f.vz_a + i, rows_in, p_vza);
   ldrows<R>(f.vx_a + i, rows_in, p_vxa);
   if (!live) return;
@@ -507,12 +516,10 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
   auto cell = [&](const int r, const int z, const size_t i, const int b) {
   float szz = p_szz[r], sxx = p_sxx[r], sxz = p_sxz[r];
   const float lam = p_lam[r], l2m = p_l2m[r], amu = p_amu[r];
-  const float gl = p_gl[r], gm = p_gm[r], w = p_w[r], h = p_h[r];
   const float va_z = p_vza[r], va_x = p_vxa[r];
   const bool interior = in_box(z, x, g.zi0, g.zi1, g.xi0, g.xi1);
   const bool src = (z == sh.src_z && x == sh.src_x);
   const int k = ring_index(g, z, x);
-  float e_own = 0.0f, gmu_own = 0.0f;
   if (interior || src || k >= 0) {
     if (src) {
       szz -= sh.src_szz_r[it];
@@ -521,15 +528,14 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
     if (interior) {
       const float dvz_dz = sdm(s_vz, b, 1, g.rdz);
       const float dvx_dx = sdm(s_vx, b, BOXZ, g.rdx);
-      const float dvx_dz = sdp(s_vx, b, 1, g.rdz);
-      const float dvz_dx = sdp(s_vz, b, BOXZ, g.rdx);
+      const float e = sdp(s_vx, b, 1, g.rdz) + sdp(s_vz, b, BOXZ, g.rdx);  // dvx_dz + dvz_dx
       szz -= (l2m * dvz_dz + lam * dvx_dx) * dt;
       sxx -= (lam * dvz_dz + l2m * dvx_dx) * dt;
-      e_own = dvx_dz + dvz_dx;
-      sxz -= amu * e_own * dt;
+      sxz -= amu * e * dt;
       const float sa = s_szz_a[b], xa = s_sxx_a[b];
-      gr.lam[i] = gl + -(sa + xa) * (dvz_dz + dvx_dx) * dt * kMega;
-      gmu_own = (-2.0f * sa * dvz_dz * dt - 2.0f * xa * dvx_dx * dt) * kMega;
+      gr.lam[i] += (sa + xa) * (dvz_dz + dvx_dx);
+      gr.mu[i] += sa * dvz_dz + xa * dvx_dx;
+      gr.tau[i] += s_sxz_a[b] * e;
     }
     if (k >= 0) {
       const float* p = st.base + static_cast<size_t>(it) * 5 * g.ring_len + k;
@@ -540,34 +546,6 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
     f.szz[i] = szz;
     f.sxx[i] = sxx;
     f.sxz[i] = sxz;
-  }
-  // mu kernel: own term plus the harmonic-average chain rule of the 2x2 blocks
-  // whose top-left corner is (z,x), (z-1,x), (z,x-1), (z-1,x-1), with the
-  // guards of el_stress.cu:118-123 (the x guard of :120 is always true).
-  if (in_box(z, x, g.zi0, g.zi1, g.xi0, g.xi1 + 1)) {
-    float acc = gm + gmu_own;
-    const float* __restrict__ hs = m.hs;
-    if (x <= g.xi1) {
-      if (h != 0.0f) acc += w * (-s_sxz_a[b] * e_own * dt * h);
-      if (z - 1 >= g.zi0) {
-        const float hj = hs[i - 1];
-        const int bj = b - 1;
-        if (hj != 0.0f)
-          acc += w * (-s_sxz_a[bj] * (sdp(s_vx, bj, 1, g.rdz) + sdp(s_vz, bj, BOXZ, g.rdx)) * dt * hj);
-      }
-    }
-    if (x - 1 >= g.xi0) {
-      const float hj = hs[i - ldz];
-      const int bj = b - BOXZ;
-      if (hj != 0.0f) acc += w * (-s_sxz_a[bj] * (sdp(s_vx, bj, 1, g.rdz) + sdp(s_vz, bj, BOXZ, g.rdx)) * dt * hj);
-      if (z - 1 >= g.zi0 && x <= g.xi1) {
-        const float h2 = hs[i - ldz - 1];
-        const int b2 = b - BOXZ - 1;
-        if (h2 != 0.0f)
-          acc += w * (-s_sxz_a[b2] * (sdp(s_vx, b2, 1, g.rdz) + sdp(s_vz, b2, BOXZ, g.rdx)) * dt * h2);
-      }
-    }
-    gr.mu[i] = acc;
   }
   // el_velocity_adj (el_velocity_adj.cu:57-102); the psi memory terms are
   // read only where their CPML coefficient is non-zero.
@@ -616,7 +594,7 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
 
 // C: res_injection (utilities.cu:569-580) + el_stress_adj (el_stress_adj.cu:53-97)
 //    + source_grad (utilities.cu:582-593) + el_velocity(isFor=false) with the
-//    density kernel (el_velocity.cu:84-117) + to_bnd(velocity).
+//    sums of the density kernel (el_velocity.cu:84-117) + to_bnd(velocity).
 //    Staged: vz_a, vx_a, szz, sxx, sxz.
 template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
@@ -626,7 +604,7 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   SWEEP_SMEM(BOXZ)
   const Grads& gr = S.gr;
   const int rev = S.nSteps - 2 - j >= 1;
-  float p_bA[R], p_bB[R], p_amu[R], p_lam[R], p_l2m[R], p_sa[R], p_xa[R], p_za[R], p_vz[R], p_vx[R], p_gd[R];
+  float p_bA[R], p_bB[R], p_amu[R], p_lam[R], p_l2m[R], p_sa[R], p_xa[R], p_za[R], p_vz[R], p_vx[R];
   ldrows<R>(m.bycA + i, rows_in, p_bA);
   ldrows<R>(m.bycB + i, rows_in, p_bB);
   ldrows<R>(m.aveMu + i, rows_in, p_amu);
@@ -639,7 +617,6 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   ldrows<R>(f.sxz_a + i, rows_in, p_za);
   ldrows<R>(f.vz + i, rev ? rows_in : 0, p_vz);
   ldrows<R>(f.vx + i, rev ? rows_in : 0, p_vx);
-  ldrows<R>(gr.den + i, rev ? rows_in : 0, p_gd);
   if (!live) return;
   const ShotD& sh = S.sh;
   const StoreD& st = S.st;
@@ -658,7 +635,7 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   auto cell = [&](const int r, const int z, const size_t i, const int b) {
   float sa = p_sa[r], xa = p_xa[r], za = p_za[r];
   const float bA = p_bA[r], bB = p_bB[r], amu = p_amu[r], lam = p_lam[r], l2m = p_l2m[r];
-  float vz = p_vz[r], vx = p_vx[r], gd = p_gd[r];
+  float vz = p_vz[r], vx = p_vx[r];
   const bool dom = in_box(z, x, g.zs0, g.zs1, g.xs0, g.xs1);
   bool injected = false;
   if (rec_tile && z >= sh.rbz0 && z <= sh.rbz1) {
@@ -709,15 +686,14 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   if (!rev) return;
   if (z == sh.src_z && x == sh.src_x) sh.gstf[it - 1] = -(sa + 3.0f * xa) * dt;
   const bool interior = in_box(z, x, g.zi0, g.zi1, g.xi0, g.xi1);
-  float tA = 0.0f, tB = 0.0f;
   const int k = ring_index(g, z, x);
   if (interior) {
     const float ea = sdp(s_szz, b, 1, g.rdz) + sdm(s_sxz, b, BOXZ, g.rdx);  // dszz_dz + dsxz_dx
     const float eb = sdm(s_sxz, b, 1, g.rdz) + sdp(s_sxx, b, BOXZ, g.rdx);  // dsxz_dz + dsxx_dx
     vz -= ea * bA * dt;
     vx -= eb * bB * dt;
-    tA = -s_vz_a[b] * ea * dt * (-bA * bA * 0.5f);
-    tB = -s_vx_a[b] * eb * dt * (-bB * bB * 0.5f);
+    gr.va[i] += s_vz_a[b] * ea;
+    gr.vb[i] += s_vx_a[b] * eb;
   }
   if (k >= 0) {
     const float* p = st.base + static_cast<size_t>(it - 1) * 5 * g.ring_len + k;
@@ -727,28 +703,6 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   if (interior || k >= 0) {
     f.vz[i] = vz;
     f.vx[i] = vx;
-  }
-  // rho kernel gather: (z,x) receives A and B of itself, A of (z-1,x) and B of
-  // (z,x-1) (el_velocity.cu:101-110; the x guard of :109 is always true).
-  if (in_box(z, x, g.zi0, g.zi1, g.xi0, g.xi1 + 1)) {
-    float acc = gd;
-    if (x <= g.xi1) {
-      acc += tA;
-      acc += tB;
-      if (z - 1 >= g.zi0) {
-        const int bj = b - 1;
-        const float bAj = m.bycA[i - 1];
-        const float ea = sdp(s_szz, bj, 1, g.rdz) + sdm(s_sxz, bj, BOXZ, g.rdx);
-        acc += -s_vz_a[bj] * ea * dt * (-bAj * bAj * 0.5f);
-      }
-    }
-    if (x - 1 >= g.xi0) {
-      const int bj = b - BOXZ;
-      const float bBj = m.bycB[i - ldz];
-      const float eb = sdm(s_sxz, bj, 1, g.rdz) + sdp(s_sxx, bj, BOXZ, g.rdx);
-      acc += -s_vx_a[bj] * eb * dt * (-bBj * bBj * 0.5f);
-    }
-    gr.den[i] = acc;
   }
   };
 #pragma unroll
@@ -1000,13 +954,67 @@ __device__ __forceinline__ void str(float* p, const float (&v)[R]) {
   }
 }
 
+// Differences of a staged array at the thread's R depths: along z (Dm, Dp) and
+// along x. With two depths (b even) the float2 at b + o (o even) holds both
+// depths' samples at offset o, so a z stencil of both takes the pairs at
+// b - 2, b, b + 2 and an x stencil those at b + k BOXZ.
+template <int R>
+__device__ __forceinline__ void dmz(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdm(a, b, 1, r);
+  } else {
+    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
+    o[0] = dd(c.x, m.y, c.y, m.x, r);
+    o[1] = dd(c.y, c.x, p.x, m.y, r);
+  }
+}
+template <int R>
+__device__ __forceinline__ void dpz(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdp(a, b, 1, r);
+  } else {
+    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
+    o[0] = dd(c.y, c.x, p.x, m.y, r);
+    o[1] = dd(p.x, c.y, p.y, c.x, r);
+  }
+}
+template <int R, int BOXZ>
+__device__ __forceinline__ void dmx(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdm(a, b, BOXZ, r);
+  } else {
+    const float2 c = ld2(a + b), m = ld2(a + b - BOXZ), p = ld2(a + b + BOXZ), m2 = ld2(a + b - 2 * BOXZ);
+    o[0] = dd(c.x, m.x, p.x, m2.x, r);
+    o[1] = dd(c.y, m.y, p.y, m2.y, r);
+  }
+}
+template <int R, int BOXZ>
+__device__ __forceinline__ void dpx(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdp(a, b, BOXZ, r);
+  } else {
+    const float2 c = ld2(a + b), p = ld2(a + b + BOXZ), p2 = ld2(a + b + 2 * BOXZ), m = ld2(a + b - BOXZ);
+    o[0] = dd(p.x, c.x, p2.x, m.x, r);
+    o[1] = dd(p.y, c.y, p2.y, m.y, r);
+  }
+}
+template <int R>
+__device__ __forceinline__ void own(const float* a, int b, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = a[b];
+  } else {
+    const float2 c = ld2(a + b);
+    o[0] = c.x;
+    o[1] = c.y;
+  }
+}
+
 // Backward fast bodies, R adjacent depths per thread (tiles of 32 R rows):
 // the own-cell operands of all R depths are loaded before the staged tiles
-// are awaited; the depths are then computed in turn (the stencil samples
-// two depths share are read once after unrolling).
-// MID: a mid tile (no CPML cell): the reverse stress update and the lambda
-// term only at cells of the reverse-time interior, the ring's stresses of
-// step it restored, and the mu gathers with the guards of the edge form.
+// are awaited.
+// MID: a mid tile (no CPML cell): the reverse stress update and the imaging
+// sums only at cells of the reverse-time interior, and the ring's stresses of
+// step it restored.
 template <int TX, int K, int R, bool MID>
 __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
@@ -1015,16 +1023,11 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
   SWEEP_SMEM(BOXZ)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
-  const float dt = g.dt;
-  float szz[R], sxx[R], sxz[R], lam[R], l2m[R], amu[R], gl[R], gm[R], w[R], h[R], va_z[R], va_x[R], hx[R];
   const uint64_t pol = media_policy();
+  float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R], gl[R], gm[R], gt[R], va_z[R], va_x[R];
   ldrm<R>(m.lam + i, lam, pol);
   ldrm<R>(m.l2m + i, l2m, pol);
   ldrm<R>(m.aveMu + i, amu, pol);
-  ldrm<R>(m.muw + i, w, pol);
-  ldrm<R>(m.hs + i, h, pol);
-  ldrm<R>(m.hs + i - ldz, hx, pol);
-  const float hz0 = ldm(m.hs + i - 1, pol), hzx0 = ldm(m.hs + i - ldz - 1, pol);
   pdl_wait();
   SWEEP_TMA(5, BOXZ)
   ldr<R>(f.szz + i, szz);
@@ -1032,144 +1035,82 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
   ldr<R>(f.sxz + i, sxz);
   ldr<R>(gr.lam + i, gl);
   ldr<R>(gr.mu + i, gm);
+  ldr<R>(gr.tau + i, gt);
   ldr<R>(f.vz_a + i, va_z);
   ldr<R>(f.vx_a + i, va_x);
-  // Fast one-row tiles share the strain e = dvx_dz + dvz_dx of the mu
-  // gathers: each thread computes its own cell's, warp 0 the tile's x0 - 1
-  // column and z0 - 1 row, and the gathers read their neighbours' from
-  // shared memory (s_e: columns x0 - 1 .. x0 + TX - 1, depths z0 - 1 ..
-  // z0 + 31, stride 33) instead of recomputing them. Same operations per value.
-  constexpr bool kShare = !MID && R == 1;
-  const bool ok = stage_wait(&bar, err);
-  if constexpr (kShare) {
-    if (!__syncthreads_and(ok)) return;  // (a uniform exit: the block meets a barrier below)
-  } else {
-    if (!ok) return;
-  }
+  if (!stage_wait(&bar, err)) return;
   const float* s_vz = sm;
   const float* s_vx = sm + N;
   const float* s_szz_a = sm + 2 * N;
   const float* s_sxx_a = sm + 3 * N;
   const float* s_sxz_a = sm + 4 * N;
-  float e_me = 0.0f, e_up = 0.0f, e_left = 0.0f, e_upleft = 0.0f;
-  if constexpr (kShare) {
-    float* s_e = sm + 5 * N;
-    const int ty = threadIdx.y, tx = threadIdx.x;
-    e_me = sdp(s_vx, b, 1, g.rdz) + sdp(s_vz, b, BOXZ, g.rdx);
-    s_e[(ty + 1) * 33 + tx + 1] = e_me;
-    if (ty == 0) {
-      const int bl = b - BOXZ;  // (z, x0 - 1)
-      s_e[tx + 1] = sdp(s_vx, bl, 1, g.rdz) + sdp(s_vz, bl, BOXZ, g.rdx);
-      if (tx <= TX) {
-        const int bu = (tx + 1) * BOXZ + 3;  // (z0 - 1, x0 - 1 + tx)
-        s_e[tx * 33] = sdp(s_vx, bu, 1, g.rdz) + sdp(s_vz, bu, BOXZ, g.rdx);
-      }
-    }
-    __syncthreads();
-    e_up = s_e[(ty + 1) * 33 + tx];
-    e_left = s_e[ty * 33 + tx + 1];
-    e_upleft = s_e[ty * 33 + tx];
-  }
-  float o_gl[R], o_gm[R], o_szz[R], o_sxx[R], o_sxz[R], o_vza[R], o_vxa[R];
+  const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
+  {
+    float dvz_dz[R], dvx_dx[R], e[R], t[R], sa[R], xa[R], za[R];
+    dmz<R>(s_vz, b, rdz, dvz_dz);
+    dmx<R, BOXZ>(s_vx, b, rdx, dvx_dx);
+    dpz<R>(s_vx, b, rdz, e);
+    dpx<R, BOXZ>(s_vz, b, rdx, t);
+    own<R>(s_szz_a, b, sa);
+    own<R>(s_sxx_a, b, xa);
+    own<R>(s_sxz_a, b, za);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int bb = b + r;
-    const int zr = z + r;
-    const float hz = r == 0 ? hz0 : h[r - 1];     // hs at (z-1, x)
-    const float hzx = r == 0 ? hzx0 : hx[r - 1];  // hs at (z-1, x-1)
-    if (special && zr == sh.src_z && x == sh.src_x) {
-      szz[r] -= sh.src_szz_r[it];
-      sxx[r] -= sh.src_sxx_r[it];
-    }
-    const bool inter = !MID || in_box(zr, x, g.zi0, g.zi1, g.xi0, g.xi1);
-    const float dvz_dz = sdm(s_vz, bb, 1, g.rdz);
-    const float dvx_dx = sdm(s_vx, bb, BOXZ, g.rdx);
-    float e_own = 0.0f, gmu_own = 0.0f;
-    if (inter) {
-      o_szz[r] = szz[r] - (l2m[r] * dvz_dz + lam[r] * dvx_dx) * dt;
-      o_sxx[r] = sxx[r] - (lam[r] * dvz_dz + l2m[r] * dvx_dx) * dt;
-      if constexpr (kShare)
-        e_own = e_me;
-      else
-        e_own = sdp(s_vx, bb, 1, g.rdz) + sdp(s_vz, bb, BOXZ, g.rdx);  // dvx_dz + dvz_dx
-      o_sxz[r] = sxz[r] - amu[r] * e_own * dt;
-      const float sa = s_szz_a[bb], xa = s_sxx_a[bb];
-      o_gl[r] = gl[r] + -(sa + xa) * (dvz_dz + dvx_dx) * dt * kMega;
-      gmu_own = (-2.0f * sa * dvz_dz * dt - 2.0f * xa * dvx_dx * dt) * kMega;
-    } else {
-      o_szz[r] = szz[r];
-      o_sxx[r] = sxx[r];
-      o_sxz[r] = sxz[r];
-      o_gl[r] = gl[r];
-    }
-    if constexpr (MID) {  // to_bnd of the stresses (the ring's values replace the update)
-      const int k = ring_index(g, zr, x);
-      if (k >= 0) {
-        const float* p = S.st.base + static_cast<size_t>(it) * 5 * g.ring_len + k;
-        o_szz[r] = p[0];
-        o_sxz[r] = p[g.ring_len];
-        o_sxx[r] = p[2 * g.ring_len];
+    for (int r = 0; r < R; ++r) {
+      e[r] += t[r];  // dvx_dz + dvz_dx
+      if (special && z + r == sh.src_z && x == sh.src_x) {
+        szz[r] -= sh.src_szz_r[it];
+        sxx[r] -= sh.src_sxx_r[it];
       }
-    }
-    // mu kernel: own term and the three neighbouring 2x2 blocks; in a fast
-    // tile all guards hold, in a mid tile they are those of el_stress.cu:118-123.
-    if (!MID || in_box(zr, x, g.zi0, g.zi1, g.xi0, g.xi1 + 1)) {
-      const bool own_col = !MID || x <= g.xi1;
-      const bool up = !MID || zr - 1 >= g.zi0;
-      const bool left = !MID || x - 1 >= g.xi0;
-      float acc = gm[r] + gmu_own;
-      if (own_col) {
-        if (h[r] != 0.0f) acc += w[r] * (-s_sxz_a[bb] * e_own * dt * h[r]);
-        if (up && hz != 0.0f) {
-          const int bj = bb - 1;
-          const float e = kShare ? e_up : sdp(s_vx, bj, 1, g.rdz) + sdp(s_vz, bj, BOXZ, g.rdx);
-          acc += w[r] * (-s_sxz_a[bj] * e * dt * hz);
+      if (!MID || in_box(z + r, x, g.zi0, g.zi1, g.xi0, g.xi1)) {
+        szz[r] -= (l2m[r] * dvz_dz[r] + lam[r] * dvx_dx[r]) * dt;
+        sxx[r] -= (lam[r] * dvz_dz[r] + l2m[r] * dvx_dx[r]) * dt;
+        sxz[r] -= amu[r] * e[r] * dt;
+        gl[r] += (sa[r] + xa[r]) * (dvz_dz[r] + dvx_dx[r]);
+        gm[r] += sa[r] * dvz_dz[r] + xa[r] * dvx_dx[r];
+        gt[r] += za[r] * e[r];
+      }
+      if constexpr (MID) {  // to_bnd of the stresses (the ring's values replace the update)
+        const int q = ring_index(g, z + r, x);
+        if (q >= 0) {
+          const float* p = S.st.base + static_cast<size_t>(it) * 5 * g.ring_len + q;
+          szz[r] = p[0];
+          sxz[r] = p[g.ring_len];
+          sxx[r] = p[2 * g.ring_len];
         }
       }
-      if (left) {
-        if (hx[r] != 0.0f) {
-          const int bj = bb - BOXZ;
-          const float e = kShare ? e_left : sdp(s_vx, bj, 1, g.rdz) + sdp(s_vz, bj, BOXZ, g.rdx);
-          acc += w[r] * (-s_sxz_a[bj] * e * dt * hx[r]);
-        }
-        if (up && own_col && hzx != 0.0f) {
-          const int b2 = bb - BOXZ - 1;
-          const float e = kShare ? e_upleft : sdp(s_vx, b2, 1, g.rdz) + sdp(s_vz, b2, BOXZ, g.rdx);
-          acc += w[r] * (-s_sxz_a[b2] * e * dt * hzx);
-        }
-      }
-      o_gm[r] = acc;
-    } else {
-      o_gm[r] = gm[r];
-    }
-    // el_velocity_adj without the psi memory terms.
-    {
-      const float dszz_dx = -sdp(s_szz_a, bb, BOXZ, g.rdx);
-      const float dsxx_dx = -sdp(s_sxx_a, bb, BOXZ, g.rdx);
-      const float dsxz_dz = -sdm(s_sxz_a, bb, 1, g.rdz);
-      o_vxa[r] = va_x[r] + (lam[r] * dszz_dx * dt + l2m[r] * dsxx_dx * dt + amu[r] * dsxz_dz * dt);
-    }
-    {
-      const float dszz_dz = -sdp(s_szz_a, bb, 1, g.rdz);
-      const float dsxx_dz = -sdp(s_sxx_a, bb, 1, g.rdz);
-      const float dsxz_dx = -sdm(s_sxz_a, bb, BOXZ, g.rdx);
-      o_vza[r] = va_z[r] + (l2m[r] * dszz_dz * dt + lam[r] * dsxx_dz * dt + amu[r] * dsxz_dx * dt);
     }
   }
-  str<R>(gr.lam + i, o_gl);
-  str<R>(f.szz + i, o_szz);
-  str<R>(f.sxx + i, o_sxx);
-  str<R>(f.sxz + i, o_sxz);
-  str<R>(gr.mu + i, o_gm);
-  str<R>(f.vx_a + i, o_vxa);
-  str<R>(f.vz_a + i, o_vza);
+  str<R>(f.szz + i, szz);
+  str<R>(f.sxx + i, sxx);
+  str<R>(f.sxz + i, sxz);
+  str<R>(gr.lam + i, gl);
+  str<R>(gr.mu + i, gm);
+  str<R>(gr.tau + i, gt);
+  // el_velocity_adj without the psi memory terms.
+  {
+    float d1[R], d2[R], d3[R];
+    dpx<R, BOXZ>(s_szz_a, b, rdx, d1);
+    dpx<R, BOXZ>(s_sxx_a, b, rdx, d2);
+    dmz<R>(s_sxz_a, b, rdz, d3);
+#pragma unroll
+    for (int r = 0; r < R; ++r) va_x[r] -= (lam[r] * d1[r] + l2m[r] * d2[r] + amu[r] * d3[r]) * dt;
+    str<R>(f.vx_a + i, va_x);
+  }
+  {
+    float d1[R], d2[R], d3[R];
+    dpz<R>(s_szz_a, b, rdz, d1);
+    dpz<R>(s_sxx_a, b, rdz, d2);
+    dmx<R, BOXZ>(s_sxz_a, b, rdx, d3);
+#pragma unroll
+    for (int r = 0; r < R; ++r) va_z[r] -= (l2m[r] * d1[r] + lam[r] * d2[r] + amu[r] * d3[r]) * dt;
+    str<R>(f.vz_a + i, va_z);
+  }
 }
 
 // MID: a mid tile (no CPML cell): the adjoint memory arrays updated in their
 // bands (el_stress_adj.cu:68-94, within 2 cells of the CPML), the reverse
-// velocity update and its density terms only at cells of the reverse-time
-// interior, the ring's velocities of step it-1 restored, and the density
-// gathers with the guards of the edge form.
+// velocity update and its imaging sums only at cells of the reverse-time
+// interior, and the ring's velocities of step it-1 restored.
 template <int TX, int K, int R, bool MID>
 __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
@@ -1178,10 +1119,9 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
   SWEEP_SMEM(BOXZ)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
-  const int rev = it >= 1;
-  const float dt = g.dt;
-  float sa[R], xa[R], za[R], bA[R], bB[R], vz[R], vx[R], gd[R], bBj[R];
+  const bool rev = it >= 1;
   const uint64_t pol = media_policy();
+  float bA[R], bB[R], sa[R], xa[R], za[R], vz[R], vx[R], ga[R], gb[R];
   ldrm<R>(m.bycA + i, bA, pol);
   ldrm<R>(m.bycB + i, bB, pol);
   pdl_wait();
@@ -1189,25 +1129,19 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
   ldr<R>(f.szz_a + i, sa);
   ldr<R>(f.sxx_a + i, xa);
   ldr<R>(f.sxz_a + i, za);
-  float bAj0 = 0.0f;
-#pragma unroll
-  for (int r = 0; r < R; ++r) vz[r] = vx[r] = gd[r] = bBj[r] = 0.0f;
-  if (rev) {
-    ldr<R>(f.vz + i, vz);
-    ldr<R>(f.vx + i, vx);
-    ldr<R>(gr.den + i, gd);
-    ldrm<R>(m.bycB + i - ldz, bBj, pol);
-    bAj0 = ldm(m.bycA + i - 1, pol);
-  }
+  ldr<R>(f.vz + i, vz);
+  ldr<R>(f.vx + i, vx);
+  ldr<R>(gr.va + i, ga);
+  ldr<R>(gr.vb + i, gb);
   if (!stage_wait(&bar, err)) return;
   const float* s_vz_a = sm;
   const float* s_vx_a = sm + N;
   const float* s_szz = sm + 2 * N;
   const float* s_sxx = sm + 3 * N;
   const float* s_sxz = sm + 4 * N;
+  const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int bb = b + r;
     if (special && z + r >= sh.rbz0 && z + r <= sh.rbz1) {
       const int2 rr = bin_range(sh, z + r, x);
       for (int k = rr.x; k < rr.y; ++k) {
@@ -1219,18 +1153,23 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
         }
       }
     }
-    {
-      const float dvz_dx = -sdp(s_vz_a, bb, BOXZ, g.rdx);
-      const float dvx_dz = -sdp(s_vx_a, bb, 1, g.rdz);
-      za[r] += dvz_dx * bA[r] * dt + dvx_dz * bB[r] * dt;
+  }
+  {
+    float d1[R], d2[R], d3[R], d4[R];
+    dpx<R, BOXZ>(s_vz_a, b, rdx, d1);
+    dpz<R>(s_vx_a, b, rdz, d2);
+    dmx<R, BOXZ>(s_vx_a, b, rdx, d3);
+    dmz<R>(s_vz_a, b, rdz, d4);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      za[r] -= (d1[r] * bA[r] + d2[r] * bB[r]) * dt;
+      xa[r] -= bB[r] * d3[r] * dt;
+      sa[r] -= bA[r] * d4[r] * dt;
     }
-    {
-      const float dvx_dx = -sdm(s_vx_a, bb, BOXZ, g.rdx);
-      const float dvz_dz = -sdm(s_vz_a, bb, 1, g.rdz);
-      xa[r] += bB[r] * dvx_dx * dt;
-      sa[r] += bA[r] * dvz_dz * dt;
-    }
-    if constexpr (MID) {
+  }
+  if constexpr (MID) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
       const int zr = z + r;
       const bool xb = (x <= g.xband_lo) || (x >= g.xband_hi);
       const bool zb = (zr <= g.zband_lo) || (zr >= g.zband_hi);
@@ -1249,273 +1188,38 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
   str<R>(f.szz_a + i, sa);
   str<R>(f.sxx_a + i, xa);
   if (!rev) return;
+  float ea[R], eb[R], t[R], wa[R], wb[R];
+  dpz<R>(s_szz, b, rdz, ea);
+  dmx<R, BOXZ>(s_sxz, b, rdx, t);
+#pragma unroll
+  for (int r = 0; r < R; ++r) ea[r] += t[r];  // dszz_dz + dsxz_dx
+  dmz<R>(s_sxz, b, rdz, eb);
+  dpx<R, BOXZ>(s_sxx, b, rdx, t);
+  own<R>(s_vz_a, b, wa);
+  own<R>(s_vx_a, b, wb);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int bb = b + r;
+    eb[r] += t[r];  // dsxz_dz + dsxx_dx
     if (special && z + r == sh.src_z && x == sh.src_x) sh.gstf[it - 1] = -(sa[r] + 3.0f * xa[r]) * dt;
-    const int zr = z + r;
-    const bool inter = !MID || in_box(zr, x, g.zi0, g.zi1, g.xi0, g.xi1);
-    const float ea = sdp(s_szz, bb, 1, g.rdz) + sdm(s_sxz, bb, BOXZ, g.rdx);  // dszz_dz + dsxz_dx
-    const float eb = sdm(s_sxz, bb, 1, g.rdz) + sdp(s_sxx, bb, BOXZ, g.rdx);  // dsxz_dz + dsxx_dx
-    if (inter) {
-      vz[r] = vz[r] - ea * bA[r] * dt;
-      vx[r] = vx[r] - eb * bB[r] * dt;
+    if (!MID || in_box(z + r, x, g.zi0, g.zi1, g.xi0, g.xi1)) {
+      vz[r] -= ea[r] * bA[r] * dt;
+      vx[r] -= eb[r] * bB[r] * dt;
+      ga[r] += wa[r] * ea[r];
+      gb[r] += wb[r] * eb[r];
     }
     if constexpr (MID) {  // to_bnd of the velocities of step it - 1
-      const int k = ring_index(g, zr, x);
-      if (k >= 0) {
-        const float* p = S.st.base + static_cast<size_t>(it - 1) * 5 * g.ring_len + k;
+      const int q = ring_index(g, z + r, x);
+      if (q >= 0) {
+        const float* p = S.st.base + static_cast<size_t>(it - 1) * 5 * g.ring_len + q;
         vz[r] = p[3 * g.ring_len];
         vx[r] = p[4 * g.ring_len];
       }
     }
-    // rho kernel gather: in a fast tile all guards hold, in a mid tile they
-    // are those of el_velocity.cu:101-110.
-    if (!MID || in_box(zr, x, g.zi0, g.zi1, g.xi0, g.xi1 + 1)) {
-      const float bAj = r == 0 ? bAj0 : bA[r - 1];  // bycA at (z-1, x)
-      float acc = gd[r];
-      if (!MID || x <= g.xi1) {
-        acc += -s_vz_a[bb] * ea * dt * (-bA[r] * bA[r] * 0.5f);
-        acc += -s_vx_a[bb] * eb * dt * (-bB[r] * bB[r] * 0.5f);
-        if (!MID || zr - 1 >= g.zi0) {
-          const int bj = bb - 1;
-          const float e = sdp(s_szz, bj, 1, g.rdz) + sdm(s_sxz, bj, BOXZ, g.rdx);
-          acc += -s_vz_a[bj] * e * dt * (-bAj * bAj * 0.5f);
-        }
-      }
-      if (!MID || x - 1 >= g.xi0) {
-        const int bj = bb - BOXZ;
-        const float e = sdm(s_sxz, bj, 1, g.rdz) + sdp(s_sxx, bj, BOXZ, g.rdx);
-        acc += -s_vx_a[bj] * e * dt * (-bBj[r] * bBj[r] * 0.5f);
-      }
-      gd[r] = acc;
-    }
   }
   str<R>(f.vz + i, vz);
   str<R>(f.vx + i, vx);
-  str<R>(gr.den + i, gd);
-}
-
-// Backward fast bodies with two adjacent depths per thread, staged samples
-// read in pairs (as the forward two-row bodies): with b even, the float2 at
-// b + o (o even) holds the depths of both cells at offset o, so a z stencil
-// of both depths takes the pairs at b - 2, b, b + 2 and an x stencil the
-// pairs at b + k BOXZ. Operation order per cell is that of the one-row body.
-template <int TX, int K>
-__device__ __forceinline__ void bwd_B_fast2(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
-  constexpr int TZ = 64, BOXZ = TZ + 8, R = 2;
-  SWEEP_FAST_SLOT(TZ)
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
-  const Grads& gr = S.gr;
-  const int it = S.nSteps - 2 - j;
-  const float dt = g.dt;
-  float szz[2], sxx[2], sxz[2], lam[2], l2m[2], amu[2], gl[2], gm[2], w[2], h[2], va_z[2], va_x[2], hx[2];
-  const uint64_t pol = media_policy();
-  ldrm<2>(m.lam + i, lam, pol);
-  ldrm<2>(m.l2m + i, l2m, pol);
-  ldrm<2>(m.aveMu + i, amu, pol);
-  ldrm<2>(m.muw + i, w, pol);
-  ldrm<2>(m.hs + i, h, pol);
-  ldrm<2>(m.hs + i - ldz, hx, pol);
-  const float hz0 = ldm(m.hs + i - 1, pol), hzx0 = ldm(m.hs + i - ldz - 1, pol);
-  pdl_wait();
-  SWEEP_TMA(5, BOXZ)
-  ldr<2>(f.szz + i, szz);
-  ldr<2>(f.sxx + i, sxx);
-  ldr<2>(f.sxz + i, sxz);
-  ldr<2>(gr.lam + i, gl);
-  ldr<2>(gr.mu + i, gm);
-  ldr<2>(f.vz_a + i, va_z);
-  ldr<2>(f.vx_a + i, va_x);
-  if (!stage_wait(&bar, err)) return;
-  const float* s_vz = sm;
-  const float* s_vx = sm + N;
-  const float* s_sza = sm + 2 * N;
-  const float* s_xxa = sm + 3 * N;
-  const float* s_xza = sm + 4 * N;
-  const float rdz = g.rdz, rdx = g.rdx;
-  constexpr int B = BOXZ;
-  // vz: z pairs and x pairs
-  const float2 VZm = ld2(s_vz + b - 2), V0 = ld2(s_vz + b), VZp = ld2(s_vz + b + 2);
-  const float2 Vp1 = ld2(s_vz + b + B), Vp2 = ld2(s_vz + b + 2 * B), Vm1 = ld2(s_vz + b - B),
-               Vm2 = ld2(s_vz + b - 2 * B);
-  // vx: z pairs at columns 0 and -1, x pairs
-  const float2 UZm = ld2(s_vx + b - 2), U0 = ld2(s_vx + b), UZp = ld2(s_vx + b + 2);
-  const float2 Um1 = ld2(s_vx + b - B), Up1 = ld2(s_vx + b + B), Um2 = ld2(s_vx + b - 2 * B);
-  const float2 UmZm = ld2(s_vx + b - B - 2), UmZp = ld2(s_vx + b - B + 2);
-  // depth b - 1 at columns +1, +2, -1, -2 (the mu gathers of the upper cell)
-  const float vz_p1m = s_vz[b + B - 1], vz_p2m = s_vz[b + 2 * B - 1], vz_m1m = s_vz[b - B - 1],
-              vz_m2m = s_vz[b - 2 * B - 1];
-  // own-cell strains
-  const float dvz_dz[2] = {dd(V0.x, VZm.y, V0.y, VZm.x, rdz), dd(V0.y, V0.x, VZp.x, VZm.y, rdz)};
-  const float dvx_dx[2] = {dd(U0.x, Um1.x, Up1.x, Um2.x, rdx), dd(U0.y, Um1.y, Up1.y, Um2.y, rdx)};
-  const float dvx_dz[2] = {dd(U0.y, U0.x, UZp.x, UZm.y, rdz), dd(UZp.x, U0.y, UZp.y, U0.x, rdz)};
-  const float dvz_dx[2] = {dd(Vp1.x, V0.x, Vp2.x, Vm1.x, rdx), dd(Vp1.y, V0.y, Vp2.y, Vm1.y, rdx)};
-  // e = dvx_dz + dvz_dx at (z, x), (z-1, x), (z, x-1), (z-1, x-1) for both depths
-  const float e_own[2] = {dvx_dz[0] + dvz_dx[0], dvx_dz[1] + dvz_dx[1]};
-  const float e_zm0 = dd(U0.x, UZm.y, U0.y, UZm.x, rdz) + dd(vz_p1m, VZm.y, vz_p2m, vz_m1m, rdx);
-  const float e_xm[2] = {dd(Um1.y, Um1.x, UmZp.x, UmZm.y, rdz) + dd(V0.x, Vm1.x, Vp1.x, Vm2.x, rdx),
-                         dd(UmZp.x, Um1.y, UmZp.y, Um1.x, rdz) + dd(V0.y, Vm1.y, Vp1.y, Vm2.y, rdx)};
-  const float e_zxm0 = dd(Um1.x, UmZm.y, Um1.y, UmZm.x, rdz) + dd(VZm.y, vz_m1m, vz_p1m, vz_m2m, rdx);
-  const float e_zm[2] = {e_zm0, e_own[0]};
-  const float e_zxm[2] = {e_zxm0, e_xm[0]};
-  // adjoint stresses
-  const float2 SA0 = ld2(s_sza + b), SAZm = ld2(s_sza + b - 2), SAZp = ld2(s_sza + b + 2);
-  const float2 SAp1 = ld2(s_sza + b + B), SAp2 = ld2(s_sza + b + 2 * B), SAm1 = ld2(s_sza + b - B);
-  const float2 XA0 = ld2(s_xxa + b), XAZm = ld2(s_xxa + b - 2), XAZp = ld2(s_xxa + b + 2);
-  const float2 XAp1 = ld2(s_xxa + b + B), XAp2 = ld2(s_xxa + b + 2 * B), XAm1 = ld2(s_xxa + b - B);
-  const float2 ZA0 = ld2(s_xza + b), ZAZm = ld2(s_xza + b - 2), ZAZp = ld2(s_xza + b + 2);
-  const float2 ZAm1 = ld2(s_xza + b - B), ZAp1 = ld2(s_xza + b + B), ZAm2 = ld2(s_xza + b - 2 * B);
-  const float2 ZAmZm = ld2(s_xza + b - B - 2);
-  const float sa_[2] = {SA0.x, SA0.y}, xa_[2] = {XA0.x, XA0.y};
-  const float za_own[2] = {ZA0.x, ZA0.y}, za_zm[2] = {ZAZm.y, ZA0.x};
-  const float za_xm[2] = {ZAm1.x, ZAm1.y}, za_zxm[2] = {ZAmZm.y, ZAm1.x};
-  const float dszz_dx[2] = {-dd(SAp1.x, SA0.x, SAp2.x, SAm1.x, rdx), -dd(SAp1.y, SA0.y, SAp2.y, SAm1.y, rdx)};
-  const float dsxx_dx[2] = {-dd(XAp1.x, XA0.x, XAp2.x, XAm1.x, rdx), -dd(XAp1.y, XA0.y, XAp2.y, XAm1.y, rdx)};
-  const float dsxz_dz[2] = {-dd(ZA0.x, ZAZm.y, ZA0.y, ZAZm.x, rdz), -dd(ZA0.y, ZA0.x, ZAZp.x, ZAZm.y, rdz)};
-  const float dszz_dz[2] = {-dd(SA0.y, SA0.x, SAZp.x, SAZm.y, rdz), -dd(SAZp.x, SA0.y, SAZp.y, SA0.x, rdz)};
-  const float dsxx_dz[2] = {-dd(XA0.y, XA0.x, XAZp.x, XAZm.y, rdz), -dd(XAZp.x, XA0.y, XAZp.y, XA0.x, rdz)};
-  const float dsxz_dx[2] = {-dd(ZA0.x, ZAm1.x, ZAp1.x, ZAm2.x, rdx), -dd(ZA0.y, ZAm1.y, ZAp1.y, ZAm2.y, rdx)};
-  float o_gl[2], o_gm[2], o_szz[2], o_sxx[2], o_sxz[2], o_vza[2], o_vxa[2];
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const float hz = r == 0 ? hz0 : h[0];
-    const float hzx = r == 0 ? hzx0 : hx[0];
-    if (special && z + r == sh.src_z && x == sh.src_x) {
-      szz[r] -= sh.src_szz_r[it];
-      sxx[r] -= sh.src_sxx_r[it];
-    }
-    o_szz[r] = szz[r] - (l2m[r] * dvz_dz[r] + lam[r] * dvx_dx[r]) * dt;
-    o_sxx[r] = sxx[r] - (lam[r] * dvz_dz[r] + l2m[r] * dvx_dx[r]) * dt;
-    o_sxz[r] = sxz[r] - amu[r] * e_own[r] * dt;
-    o_gl[r] = gl[r] + -(sa_[r] + xa_[r]) * (dvz_dz[r] + dvx_dx[r]) * dt * kMega;
-    const float gmu_own = (-2.0f * sa_[r] * dvz_dz[r] * dt - 2.0f * xa_[r] * dvx_dx[r] * dt) * kMega;
-    float acc = gm[r] + gmu_own;
-    if (h[r] != 0.0f) acc += w[r] * (-za_own[r] * e_own[r] * dt * h[r]);
-    if (hz != 0.0f) acc += w[r] * (-za_zm[r] * e_zm[r] * dt * hz);
-    if (hx[r] != 0.0f) acc += w[r] * (-za_xm[r] * e_xm[r] * dt * hx[r]);
-    if (hzx != 0.0f) acc += w[r] * (-za_zxm[r] * e_zxm[r] * dt * hzx);
-    o_gm[r] = acc;
-    o_vxa[r] = va_x[r] + (lam[r] * dszz_dx[r] * dt + l2m[r] * dsxx_dx[r] * dt + amu[r] * dsxz_dz[r] * dt);
-    o_vza[r] = va_z[r] + (l2m[r] * dszz_dz[r] * dt + lam[r] * dsxx_dz[r] * dt + amu[r] * dsxz_dx[r] * dt);
-  }
-  str<2>(gr.lam + i, o_gl);
-  str<2>(f.szz + i, o_szz);
-  str<2>(f.sxx + i, o_sxx);
-  str<2>(f.sxz + i, o_sxz);
-  str<2>(gr.mu + i, o_gm);
-  str<2>(f.vx_a + i, o_vxa);
-  str<2>(f.vz_a + i, o_vza);
-}
-
-template <int TX, int K>
-__device__ __forceinline__ void bwd_C_fast2(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
-  constexpr int TZ = 64, BOXZ = TZ + 8, R = 2;
-  SWEEP_FAST_SLOT(TZ)
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
-  const Grads& gr = S.gr;
-  const int it = S.nSteps - 2 - j;
-  const int rev = it >= 1;
-  const float dt = g.dt;
-  float sa[2], xa[2], za[2], bA[2], bB[2], vz[2], vx[2], gd[2], bBj[2];
-  const uint64_t pol = media_policy();
-  ldrm<2>(m.bycA + i, bA, pol);
-  ldrm<2>(m.bycB + i, bB, pol);
-  pdl_wait();
-  SWEEP_TMA(5, BOXZ)
-  ldr<2>(f.szz_a + i, sa);
-  ldr<2>(f.sxx_a + i, xa);
-  ldr<2>(f.sxz_a + i, za);
-  float bAj0 = 0.0f;
-  vz[0] = vz[1] = vx[0] = vx[1] = gd[0] = gd[1] = bBj[0] = bBj[1] = 0.0f;
-  if (rev) {
-    ldr<2>(f.vz + i, vz);
-    ldr<2>(f.vx + i, vx);
-    ldr<2>(gr.den + i, gd);
-    ldrm<2>(m.bycB + i - ldz, bBj, pol);
-    bAj0 = ldm(m.bycA + i - 1, pol);
-  }
-  if (!stage_wait(&bar, err)) return;
-  const float* s_vza = sm;
-  const float* s_vxa = sm + N;
-  const float* s_szz = sm + 2 * N;
-  const float* s_sxx = sm + 3 * N;
-  const float* s_sxz = sm + 4 * N;
-  const float rdz = g.rdz, rdx = g.rdx;
-  constexpr int B = BOXZ;
-  const float2 VA0 = ld2(s_vza + b), VAZm = ld2(s_vza + b - 2), VAZp = ld2(s_vza + b + 2);
-  const float2 VAp1 = ld2(s_vza + b + B), VAp2 = ld2(s_vza + b + 2 * B), VAm1 = ld2(s_vza + b - B);
-  const float2 XA0 = ld2(s_vxa + b), XAZm = ld2(s_vxa + b - 2), XAZp = ld2(s_vxa + b + 2);
-  const float2 XAm1 = ld2(s_vxa + b - B), XAp1 = ld2(s_vxa + b + B), XAm2 = ld2(s_vxa + b - 2 * B);
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    if (special && z + r >= sh.rbz0 && z + r <= sh.rbz1) {
-      const int2 rr = bin_range(sh, z + r, x);
-      for (int k = rr.x; k < rr.y; ++k) {
-        const int q = sh.blk_rec[k];
-        if (sh.rec_z[q] == z + r && sh.rec_x[q] == x) {
-          const float rv = sh.res[static_cast<size_t>(q) * sh.nSteps + it];
-          sa[r] += rv;
-          xa[r] += 3.0f * rv;
-        }
-      }
-    }
-  }
-  {
-    const float dvz_dx[2] = {-dd(VAp1.x, VA0.x, VAp2.x, VAm1.x, rdx), -dd(VAp1.y, VA0.y, VAp2.y, VAm1.y, rdx)};
-    const float dvx_dz[2] = {-dd(XA0.y, XA0.x, XAZp.x, XAZm.y, rdz), -dd(XAZp.x, XA0.y, XAZp.y, XA0.x, rdz)};
-    const float dvx_dx[2] = {-dd(XA0.x, XAm1.x, XAp1.x, XAm2.x, rdx), -dd(XA0.y, XAm1.y, XAp1.y, XAm2.y, rdx)};
-    const float dvz_dz[2] = {-dd(VA0.x, VAZm.y, VA0.y, VAZm.x, rdz), -dd(VA0.y, VA0.x, VAZp.x, VAZm.y, rdz)};
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      za[r] += dvz_dx[r] * bA[r] * dt + dvx_dz[r] * bB[r] * dt;
-      xa[r] += bB[r] * dvx_dx[r] * dt;
-      sa[r] += bA[r] * dvz_dz[r] * dt;
-    }
-  }
-  str<2>(f.sxz_a + i, za);
-  str<2>(f.szz_a + i, sa);
-  str<2>(f.sxx_a + i, xa);
-  if (!rev) return;
-  const float2 PZm = ld2(s_szz + b - 2), PZ0 = ld2(s_szz + b), PZp = ld2(s_szz + b + 2);
-  const float2 Q0 = ld2(s_sxz + b), Qm1 = ld2(s_sxz + b - B), Qp1 = ld2(s_sxz + b + B), Qm2 = ld2(s_sxz + b - 2 * B);
-  const float2 QZm = ld2(s_sxz + b - 2), QZp = ld2(s_sxz + b + 2);
-  const float2 QmZm = ld2(s_sxz + b - B - 2), QmZp = ld2(s_sxz + b - B + 2);
-  const float2 X0 = ld2(s_sxx + b), Xp1 = ld2(s_sxx + b + B), Xp2 = ld2(s_sxx + b + 2 * B), Xm1 = ld2(s_sxx + b - B),
-               Xm2 = ld2(s_sxx + b - 2 * B);
-  // sxz at depth b - 1, columns -1, +1, -2 (the upper cell's z-neighbour gather)
-  const float q_m1m = s_sxz[b - B - 1], q_p1m = s_sxz[b + B - 1], q_m2m = s_sxz[b - 2 * B - 1];
-  // ea = dszz_dz + dsxz_dx, eb = dsxz_dz + dsxx_dx at (z, x) for both depths
-  const float ea[2] = {dd(PZ0.y, PZ0.x, PZp.x, PZm.y, rdz) + dd(Q0.x, Qm1.x, Qp1.x, Qm2.x, rdx),
-                       dd(PZp.x, PZ0.y, PZp.y, PZ0.x, rdz) + dd(Q0.y, Qm1.y, Qp1.y, Qm2.y, rdx)};
-  const float eb[2] = {dd(Q0.x, QZm.y, Q0.y, QZm.x, rdz) + dd(Xp1.x, X0.x, Xp2.x, Xm1.x, rdx),
-                       dd(Q0.y, Q0.x, QZp.x, QZm.y, rdz) + dd(Xp1.y, X0.y, Xp2.y, Xm1.y, rdx)};
-  // ea at (z-1, x): the upper cell's from depth b - 1, the lower cell's is ea[0]
-  const float ea_zm0 = dd(PZ0.x, PZm.y, PZ0.y, PZm.x, rdz) + dd(QZm.y, q_m1m, q_p1m, q_m2m, rdx);
-  // eb at (z, x-1)
-  const float eb_xm[2] = {dd(Qm1.x, QmZm.y, Qm1.y, QmZm.x, rdz) + dd(X0.x, Xm1.x, Xp1.x, Xm2.x, rdx),
-                          dd(Qm1.y, Qm1.x, QmZp.x, QmZm.y, rdz) + dd(X0.y, Xm1.y, Xp1.y, Xm2.y, rdx)};
-  const float ea_zm[2] = {ea_zm0, ea[0]};
-  const float va_own[2] = {VA0.x, VA0.y}, va_zm[2] = {VAZm.y, VA0.x};
-  const float xa_own[2] = {XA0.x, XA0.y}, xa_xm[2] = {XAm1.x, XAm1.y};
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    if (special && z + r == sh.src_z && x == sh.src_x) sh.gstf[it - 1] = -(sa[r] + 3.0f * xa[r]) * dt;
-    vz[r] = vz[r] - ea[r] * bA[r] * dt;
-    vx[r] = vx[r] - eb[r] * bB[r] * dt;
-    const float bAj = r == 0 ? bAj0 : bA[0];
-    float acc = gd[r];
-    acc += -va_own[r] * ea[r] * dt * (-bA[r] * bA[r] * 0.5f);
-    acc += -xa_own[r] * eb[r] * dt * (-bB[r] * bB[r] * 0.5f);
-    acc += -va_zm[r] * ea_zm[r] * dt * (-bAj * bAj * 0.5f);
-    acc += -xa_xm[r] * eb_xm[r] * dt * (-bBj[r] * bBj[r] * 0.5f);
-    gd[r] = acc;
-  }
-  str<2>(f.vz + i, vz);
-  str<2>(f.vx + i, vx);
-  str<2>(gr.den + i, gd);
+  str<R>(gr.va + i, ga);
+  str<R>(gr.vb + i, gb);
 }
 
 // ---------------------------------------------------------------------------
@@ -1565,10 +1269,7 @@ template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R)
   if (fast) {
-    if constexpr (R == 1)
-      bwd_B_fast<TX, K, 1, false>(P, shot, z0, x0, j, err);
-    else
-      bwd_B_fast2<TX, K>(P, shot, z0, x0, j, err);
+    bwd_B_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   } else if (mid) {
     bwd_B_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
   } else {
@@ -1580,10 +1281,7 @@ template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_C(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R)
   if (fast) {
-    if constexpr (R == 1)
-      bwd_C_fast<TX, K, 1, false>(P, shot, z0, x0, j, err);
-    else
-      bwd_C_fast2<TX, K>(P, shot, z0, x0, j, err);
+    bwd_C_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   } else if (mid) {
     bwd_C_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
   } else {
@@ -1917,7 +1615,14 @@ __global__ void k_src_terms(int nt, float dt, const float* __restrict__ amp, flo
 
 // Adds the per-shot gradients and / or illuminations of a shot group into
 // the global ones, in group order (deterministic): shot k's sub-grid column j
-// is global padded column x_off[k] + j.
+// is global padded column x_off[k] + j. The gradients come out of the sweeps'
+// sums over time through the imaging chain rules: lambda and mu directly, mu
+// through the 2x2 harmonic averages whose top-left corner is (z, x), (z-1, x),
+// (z, x-1), (z-1, x-1) (hs = aveMu / sum(1/mu) 1e6, muw = 1 / mu^2), with the
+// guards of el_stress.cu:118-123 (the x guard of :120 is always true), and rho
+// through the buoyancies of (z, x), (z-1, x) and (z, x-1)
+// (el_velocity.cu:101-110; the x guard of :109 is always true). The sums are
+// zero outside a shot's reverse-time interior.
 __global__ void k_reduce_grads(int nz, int nx, int ldz, int nshots, const ShotSlot* __restrict__ slots, float* g_lam,
                                float* g_mu, float* g_den, float* g_illum) {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1927,12 +1632,22 @@ __global__ void k_reduce_grads(int nz, int nx, int ldz, int nshots, const ShotSl
   if (g_lam) {
     float a = g_lam[i], b = g_mu[i], c = g_den[i];
     for (int k = 0; k < nshots; ++k) {
-      const int xs = x - slots[k].x_off;
-      if (xs < 0 || xs >= slots[k].g.nx) continue;
-      const size_t j = static_cast<size_t>(xs) * ldz + z;
-      a += slots[k].gr.lam[j];
-      b += slots[k].gr.mu[j];
-      c += slots[k].gr.den[j];
+      const ShotSlot& S = slots[k];
+      const Geo& g = S.g;
+      const int xs = x - S.x_off;
+      if (!in_box(z, xs, g.zi0, g.zi1, g.xi0, g.xi1 + 1)) continue;
+      const size_t j = static_cast<size_t>(xs) * ldz + z, l = j - ldz;
+      const float* __restrict__ hs = S.m.hs;
+      const float* __restrict__ tau = S.gr.tau;
+      const float dt = g.dt;
+      a -= S.gr.lam[j] * dt * kMega;
+      auto block = [&](size_t q) { return hs[q] != 0.0f ? hs[q] * tau[q] : 0.0f; };  // hs = 0: fluid, no shear term
+      float t = block(l);
+      if (xs <= g.xi1) t += block(j) + block(j - 1) + block(l - 1);
+      b -= 2.0f * S.gr.mu[j] * dt * kMega + S.m.muw[j] * (t * dt);
+      const float bA = S.m.bycA[j], bAu = S.m.bycA[j - 1], bB = S.m.bycB[j], bBl = S.m.bycB[l];
+      c += 0.5f * dt *
+           (bA * bA * S.gr.va[j] + bB * bB * S.gr.vb[j] + bAu * bAu * S.gr.va[j - 1] + bBl * bBl * S.gr.vb[l]);
     }
     g_lam[i] = a;
     g_mu[i] = b;
@@ -1966,13 +1681,6 @@ template <int TX, int BOXZ>
 constexpr size_t smem_bytes(int na) {
   return static_cast<size_t>(na) * BOXZ * (TX + 4) * sizeof(float);
 }
-// Backward sweep B, one-row tiles: the five staged boxes, then the strains its
-// fast bodies' mu gathers share ((TX + 1) columns x 33 depths).
-template <int TX>
-constexpr size_t bwd_B_smem_one_row() {
-  return smem_bytes<TX, kBoxZ>(5) + static_cast<size_t>((TX + 1) * 33) * sizeof(float);
-}
-
 }  // namespace
 
 #define FWIGB_DISPATCH_TX(tx, ...) \
@@ -2049,10 +1757,10 @@ int launch_bwd_B(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>&
                                      smem_bytes<TX, kBoxZFwd>(5), s, p, j, err))
   else if (regs > 32)
     FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_B<TX, K, 1, 1536>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
-                                     bwd_B_smem_one_row<TX>(), s, p, j, err))
+                                     smem_bytes<TX, kBoxZ>(5), s, p, j, err))
   else
     FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_B<TX, K, 1, 2048>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
-                                     bwd_B_smem_one_row<TX>(), s, p, j, err))
+                                     smem_bytes<TX, kBoxZ>(5), s, p, j, err))
   return 1;
 }
 
