@@ -407,7 +407,8 @@ struct ShotPlan {
   int nbin_z = 0, nbin = 0;
   size_t src_off = 0;   // floats: 2 * nSteps (szz and sxx source terms)
   size_t rec_off = 0;   // ints: 2 * nrec (sub-grid z, then x)
-  size_t blk_off = 0;   // ints: nbin + 1 + nrec (receiver bins, CSR)
+  size_t blk_off = 0;   // ints: nbin + 1 + nrec (receiver bins, CSR), then nrec + map_cells (receiver map)
+  size_t map_cells = 0; // cells of the receiver map (0: none)
   size_t data_off = 0;  // floats: obs | syn | res, each nrec * nSteps
   size_t taper_off = 0; // floats: 2 * nSteps, or 2 * nrec * nSteps with per-trace windows
   size_t filt_off = 0;  // floats: the band-pass impulse response (2 * nSteps), when filtering
@@ -467,6 +468,11 @@ struct fwigb_ctx {
   std::vector<int> pack_nx;
   // Launch extents per pack.
   std::vector<SweepGrid> pack_grid;
+  // The group's marching plan (march.cu) when the call runs that way.
+  bool marching = false;
+  int sms = 0;
+  MarchPack march{};
+  DevBuf march_flags;
   int last_groups = 0;
   // CUDA graph of a single-group call's whole launch sequence, replayed while
   // everything it was captured from is unchanged (graph_key).
@@ -675,6 +681,7 @@ int open_ctx(const char* para_fname, int device, fwigb_ctx* ctx) {
     return FWIGB_ERR_PARAM;
   }
   CK(cudaSetDevice(device));
+  CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, device));
   CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   return setup_geometry(ctx);
 }
@@ -778,7 +785,20 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
     pl.rec_off = n_rec;
     n_rec += 2 * static_cast<size_t>(pl.nrec);
     pl.blk_off = n_blk;
-    n_blk += static_cast<size_t>(pl.nbin) + 1 + pl.nrec;
+    // Bounding box of the receivers and the source (sub-grid cells), and a map
+    // of it to the receivers unless that took more room than their gathers
+    // (scattered receivers with a short record).
+    pl.rbz0 = pl.rbz1 = sg.z_src;
+    pl.rbx0 = pl.rbx1 = sg.x_src - pl.x_off;
+    for (int r = 0; r < pl.nrec; ++r) {
+      pl.rbz0 = std::min(pl.rbz0, sg.z_rec[r]);
+      pl.rbz1 = std::max(pl.rbz1, sg.z_rec[r]);
+      pl.rbx0 = std::min(pl.rbx0, sg.x_rec[r] - pl.x_off);
+      pl.rbx1 = std::max(pl.rbx1, sg.x_rec[r] - pl.x_off);
+    }
+    const size_t box = static_cast<size_t>(pl.rbz1 - pl.rbz0 + 1) * (pl.rbx1 - pl.rbx0 + 1);
+    pl.map_cells = box <= static_cast<size_t>(pl.nrec) * pl.nSteps ? box : 0;
+    n_blk += static_cast<size_t>(pl.nbin) + 1 + 2 * static_cast<size_t>(pl.nrec) + pl.map_cells;
     pl.data_off = n_data;
     n_data += 3 * static_cast<size_t>(pl.nrec) * pl.nSteps;
     pl.taper_off = n_taper;
@@ -867,17 +887,20 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
     int* off = hblk.data() + pl.blk_off;
     int* lst = off + pl.nbin + 1;
     std::vector<int> cnt(pl.nbin + 1, 0);
-    // Bounding box of the receivers and the source (sub-grid cells).
-    pl.rbz0 = pl.rbz1 = g.z_src;
-    pl.rbx0 = pl.rbx1 = g.x_src - pl.x_off;
     for (int r = 0; r < pl.nrec; ++r) {
       rz[r] = g.z_rec[r];
       rx[r] = g.x_rec[r] - pl.x_off;
       cnt[(rz[r] / kBinZ) + (rx[r] / kBinX) * pl.nbin_z + 1]++;
-      pl.rbz0 = std::min(pl.rbz0, rz[r]);
-      pl.rbz1 = std::max(pl.rbz1, rz[r]);
-      pl.rbx0 = std::min(pl.rbx0, rx[r]);
-      pl.rbx1 = std::max(pl.rbx1, rx[r]);
+    }
+    if (pl.map_cells) {
+      int* next = lst + pl.nrec;
+      int* map = next + pl.nrec;
+      std::fill(map, map + pl.map_cells, -1);
+      for (int r = pl.nrec - 1; r >= 0; --r) {  // backwards: each cell's receivers come out in ascending order
+        int& at = map[static_cast<size_t>(rx[r] - pl.rbx0) * (pl.rbz1 - pl.rbz0 + 1) + (rz[r] - pl.rbz0)];
+        next[r] = at;
+        at = r | (at >= 0 ? kRecMore : 0);
+      }
     }
     for (int b = 0; b < pl.nbin; ++b) cnt[b + 1] += cnt[b];
     for (int b = 0; b <= pl.nbin; ++b) off[b] = cnt[b];
@@ -1043,6 +1066,21 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
   return n;
 }
 
+// Whether the staged shots run as marching kernels (march.cu) rather than as
+// tile sweeps, one launch per sweep and step: small calls, of at most
+// kMarchCells cells in at most kPackShots shots (all shots of the call, so
+// that the grouping does not change the choice). Microseconds a step, marching
+// against tiles: 16k cells 9.2 / 21.1, 100k 13.0 / 22.7, 290k (one shot) 25.4 /
+// 25.2, 400k (4 and 8 shots) 31.7 / 34.8 and 33.3 / 37.6, 590k 40.0 / 39.7,
+// 970k 63 / 50.
+// Fixed tile shapes and per-sweep timing ask for the sweeps themselves.
+constexpr size_t kMarchCells = 400000;
+bool marches(const fwigb_ctx* ctx) {
+  size_t cells = 0;
+  for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
+  return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
+}
+
 // Builds and uploads the slots and tensor maps of a group's members.
 int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   const size_t ldz = ctx->geo.ldz;
@@ -1089,6 +1127,8 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
     sh.blk_off = ctx->shot_blk.as<int>(pl.blk_off);
     sh.blk_rec = sh.blk_off + pl.nbin + 1;
     sh.nbin_z = pl.nbin_z;
+    sh.rec_next = pl.map_cells ? sh.blk_rec + pl.nrec : nullptr;
+    sh.rec_map = pl.map_cells ? sh.rec_next + pl.nrec : nullptr;
     sh.rbz0 = pl.rbz0;
     sh.rbz1 = pl.rbz1;
     sh.rbx0 = pl.rbx0;
@@ -1142,6 +1182,14 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
         pk.maps[k % kPackShots] = maps[static_cast<size_t>(w) * ctx->group_cap + k];
         pk.slots[k % kPackShots] = slots[k];
       }
+  }
+  ctx->marching = marches(ctx);
+  if (ctx->marching) {
+    std::memset(static_cast<void*>(&ctx->march), 0, sizeof(ctx->march));
+    ctx->march.nshots = G;
+    for (int k = 0; k < G; ++k) ctx->march.slots[k] = slots[k];
+    ctx->marching = march_plan(ctx->march, ctx->sms);
+    if (ctx->marching) CK(ctx->march_flags.ensure(2 * march_flag_bytes(ctx->march)));
   }
   // Device copy of the slots for the gradient reduction.
   CK(cudaMemcpyAsync(ctx->g_slots.p, slots.data(), slots.size() * sizeof(ShotSlot), cudaMemcpyHostToDevice,
@@ -1328,7 +1376,7 @@ int run(fwigb_ctx* ctx, int calc_id) {
     const int G = static_cast<int>(mem.size());
     int nx_max = 0;
     TRY_RC(build_group(ctx, mem, nx_max));
-    if (ctx->autotune && (!ctx->tuned_fwd || (adj && !ctx->tuned_bwd))) TRY_RC(autotune(ctx, G, nx_max, adj));
+    if (!ctx->marching && ctx->autotune && (!ctx->tuned_fwd || (adj && !ctx->tuned_bwd))) TRY_RC(autotune(ctx, G, nx_max, adj));
     const ShotSlot* slots = ctx->g_slots.as<ShotSlot>();
     (void)nx_max;
     std::vector<int> nst(G);
@@ -1352,7 +1400,14 @@ int run(fwigb_ctx* ctx, int calc_id) {
       if (adj || ctx->illum)
         CK(cudaMemsetAsync(ctx->g_grads.p, 0, static_cast<size_t>(G) * ctx->grads_stride * sizeof(float), s));
       const int ntop = nst[0];
-      for (int it = 0; it <= ntop - 2; ++it) {
+      unsigned* done = ctx->march_flags.as<unsigned>();
+      const size_t flag_bytes = ctx->marching ? march_flag_bytes(ctx->march) : 0;
+      if (ctx->marching) {
+        CK(cudaMemsetAsync(done, 0, 2 * flag_bytes, s));
+        CK(launch_march(s, ctx->march, false, (adj ? 1 : 0) | (ctx->inject_timeout ? 2 : 0), done, d_err));
+        ++group_launches;
+      }
+      for (int it = 0; it <= ntop - 2 && !ctx->marching; ++it) {
         const int a = active(it);
         const int f1_flags = (adj ? 1 : 0) | (ctx->inject_timeout && it == 0 ? 2 : 0);
         TIMED(0, group_launches += launch_sweep(ctx, 0, ctx->tx[0], ctx->rows[0], a, it, f1_flags, d_err));
@@ -1443,11 +1498,16 @@ int run(fwigb_ctx* ctx, int calc_id) {
         // then res_injection(nSteps-1) + el_stress_adj, source_grad(nSteps-2),
         // reverse velocity of step nSteps-2 ... (libCUFD.cu:353-445), with
         // backward iteration j meaning step nSteps_k - 2 - j of member k.
-        TIMED(3, group_launches += launch_sweep(ctx, 3, ctx->tx[3], ctx->rows[3], G, -1, 0, d_err));
-        for (int j = 0; j <= ntop - 2; ++j) {
-          const int a = active(j);
-          TIMED(2, group_launches += launch_sweep(ctx, 2, ctx->tx[2], ctx->rows[2], a, j, 0, d_err));
-          TIMED(3, group_launches += launch_sweep(ctx, 3, ctx->tx[3], ctx->rows[3], a, j, 0, d_err));
+        if (ctx->marching) {
+          CK(launch_march(s, ctx->march, true, 0, done + flag_bytes / sizeof(unsigned), d_err));
+          ++group_launches;
+        } else {
+          TIMED(3, group_launches += launch_sweep(ctx, 3, ctx->tx[3], ctx->rows[3], G, -1, 0, d_err));
+          for (int j = 0; j <= ntop - 2; ++j) {
+            const int a = active(j);
+            TIMED(2, group_launches += launch_sweep(ctx, 2, ctx->tx[2], ctx->rows[2], a, j, 0, d_err));
+            TIMED(3, group_launches += launch_sweep(ctx, 3, ctx->tx[3], ctx->rows[3], a, j, 0, d_err));
+          }
         }
       }
       if (adj || ctx->illum) {
@@ -1498,7 +1558,12 @@ int run(fwigb_ctx* ctx, int calc_id) {
       };
       static_assert(sizeof(SweepPack<1>) % 8 == 0 && sizeof(SweepPack<kPackShots>) % 8 == 0,
                     "launch parameters are compared as 64-bit words");
-      if (G == 1)
+      key.push_back(ctx->marching);
+      key.push_back(reinterpret_cast<uint64_t>(ctx->march_flags.p));
+      static_assert(sizeof(MarchPack) % 8 == 0, "launch parameters are compared as 64-bit words");
+      if (ctx->marching)
+        add_words(&ctx->march, sizeof(MarchPack));
+      else if (G == 1)
         add_words(ctx->pack1.data(), ctx->pack1.size() * sizeof(SweepPack<1>));
       else
         add_words(ctx->packs.data(), ctx->packs.size() * sizeof(SweepPack<kPackShots>));
@@ -1690,7 +1755,7 @@ int fwigb_destroy(fwigb_ctx* ctx) {
                     &ctx->shot_supd, &ctx->supd_part, &ctx->supd_coef, &ctx->supd_k,
                     &ctx->g_fields,
                     &ctx->g_store, &ctx->g_grads,
-                    &ctx->g_slots})
+                    &ctx->g_slots, &ctx->march_flags})
     b->release();
   for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);

@@ -22,6 +22,8 @@ namespace fwigb {
 constexpr int kTileZ = 32;
 constexpr int kRowsFwd = 2;
 constexpr int kTileZFwd = kTileZ * kRowsFwd;
+// A receiver index in ShotD::rec_map / rec_next whose cell holds a further one.
+constexpr int kRecMore = 1 << 30;
 // Receivers are binned on a fixed 32 x 8 grid, independent of the sweep tile.
 constexpr int kBinZ = 32;
 constexpr int kBinX = 8;
@@ -127,6 +129,9 @@ struct ShotD {
   int nrec, nSteps;
   const int* rec_z;       // receiver cells
   const int* rec_x;
+  const int* rec_map;     // per cell of the bounding box below (z fastest): -1, or its first receiver, plus
+                          // kRecMore when rec_next names another on the same cell; null: the bins instead
+  const int* rec_next;    // per receiver: as rec_map, the next one on its cell
   const int* blk_off;     // receivers per 32 x 8 bin (CSR over the bins)
   const int* blk_rec;
   int nbin_z;             // bins along z
@@ -225,6 +230,24 @@ int launch_bwd_B(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>&
 template <int K>
 int launch_bwd_C(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>& p, int nshots, const SweepGrid& gr,
                  int j, unsigned* err);
+// ---- marching kernels (march.cu): one launch per pass over time for up to
+// kPackShots shots. Block b belongs to the shot k with first[k] <= b <
+// first[k + 1] and holds an even share of its columns.
+constexpr int kMarchThreads = 1024;
+struct MarchPack {
+  int nshots, threads, smem;
+  int first[kPackShots + 1];
+  ShotSlot slots[kPackShots];
+};
+static_assert(sizeof(MarchPack) < 32000, "march pack exceeds the kernel parameter limit");
+// Fills `first` and `threads` for a GPU of `sms` SMs (one block each); false
+// when the shots have more strips than that.
+bool march_plan(MarchPack& p, int sms);
+// Bytes of the strips' flags; they are zeroed before each pass.
+size_t march_flag_bytes(const MarchPack& p);
+// flags: as launch_fwd_stress (forward pass only).
+cudaError_t launch_march(cudaStream_t s, const MarchPack& p, bool backward, int flags, unsigned* done, unsigned* err);
+
 // Adds the per-shot gradients (when g_lam is not null) and illuminations (when
 // g_illum is not null) of the first nshots slots into the global ones.
 void launch_reduce_grads(cudaStream_t s, int nz, int nx, int ldz, int nshots, const ShotSlot* slots, float* g_lam,

@@ -17,6 +17,7 @@
 // cell's own time-dependent factor and one kernel per call gathers them (see
 // "Imaging" below), so there are no atomics and the sums are deterministic.
 #include "fwigb_kernels.h"
+#include "sweep_cells.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -26,16 +27,10 @@
 namespace fwigb {
 namespace {
 
-constexpr float C1 = 1.125f;          // 9/8  (el_stress.cu:42)
-constexpr float C2 = 1.0f / 24.0f;    // 1/24 (el_stress.cu:43)
-constexpr float kMega = 1.0e6f;       // MEGA (utilities.h:16)
-
-// Bounded waits: a sweep that has waited this long (global timer) for its
-// staged tiles gives up, raises its error word and returns instead of
-// hanging. Each poll asks the hardware to suspend the thread until the
-// barrier phase completes or kWaitHintNs pass, so a waiting warp issues a
-// few instructions instead of spinning.
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;
+// Bounded waits (kWaitLimitNs) for the staged tiles: each poll asks the
+// hardware to suspend the thread until the barrier phase completes or
+// kWaitHintNs pass, so a waiting warp issues a few instructions instead of
+// spinning.
 constexpr unsigned kWaitHintNs = 1000000u;
 // Polls (without a suspend hint) of the injected wait of the timeout test
 // hook (stage_wait).
@@ -69,11 +64,6 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t* bar, unsigned parit
       : "r"(smem_u32(bar)), "r"(parity), "r"(kWaitHintNs)
       : "memory");
   return ok != 0;
-}
-__device__ __forceinline__ unsigned long long global_timer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 // Waits for phase `parity` of the barrier, at most kWaitLimitNs.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity) {
@@ -148,16 +138,7 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar, unsigned* err, bool in
   return true;
 }
 
-// Staggered 4th-order differences. Dm uses (i-2, i-1, i, i+1), Dp
-// (i-1, i, i+1, i+2); `s` is the stride of the direction and r the
-// reciprocal spacing. sdm / sdp read a staged tile (32-bit indices), gdm / gdp
-// global memory.
-__device__ __forceinline__ float sdm(const float* a, int i, int s, float r) {
-  return (C1 * (a[i] - a[i - s]) - C2 * (a[i + s] - a[i - 2 * s])) * r;
-}
-__device__ __forceinline__ float sdp(const float* a, int i, int s, float r) {
-  return (C1 * (a[i + s] - a[i]) - C2 * (a[i + 2 * s] - a[i - s])) * r;
-}
+// sdm / sdp on global memory.
 __device__ __forceinline__ float gdm(const float* __restrict__ a, size_t i, size_t s, float r) {
   return (C1 * (a[i] - a[i - s]) - C2 * (a[i + s] - a[i - 2 * s])) * r;
 }
@@ -165,52 +146,10 @@ __device__ __forceinline__ float gdp(const float* __restrict__ a, size_t i, size
   return (C1 * (a[i + s] - a[i]) - C2 * (a[i + 2 * s] - a[i - s])) * r;
 }
 
-// Index of cell (z, x) in the per-step boundary ring, or -1. Top and bottom
-// bands are stored column by column (5 depths each), left and right bands
-// column by column over their height, so a warp of consecutive depths writes
-// consecutive words.
-__device__ __forceinline__ int ring_index(const Geo& g, int z, int x) {
-  if (z < g.rz0 || z > g.rz1 || x < g.rx0 || x > g.rx1) return -1;
-  if (z <= g.rz0 + 4) return (x - g.rx0) * 5 + (z - g.rz0);
-  if (z >= g.rz1 - 4) return 5 * g.ringW + (x - g.rx0) * 5 + (z - (g.rz1 - 4));
-  if (x <= g.rx0 + 4) return 10 * g.ringW + (x - g.rx0) * g.ringH + (z - (g.rz0 + 5));
-  if (x >= g.rx1 - 4) return 10 * g.ringW + 5 * g.ringH + (x - (g.rx1 - 4)) * g.ringH + (z - (g.rz0 + 5));
-  return -1;
-}
-
-// from_bnd of step it for cell (z, x) when it lies in the ring: the stresses
-// before the step's update and the velocities of the staged tile
-// (Boundary.cu:55-76).
-__device__ __forceinline__ void ring_save(const Geo& g, const StoreD& st, int it, int z, int x, float szz, float sxz,
-                                          float sxx, float vz, float vx) {
-  const int k = ring_index(g, z, x);
-  if (k < 0) return;
-  float* p = st.base + static_cast<size_t>(it) * 5 * g.ring_len + k;
-  p[0] = szz;
-  p[g.ring_len] = sxz;
-  p[2 * g.ring_len] = sxx;
-  p[3 * g.ring_len] = vz;
-  p[4 * g.ring_len] = vx;
-}
-
-// a / K of the CPML formulas, with the division skipped where K == 1 (exact:
-// a / 1 == a), i.e. everywhere outside the CPML.
-__device__ __forceinline__ float kdiv(float a, float K) { return K == 1.0f ? a : a / K; }
-
-__device__ __forceinline__ bool in_box(int z, int x, int z0, int z1, int x0, int x1) {
-  return z >= z0 && z <= z1 && x >= x0 && x <= x1;
-}
-
 // Whether the tile of tz depths x tx columns at (z0, x0) meets the bounding
 // box of the shot's receivers and source.
 __device__ __forceinline__ bool tile_meets_shot_box(const ShotD& sh, int z0, int x0, int tz, int tx) {
   return !(z0 + tz - 1 < sh.rbz0 || z0 > sh.rbz1 || x0 + tx - 1 < sh.rbx0 || x0 > sh.rbx1);
-}
-
-// Receiver list of the 32 x 8 bin holding (z, x).
-__device__ __forceinline__ int2 bin_range(const ShotD& sh, int z, int x) {
-  const int b = (z / kBinZ) + (x / kBinX) * sh.nbin_z;
-  return make_int2(sh.blk_off[b], sh.blk_off[b + 1]);
 }
 
 // Every sweep is one launch per time step for a pack of shots: blockIdx.z is
@@ -404,14 +343,7 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
     }
     // The velocity sweep that follows does not change the stresses, so the
     // sample of step it+1 is taken here.
-    if (rec_tile && z >= sh.rbz0 && z <= sh.rbz1) {
-      const int2 rr = bin_range(sh, z, x);
-      for (int k = rr.x; k < rr.y; ++k) {
-        const int r = sh.blk_rec[k];
-        if (sh.rec_z[r] == z && sh.rec_x[r] == x)
-          sh.data[static_cast<size_t>(r) * sh.nSteps + it + 1] = szz + 3.0f * sxx;
-      }
-    }
+    if (rec_tile) record(sh, it, first_receiver(sh, z, x), z, x, szz, sxx);
   };
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -637,19 +569,8 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   const float bA = p_bA[r], bB = p_bB[r], amu = p_amu[r], lam = p_lam[r], l2m = p_l2m[r];
   float vz = p_vz[r], vx = p_vx[r];
   const bool dom = in_box(z, x, g.zs0, g.zs1, g.xs0, g.xs1);
-  bool injected = false;
-  if (rec_tile && z >= sh.rbz0 && z <= sh.rbz1) {
-    const int2 rr = bin_range(sh, z, x);
-    for (int k = rr.x; k < rr.y; ++k) {
-      const int r = sh.blk_rec[k];
-      if (sh.rec_z[r] == z && sh.rec_x[r] == x) {
-        const float rv = sh.res[static_cast<size_t>(r) * sh.nSteps + it];
-        sa += rv;
-        xa += 3.0f * rv;
-        injected = true;
-      }
-    }
-  }
+  const int rec = rec_tile ? first_receiver(sh, z, x) : -1;
+  inject_res(sh, it, rec, z, x, sa, xa);
   if (dom) {
     {
       const float dvz_dx = -sdp(s_vz_a, b, BOXZ, g.rdx);
@@ -679,7 +600,7 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
     if (xb) f.m_dvx_dx[i] = c.b_x[x] * f.m_dvx_dx[i] + lam * sa * dt + l2m * xa * dt;
     if (zb) f.m_dvz_dz[i] = c.b_z[z] * f.m_dvz_dz[i] + l2m * sa * dt + lam * xa * dt;
   }
-  if (dom || injected) {
+  if (dom || rec >= 0) {
     f.szz_a[i] = sa;
     f.sxx_a[i] = xa;
   }
@@ -786,14 +707,7 @@ __device__ __forceinline__ void fwd_stress_fast1(const SweepPack<K>& P, int shot
       szz += sh.src_szz[it];
       sxx += sh.src_sxx[it];
     }
-    if (z >= sh.rbz0 && z <= sh.rbz1) {
-      const int2 rr = bin_range(sh, z, x);
-      for (int k = rr.x; k < rr.y; ++k) {
-        const int r = sh.blk_rec[k];
-        if (sh.rec_z[r] == z && sh.rec_x[r] == x)
-          sh.data[static_cast<size_t>(r) * sh.nSteps + it + 1] = szz + 3.0f * sxx;
-      }
-    }
+    record(sh, it, first_receiver(sh, z, x), z, x, szz, sxx);
   }
   f.szz[i] = szz;
   f.sxx[i] = sxx;
@@ -879,13 +793,7 @@ __device__ __forceinline__ void fwd_stress_fast2(const SweepPack<K>& P, int shot
         *szr[r] += sh.src_szz[it];
         *sxr[r] += sh.src_sxx[it];
       }
-      if (zr < sh.rbz0 || zr > sh.rbz1) continue;
-      const int2 rr = bin_range(sh, zr, x);
-      for (int k = rr.x; k < rr.y; ++k) {
-        const int q = sh.blk_rec[k];
-        if (sh.rec_z[q] == zr && sh.rec_x[q] == x)
-          sh.data[static_cast<size_t>(q) * sh.nSteps + it + 1] = *szr[r] + 3.0f * *sxr[r];
-      }
+      record(sh, it, first_receiver(sh, zr, x), zr, x, *szr[r], *sxr[r]);
     }
   }
   st2(f.szz + i, szz0, szz1);
@@ -1142,17 +1050,7 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
   const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    if (special && z + r >= sh.rbz0 && z + r <= sh.rbz1) {
-      const int2 rr = bin_range(sh, z + r, x);
-      for (int k = rr.x; k < rr.y; ++k) {
-        const int q = sh.blk_rec[k];
-        if (sh.rec_z[q] == z + r && sh.rec_x[q] == x) {
-          const float rv = sh.res[static_cast<size_t>(q) * sh.nSteps + it];
-          sa[r] += rv;
-          xa[r] += 3.0f * rv;
-        }
-      }
-    }
+    if (special) inject_res(sh, it, first_receiver(sh, z + r, x), z + r, x, sa[r], xa[r]);
   }
   {
     float d1[R], d2[R], d3[R], d4[R];
