@@ -50,6 +50,8 @@ SIGNATURES = {
     "fwigb_cufd": ([_D, _D, _D, _D, _D, _D, _D, _D, _D, ctypes.c_int, ctypes.c_int, ctypes.c_int, _I,
                     ctypes.c_char_p], ctypes.c_int),
     "fwigb_set_model": ([_V, _D, _D, _D], ctypes.c_int),
+    "fwigb_set_model_vp": ([_V, _D, _D, _D, ctypes.c_double, ctypes.c_double], ctypes.c_int),
+    "fwigb_fetch_vp_gradient": ([_V, _D], ctypes.c_int),
     "fwigb_stage_shots": ([_V, _D, ctypes.c_int, _I, ctypes.c_int, ctypes.c_int, _F], ctypes.c_int),
     "fwigb_run": ([_V, ctypes.c_int], ctypes.c_int),
     "fwigb_fetch": ([_V, _D, _D, _D, _D, _D, _F], ctypes.c_int),

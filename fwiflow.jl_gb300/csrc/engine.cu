@@ -483,6 +483,8 @@ struct fwigb_ctx {
   bool illum = false;       // accumulate the source illumination in the runs
   bool illum_valid = false; // the last run accumulated it
   bool model_set = false;
+  DevBuf vp;                // the Vp of a fwigb_set_model_vp model and its mask (row-major doubles)
+  bool vp_model = false, vp_masked = false;
   int last_calc = -1;
   long long launches = 0;
   int tx[4] = {8, 8, 8, 8};    // tile width per sweep (F1, F2, B, C)
@@ -692,26 +694,14 @@ int open_ctx(const char* para_fname, int device, fwigb_ctx* ctx) {
 // context) persist and are still reported by the next call that fails.
 void clear_stale_error() { cudaGetLastError(); }
 
-int set_model(fwigb_ctx* ctx, const double* lam, const double* mu, const double* den) {
-  if (!lam || !mu || !den) {
-    ctx->err = "null model array";
-    return FWIGB_ERR_ARG;
-  }
-  CK(cudaSetDevice(ctx->device));
-  clear_stale_error();
-  const size_t nh = ctx->ncell, n = ctx->cells;
-  const int ldz = ctx->geo.ldz;
-  double* st = ctx->stage.as<double>();
-  CK(cudaMemcpyAsync(st, lam, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(st + nh, mu, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(st + 2 * nh, den, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-  unsigned* cpbits = reinterpret_cast<unsigned*>(ctx->scal.as<char>() + 8);
-  CK(cudaMemsetAsync(cpbits, 0, sizeof(unsigned), ctx->stream));
+// Finishes a model whose lambda, mu and density are in the media buffer:
+// derived media and the Courant check.
+int finish_model(fwigb_ctx* ctx) {
+  const size_t n = ctx->cells;
+  const unsigned* cpbits = reinterpret_cast<unsigned*>(ctx->scal.as<char>() + 8);
   float* b = ctx->media.as<float>();
-  launch_media_from_rowmajor(ctx->stream, ctx->p.nz, ctx->p.nx, ldz, st, st + nh, st + 2 * nh, b, b + n, b + 2 * n,
-                             cpbits);
-  launch_media_derived(ctx->stream, ctx->p.nz, ctx->p.nx, ldz, b, b + n, b + 2 * n, b + 3 * n, b + 4 * n, b + 5 * n,
-                       b + 6 * n, b + 7 * n, b + 8 * n);
+  launch_media_derived(ctx->stream, ctx->p.nz, ctx->p.nx, ctx->geo.ldz, b, b + n, b + 2 * n, b + 3 * n, b + 4 * n,
+                       b + 5 * n, b + 6 * n, b + 7 * n, b + 8 * n);
   CK(cudaGetLastError());
   unsigned bits = 0;
   CK(cudaMemcpyAsync(&bits, cpbits, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
@@ -729,6 +719,55 @@ int set_model(fwigb_ctx* ctx, const double* lam, const double* mu, const double*
     return FWIGB_ERR_COURANT;
   }
   ctx->model_set = true;
+  return FWIGB_OK;
+}
+
+int set_model(fwigb_ctx* ctx, const double* lam, const double* mu, const double* den) {
+  if (!lam || !mu || !den) {
+    ctx->err = "null model array";
+    return FWIGB_ERR_ARG;
+  }
+  CK(cudaSetDevice(ctx->device));
+  clear_stale_error();
+  ctx->vp_model = false;
+  const size_t nh = ctx->ncell, n = ctx->cells;
+  double* st = ctx->stage.as<double>();
+  CK(cudaMemcpyAsync(st, lam, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(st + nh, mu, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(st + 2 * nh, den, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  unsigned* cpbits = reinterpret_cast<unsigned*>(ctx->scal.as<char>() + 8);
+  CK(cudaMemsetAsync(cpbits, 0, sizeof(unsigned), ctx->stream));
+  float* b = ctx->media.as<float>();
+  launch_media_from_rowmajor(ctx->stream, ctx->p.nz, ctx->p.nx, ctx->geo.ldz, st, st + nh, st + 2 * nh, b, b + n,
+                             b + 2 * n, cpbits);
+  return finish_model(ctx);
+}
+
+// A Vp model (k_media_from_vp); v and mask stay on the device for
+// fetch_vp_gradient, until the next model.
+int set_model_vp(fwigb_ctx* ctx, const double* vp, const double* vp0, const double* mask, double vmin, double vmax) {
+  if (!vp || (vp0 && !mask)) {
+    ctx->err = "null model array";
+    return FWIGB_ERR_ARG;
+  }
+  CK(cudaSetDevice(ctx->device));
+  clear_stale_error();
+  ctx->vp_model = false;
+  const size_t nh = ctx->ncell, n = ctx->cells;
+  CK(ctx->vp.ensure(2 * nh * sizeof(double)));
+  double* st = ctx->stage.as<double>();
+  double *v = ctx->vp.as<double>(), *m = ctx->vp.as<double>(nh);
+  CK(cudaMemcpyAsync(st, vp, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  if (vp0) CK(cudaMemcpyAsync(st + nh, vp0, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  if (mask) CK(cudaMemcpyAsync(m, mask, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  unsigned* cpbits = reinterpret_cast<unsigned*>(ctx->scal.as<char>() + 8);
+  CK(cudaMemsetAsync(cpbits, 0, sizeof(unsigned), ctx->stream));
+  float* b = ctx->media.as<float>();
+  launch_media_from_vp(ctx->stream, ctx->p.nz, ctx->p.nx, ctx->geo.ldz, st, vp0 ? st + nh : nullptr, m, vmin, vmax, v,
+                       b, b + n, b + 2 * n, cpbits);
+  TRY_RC(finish_model(ctx));
+  ctx->vp_model = true;
+  ctx->vp_masked = mask != nullptr;
   return FWIGB_OK;
 }
 
@@ -1755,7 +1794,7 @@ int fwigb_destroy(fwigb_ctx* ctx) {
                     &ctx->shot_supd, &ctx->supd_part, &ctx->supd_coef, &ctx->supd_k,
                     &ctx->g_fields,
                     &ctx->g_store, &ctx->g_grads,
-                    &ctx->g_slots, &ctx->march_flags})
+                    &ctx->g_slots, &ctx->march_flags, &ctx->vp})
     b->release();
   for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
@@ -1801,6 +1840,31 @@ int fwigb_set_model(fwigb_ctx* ctx, const double* lambda, const double* mu, cons
   if (!ctx) return FWIGB_ERR_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
   return set_model(ctx, lambda, mu, den);
+}
+
+int fwigb_set_model_vp(fwigb_ctx* ctx, const double* vp, const double* vp0, const double* mask, double vmin,
+                       double vmax) {
+  if (!ctx) return FWIGB_ERR_ARG;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  return set_model_vp(ctx, vp, vp0, mask, vmin, vmax);
+}
+
+int fwigb_fetch_vp_gradient(fwigb_ctx* ctx, double* g_vp) {
+  if (!ctx || !g_vp) return FWIGB_ERR_ARG;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  if (!ctx->vp_model || ctx->last_calc != 1) {
+    ctx->err = "the Vp gradient needs a Vp model (fwigb_set_model_vp) and a run with gradients";
+    return FWIGB_ERR_ARG;
+  }
+  CK(cudaSetDevice(ctx->device));
+  const size_t n = ctx->cells;
+  const float* g = ctx->grads.as<float>();
+  double* st = ctx->stage.as<double>();
+  launch_vp_gradient(ctx->stream, ctx->p.nz, ctx->p.nx, ctx->geo.ldz, ctx->vp.as<double>(),
+                     ctx->vp_masked ? ctx->vp.as<double>(ctx->ncell) : nullptr, g, g + n, g + 2 * n, st);
+  CK(cudaMemcpyAsync(g_vp, st, ctx->ncell * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return FWIGB_OK;
 }
 
 int fwigb_stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* shot_ids, int n_shots,

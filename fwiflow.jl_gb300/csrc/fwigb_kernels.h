@@ -257,6 +257,12 @@ void launch_reduce_grads(cudaStream_t s, int nz, int nx, int ldz, int nshots, co
 // cpmax_bits receives atomicMax of the P velocity's float bits.
 void launch_media_from_rowmajor(cudaStream_t s, int nz, int nx, int ldz, const double* lam_mpa, const double* mu_mpa,
                                 const double* den, float* lam, float* mu, float* den_f, unsigned* cpmax_bits);
+// The same from a Vp model (k_media_from_vp), and its gradient (k_vp_gradient).
+void launch_media_from_vp(cudaStream_t s, int nz, int nx, int ldz, const double* vp, const double* vp0,
+                          const double* mask, double vmin, double vmax, double* v, float* lam, float* mu, float* den,
+                          unsigned* cpmax_bits);
+void launch_vp_gradient(cudaStream_t s, int nz, int nx, int ldz, const double* v, const double* mask,
+                        const float* g_lam, const float* g_mu, const float* g_den, double* out);
 void launch_media_derived(cudaStream_t s, int nz, int nx, int ldz, const float* lam, const float* mu,
                           const float* den, float* l2m, float* aveMu, float* bycA, float* bycB, float* hs,
                           float* muw);

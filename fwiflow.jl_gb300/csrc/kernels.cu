@@ -1227,6 +1227,83 @@ __global__ void k_media_from_rowmajor(int nz, int nx, int ldz, const double* __r
   atomicMax(cpmax_bits, __float_as_uint(cpmax));
 }
 
+// The media of a Vp model with Vs = Vp / sqrt(3) and Gardner's density
+// rho = 310 Vp^(1/4), formed in double as velocity_to_moduli does
+// (src/Utils.jl:221-227): Vp = vp0 (1 - mask) + vp mask within [vmin, vmax] (vp
+// itself when vp0 is null), row-major, kept in v. On the host these were a
+// dozen passes and two pow per cell, half the time of a gradient call on the
+// largest grid: 57 of 284 ms on 1120 x 3152 cells. Bound by the uploads of its
+// three inputs, as k_media_from_rowmajor.
+__global__ void k_media_from_vp(int nz, int nx, int ldz, const double* __restrict__ vp, const double* __restrict__ vp0,
+                                const double* __restrict__ mask, double vmin, double vmax, double* __restrict__ v,
+                                float* lam, float* mu, float* den, unsigned* cpmax_bits) {
+  __shared__ float tl[kT][kT + 1], tm[kT][kT + 1], td[kT][kT + 1];
+  const int x0 = blockIdx.x * kT, z0 = blockIdx.y * kT;
+  for (int r = threadIdx.y; r < kT; r += blockDim.y) {
+    const int z = z0 + r, x = x0 + threadIdx.x;
+    if (z < nz && x < nx) {
+      const size_t s = static_cast<size_t>(z) * nx + x;
+      double c = vp[s];
+      if (vp0) {
+        c = __dadd_rn(__dmul_rn(vp0[s], 1.0 - mask[s]), __dmul_rn(c, mask[s]));
+        c = c < vmin ? vmin : (c > vmax ? vmax : c);  // (a NaN stays one)
+      }
+      v[s] = c;
+      const double cs = c / 1.7320508075688772, rho = 310.0 * sqrt(sqrt(c));
+      const double cs2 = __dmul_rn(cs, cs);
+      const double l = __dadd_rn(__dmul_rn(c, c), -2.0 * cs2) * rho / 1e6, u = cs2 * rho / 1e6;
+      tl[r][threadIdx.x] = static_cast<float>(l * 1e6);
+      tm[r][threadIdx.x] = static_cast<float>(u * 1e6);
+      td[r][threadIdx.x] = static_cast<float>(rho);
+    }
+  }
+  __syncthreads();
+  float cpmax = 0.0f;
+  for (int r = threadIdx.y; r < kT; r += blockDim.y) {
+    const int x = x0 + r, z = z0 + threadIdx.x;
+    if (z < nz && x < nx) {
+      const size_t d = static_cast<size_t>(x) * ldz + z;
+      const float l = tl[threadIdx.x][r], u = tm[threadIdx.x][r], rho = td[threadIdx.x][r];
+      lam[d] = l;
+      mu[d] = u;
+      den[d] = rho;
+      const float cp = static_cast<float>(sqrt((l + 2.0 * u) / rho));  // velInit (utilities.cu:119-121)
+      cpmax = fmaxf(cpmax, cp);
+    }
+  }
+  atomicMax(cpmax_bits, __float_as_uint(cpmax));  // (see k_media_from_rowmajor)
+}
+
+// dJ/dVp of that model, row-major: the chain rule of lambda = mu = rho Vp^2 /
+// 3e6 MPa and rho = 310 Vp^(1/4) on the column-major gradients, times mask
+// (when not null). The host's form took 95 of 284 ms on 1120 x 3152 cells.
+__global__ void k_vp_gradient(int nz, int nx, int ldz, const double* __restrict__ v, const double* __restrict__ mask,
+                              const float* __restrict__ g_lam, const float* __restrict__ g_mu,
+                              const float* __restrict__ g_den, double* __restrict__ out) {
+  __shared__ double tm[kT][kT + 1];
+  __shared__ float td[kT][kT + 1];
+  const int z0 = blockIdx.x * kT, x0 = blockIdx.y * kT;
+  for (int r = threadIdx.y; r < kT; r += blockDim.y) {
+    const int x = x0 + r, z = z0 + threadIdx.x;
+    if (z < nz && x < nx) {
+      const size_t i = static_cast<size_t>(x) * ldz + z;
+      tm[r][threadIdx.x] = static_cast<double>(g_lam[i]) + static_cast<double>(g_mu[i]);
+      td[r][threadIdx.x] = g_den[i];
+    }
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < kT; r += blockDim.y) {
+    const int z = z0 + r, x = x0 + threadIdx.x;
+    if (z < nz && x < nx) {
+      const size_t i = static_cast<size_t>(z) * nx + x;
+      const double c = v[i], q = sqrt(sqrt(c)), rho = 310.0 * q, drho = 77.5 / (q * q * q);
+      const double dmod = (drho * c * c + 2.0 * rho * c) / 3e6;
+      const double g = tm[threadIdx.x][r] * dmod + static_cast<double>(td[threadIdx.x][r]) * drho;
+      out[i] = mask ? g * mask[i] : g;
+    }
+  }
+}
+
 // aveMuInit / aveBycInit (utilities.cu:125-152) plus the terms of the fused
 // imaging sweeps.
 __global__ void k_media_derived(int nz, int nx, int ldz, const float* __restrict__ lam,
@@ -1747,6 +1824,19 @@ void launch_media_from_rowmajor(cudaStream_t s, int nz, int nx, int ldz, const d
                                 const double* den, float* lam, float* mu, float* den_f, unsigned* cpmax_bits) {
   dim3 grid((nx + kT - 1) / kT, (nz + kT - 1) / kT);
   k_media_from_rowmajor<<<grid, dim3(kT, 8), 0, s>>>(nz, nx, ldz, lam_mpa, mu_mpa, den, lam, mu, den_f, cpmax_bits);
+}
+
+void launch_media_from_vp(cudaStream_t s, int nz, int nx, int ldz, const double* vp, const double* vp0,
+                          const double* mask, double vmin, double vmax, double* v, float* lam, float* mu, float* den,
+                          unsigned* cpmax_bits) {
+  dim3 grid((nx + kT - 1) / kT, (nz + kT - 1) / kT);
+  k_media_from_vp<<<grid, dim3(kT, 8), 0, s>>>(nz, nx, ldz, vp, vp0, mask, vmin, vmax, v, lam, mu, den, cpmax_bits);
+}
+
+void launch_vp_gradient(cudaStream_t s, int nz, int nx, int ldz, const double* v, const double* mask,
+                        const float* g_lam, const float* g_mu, const float* g_den, double* out) {
+  dim3 grid((nz + kT - 1) / kT, (nx + kT - 1) / kT);
+  k_vp_gradient<<<grid, dim3(kT, 8), 0, s>>>(nz, nx, ldz, v, mask, g_lam, g_mu, g_den, out);
 }
 
 void launch_media_derived(cudaStream_t s, int nz, int nx, int ldz, const float* lam, const float* mu,

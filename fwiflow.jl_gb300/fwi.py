@@ -151,6 +151,23 @@ class FwiContext:
         lam, mu, den = self._model(lam, mu, den)
         _lib.check(self._lib.fwigb_set_model(self._h, _lib.dptr(lam), _lib.dptr(mu), _lib.dptr(den)), self._h)
 
+    def set_model_vp(self, vp, vp0=None, mask=None, vmin: float = 0.0, vmax: float = np.inf) -> None:
+        """Model from a P velocity with Vs = Vp / sqrt(3) and Gardner density,
+        formed on the device: vp0 (1 - mask) + vp mask within [vmin, vmax], or
+        vp itself without vp0."""
+        shape = (self.nz, self.nx)
+        a = [None if v is None else np.ascontiguousarray(np.broadcast_to(np.asarray(v, dtype=np.float64), shape))
+             for v in (vp, vp0, mask)]
+        _lib.check(self._lib.fwigb_set_model_vp(self._h, *(_lib.dptr(v) for v in a), float(vmin), float(vmax)),
+                   self._h)
+
+    def vp_gradient(self) -> np.ndarray:
+        """dJ/dVp of the last run with gradients under a set_model_vp model,
+        times its mask, [nz][nx] float64."""
+        out = np.empty((self.nz, self.nx))
+        _lib.check(self._lib.fwigb_fetch_vp_gradient(self._h, _lib.dptr(out)), self._h)
+        return out
+
     def stage_shots(self, stf, shot_ids, obs: Optional[Sequence[np.ndarray]] = None, with_obs: bool = True) -> None:
         stf, ids = self._stf_ids(stf, shot_ids)
         blk = self._obs_block(obs, ids) if obs is not None else None
@@ -165,7 +182,7 @@ class FwiContext:
         out = np.zeros(1)
         gl = gm = gd = gs = None
         if grads:
-            gl, gm, gd = (np.zeros((self.nz, self.nx)) for _ in range(3))
+            gl, gm, gd = (np.empty((self.nz, self.nx)) for _ in range(3))  # (fetch fills them)
             gs = np.zeros((n_shots, self.nSteps))
         _lib.check(self._lib.fwigb_fetch(self._h, _lib.dptr(out) if misfit else None, _lib.dptr(gl), _lib.dptr(gm),
                                          _lib.dptr(gd), _lib.dptr(gs), None), self._h)

@@ -95,23 +95,32 @@ class VpProblem:
         v = self.full(vp)
         return float(np.linalg.norm(v[m] - self.vp_true[m]) / np.linalg.norm(self.vp_true[m]))
 
+    def _set_model(self, vp) -> bool:
+        """The model moduli_of_vp(self.full(vp)); formed on the device (True) when the limits are numbers."""
+        on_device = np.isscalar(self.vmin) and np.isscalar(self.vmax)
+        if on_device:
+            self.ctx.set_model_vp(vp, self.vp0, self.mask, self.vmin, self.vmax)
+        else:
+            self.ctx.set_model(*moduli_of_vp(self.full(vp)))
+        return on_device
+
     def misfit(self, vp) -> float:
-        self.ctx.set_model(*moduli_of_vp(self.full(vp)))
+        self._set_model(vp)
         self.ctx.run(0)
         self.evals += 1
         return self.ctx.fetch(misfit=True)[0]
 
     def misfit_grad(self, vp, illumination: bool = False):
         """(misfit, dJ/dVp masked, (g_lambda, g_mu, g_den), illumination or None)."""
-        v = self.full(vp)
         self.ctx.set_illumination(illumination)
-        self.ctx.set_model(*moduli_of_vp(v))
+        on_device = self._set_model(vp)
         self.ctx.run(1)
         J, gl, gm, gd, _ = self.ctx.fetch(misfit=True, grads=True, n_shots=self.n_shots)
         illum = self.ctx.illumination() if illumination else None
         self.ctx.set_illumination(False)
         self.evals += 1
-        return J, chain_to_vp(v, gl, gm, gd) * self.mask, (gl, gm, gd), illum
+        g = self.ctx.vp_gradient() if on_device else chain_to_vp(self.full(vp), gl, gm, gd) * self.mask
+        return J, g, (gl, gm, gd), illum
 
 
 def _line_search(problem: VpProblem, vp, J, d, step: float):

@@ -117,6 +117,16 @@ int fwigb_cufd(double *misfit, double *grad_Lambda, double *grad_Mu, double *gra
  * staggered media and checks the Courant number (libCUFD.cu:67-96). */
 int fwigb_set_model(fwigb_ctx *ctx, const double *lambda, const double *mu, const double *den);
 
+/* Model from a P velocity (row-major double [nz][nx], m/s) with Vs = Vp /
+ * sqrt(3) and rho = 310 Vp^(1/4): Vp = vp0 (1 - mask) + vp mask, limited to
+ * [vmin, vmax], or vp itself when vp0 is NULL. As fwigb_set_model otherwise. */
+int fwigb_set_model_vp(fwigb_ctx *ctx, const double *vp, const double *vp0, const double *mask, double vmin,
+                       double vmax);
+
+/* dJ/dVp [nz][nx] of the last run with gradients under that model, times the
+ * model's mask (if any). */
+int fwigb_fetch_vp_gradient(fwigb_ctx *ctx, double *g_vp);
+
 /* Stages the shots of a call: source rows of stf, receivers, and (when
  * with_obs) observed data, from `obs` ([n_shots][nrec_max][nSteps] float, may
  * be NULL) or else from data_dir_name/Shot<id>.bin. */
