@@ -88,6 +88,11 @@ SIGNATURES = {
                         ctypes.c_float, ctypes.c_int, _V], ctypes.c_int),
     "fwigb_cnn_pack_weights": ([_V, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _V, _V],
                                ctypes.c_int),
+    "fwigb_cnn_pack_image": ([_V, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _V, _V],
+                             ctypes.c_int),
+    "fwigb_cnn_feature_scratch": ([], ctypes.c_int),
+    "fwigb_cnn_features": ([_V, _V, _V, _V, _V, ctypes.c_int, ctypes.c_int, _V, _V, _V], ctypes.c_int),
+    "fwigb_cnn_apply_gain": ([_V, _V, _V, _V, _V, ctypes.c_int, ctypes.c_int, _V, _V], ctypes.c_int),
     "fwigb_cnn_mse_grad": ([_V, _V, _V, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_float, _V, _V, _V],
                            ctypes.c_int),
     "fwigb_set_tile_config": ([_V, _I], ctypes.c_int),

@@ -160,10 +160,33 @@ class CnnPreconditioner:
         if rc != 0:
             raise _lib.FwiError(rc, "CNN kernel launch failed")
 
+    def _upload(self, *arrays):
+        """Model-shaped arrays as one device tensor (len(arrays), Hz, Wx) of doubles."""
+        torch = _torch()
+        out = torch.empty((len(arrays), self.Hz, self.Wx), dtype=torch.float64, device=self.dev)
+        for k, a in enumerate(arrays):
+            a = np.ascontiguousarray(a, dtype=np.float64)
+            if a.shape != (self.Hz, self.Wx) or not a.flags.writeable:  # (torch warns of read-only arrays)
+                a = np.array(np.broadcast_to(a, (self.Hz, self.Wx)))
+            out[k].copy_(torch.from_numpy(a))
+        return out
+
+    def _pack(self, chans, c_pad: int, out) -> None:
+        """(C, nz, nx) arrays into the image tensor `out` (FP32 or BF16)."""
+        torch = _torch()
+        if len(chans) > c_pad:
+            raise ValueError(f"{len(chans)} channels do not fit an image of {c_pad}")
+        self._ck(self.lib.fwigb_cnn_pack_image(self._p(self._upload(*chans)), len(chans), self.Hz, self.Wx, c_pad,
+                                               int(out.dtype == torch.bfloat16), self._p(out), self._s()))
+
     def to_image(self, chans: np.ndarray, c_pad: int, dtype):
         """(C, nz, nx) numpy -> device [npix][c_pad] in the kernels' layout."""
         torch = _torch()
         c = chans.shape[0]
+        if dtype in (torch.float32, torch.bfloat16) and 1 <= c <= c_pad <= 16:
+            out = torch.empty((self.npix, c_pad), dtype=dtype, device=self.dev)
+            self._pack(chans, c_pad, out)
+            return out
         a = np.zeros((self.Wx, self.Hz, c_pad), dtype=np.float32)
         a[:, :, :c] = np.transpose(chans, (2, 1, 0))
         return torch.from_numpy(a.reshape(self.npix, c_pad)).to(device=self.dev, dtype=dtype)
@@ -263,12 +286,11 @@ class CnnPreconditioner:
 
     # -- data
     def stage(self, feats: np.ndarray, target: Optional[np.ndarray] = None, mask: Optional[np.ndarray] = None):
-        torch = _torch()
-        self.x0.copy_(self.to_image(feats, 16, torch.bfloat16))
+        self._pack(feats, 16, self.x0)
         if target is not None:
-            self.target.copy_(self.to_image(target, N_OUT, torch.float32))
+            self._pack(target, N_OUT, self.target)
         if mask is not None:
-            self.mask.copy_(torch.from_numpy(np.ascontiguousarray(mask.T.reshape(-1), dtype=np.float32)).to(self.dev))
+            self._pack([mask], 1, self.mask)
 
     def train(self, samples: Sequence[tuple], epochs: int, lr: float = 1e-3, seed: int = 0,
               log: Optional[List[float]] = None) -> List[float]:
@@ -306,9 +328,15 @@ class CnnPreconditioner:
     def precondition(self, g_lambda, g_mu, g_den, illum, mask) -> np.ndarray:
         """Preconditioned lambda / mu / rho gradients (3, nz, nx): each
         gradient times exp of its predicted log-gain, zero outside the mask."""
-        out = self.predict(features(g_lambda, g_mu, g_den, illum, mask))
-        gain = np.exp(np.clip(out, -30.0, 5.0))
-        return np.stack([g_lambda, g_mu, g_den]) * gain * mask
+        torch = _torch()
+        a = self._upload(g_lambda, g_mu, g_den, illum, mask)
+        g, (e, m) = [self._p(v) for v in a[:3]], (self._p(v) for v in a[3:])
+        scratch = torch.empty(self.lib.fwigb_cnn_feature_scratch(), dtype=torch.float64, device=self.dev)
+        s = self._s()
+        self._ck(self.lib.fwigb_cnn_features(*g, e, m, self.Hz, self.Wx, self._p(scratch), self._p(self.x0), s))
+        out = torch.empty((3, self.Hz, self.Wx), dtype=torch.float64, device=self.dev)
+        self._ck(self.lib.fwigb_cnn_apply_gain(self._p(self.forward()), *g, m, self.Hz, self.Wx, self._p(out), s))
+        return out.cpu().numpy()
 
     def state(self) -> dict:
         return {f"W{k}": self.W[k].cpu().numpy() for k in range(DEPTH)} | \

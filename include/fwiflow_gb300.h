@@ -297,6 +297,21 @@ int fwigb_cnn_adam(float *w, const float *grad, float *m1, float *m2, int n, flo
  * gradient: W'[tap][co][ci] = W[8 - tap][ci][co]. */
 int fwigb_cnn_pack_weights(const float *w, int cin, int cout, int cin_pad, int cout_pad, int transposed, void *frag,
                            void *stream);
+/* Model-shaped arrays (row-major double [c][nz][nx], on the device) to an
+ * image: out[x * nz + z][c_pad] in FP32, rounded to BF16 when bf16; channels
+ * past c are zero. c_pad at most 16. */
+int fwigb_cnn_pack_image(const double *chans, int c, int nz, int nx, int c_pad, int bf16, void *out, void *stream);
+/* The network's 16-channel BF16 input of an FWI iteration: the gradients in
+ * units of their RMS where mask > 0, the illumination over its maximum there,
+ * and its log10 on [0, 1]. Device arrays as above; scratch holds
+ * fwigb_cnn_feature_scratch() doubles. */
+int fwigb_cnn_feature_scratch(void);
+int fwigb_cnn_features(const double *g_lambda, const double *g_mu, const double *g_den, const double *illum,
+                       const double *mask, int nz, int nx, double *scratch, void *x_bf16, void *stream);
+/* result[c][nz][nx] = g_c exp(y_c within [-30, 5]) mask for the network's
+ * output y (FP32 [pixel][16]). */
+int fwigb_cnn_apply_gain(const float *y, const double *g_lambda, const double *g_mu, const double *g_den,
+                         const double *mask, int nz, int nx, double *result, void *stream);
 /* Masked MSE of the first nc channels of y (FP32 [npix][c_pad]) against
  * target (FP32 [npix][nc]): per-256-pixel partial loss sums, and
  * dy = 2 (y - target) mask * inv_count as BF16 [npix][c_pad]. c_pad = 16. */
