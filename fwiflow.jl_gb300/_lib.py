@@ -82,6 +82,8 @@ SIGNATURES = {
                                    _V], ctypes.c_int),
     "fwigb_cnn_wgrad_partials": ([_V, _V, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _V, _V],
                                  ctypes.c_int),
+    "fwigb_cnn_wgrad_blocks": ([ctypes.c_int, ctypes.c_int], ctypes.c_int),
+    "fwigb_cnn_wgrad": ([_V, _V, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _V, _V, _V], ctypes.c_int),
     "fwigb_cnn_reduce_partials": ([_V, ctypes.c_int, ctypes.c_int, _V, _V], ctypes.c_int),
     "fwigb_cnn_bias_partials": ([_V, ctypes.c_longlong, ctypes.c_int, ctypes.c_int, _V, _V], ctypes.c_int),
     "fwigb_cnn_adam": ([_V, _V, _V, _V, ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float,

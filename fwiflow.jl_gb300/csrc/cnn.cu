@@ -485,11 +485,15 @@ __global__ void k_pack_weights_tc(const float* __restrict__ w, int cin, int cout
   out[u] = make_uint4(h[0], h[1], h[2], h[3]);
 }
 
-// Weight gradient partials. One block (9 warps, warp = tap) per 32 x 8 pixel
-// tile: dW_tap[ci][co] += sum over the tile's pixels p of X(p + off_tap)[ci] *
-// dZ(p)[co], as a GEMM with K = pixels: A = X_tap^T and B = dZ, both read
-// pixel-major from shared memory with ldmatrix.trans. Writes the block's
-// partial [9][CIN][COUT] (FP32) to part + block * 9*CIN*COUT.
+// Weight gradient partials. A block (9 warps, warp = tap) takes every
+// gridDim.x-th 32 x 8 pixel tile: dW_tap[ci][co] += sum over the tile's pixels
+// p of X(p + off_tap)[ci] * dZ(p)[co], as a GEMM with K = pixels: A = X_tap^T
+// and B = dZ, both read pixel-major from shared memory with ldmatrix.trans,
+// the accumulators staying in registers from tile to tile. Writes the block's
+// partial [9][CIN][COUT] (FP32) to part + block * 9*CIN*COUT. (A partial per
+// tile is 36 KB written and read again for 48 KB of input. With four blocks per
+// SM instead, 608 x 1600 pixels, 32 -> 32 channels: 91 -> 68 us, and 608
+// partials to sum instead of 3800.)
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(288) k_conv3x3_wgrad(const __nv_bfloat16* __restrict__ x_in,
                                                        const __nv_bfloat16* __restrict__ dz, int Hz, int Wx,
@@ -498,20 +502,6 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad(const __nv_bfloat16* __re
   constexpr int MT = CIN / 16, NT = COUT / 8;
   __shared__ __align__(16) __nv_bfloat16 s_x[kHz * kHx * CSX];
   __shared__ __align__(16) __nv_bfloat16 s_dz[kTz * kTx * CSZ];
-  const int z0 = blockIdx.x * kTz, x0 = blockIdx.y * kTx;
-  load_tile<CIN>(x_in, Hz, Wx, z0, x0, s_x);
-  {
-    constexpr int CH = COUT / 8;
-    for (int k = threadIdx.x; k < kTz * kTx * CH; k += blockDim.x) {
-      const int ch = k % CH, pix = k / CH;
-      const int zz = pix % kTz, xx = pix / kTz;
-      const int x = x0 + xx;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (x < Wx) v = *reinterpret_cast<const uint4*>(dz + (static_cast<size_t>(x) * Hz + z0 + zz) * COUT + ch * 8);
-      *reinterpret_cast<uint4*>(s_dz + pix * CSZ + ch * 8) = v;
-    }
-  }
-  __syncthreads();
   const int tap = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ky = tap / 3, kx = tap % 3;
   const int g = lane >> 2, t = lane & 3, q = lane >> 3, r8 = lane & 7;
@@ -526,25 +516,40 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad(const __nv_bfloat16* __re
   const int a_px = (q >> 1) * 8 + r8, a_c = (q & 1) * 8;
   // B fragment rows: pixel (q & 1) * 8 + r8, channel offset (q >> 1) * 8.
   const int b_px = (q & 1) * 8 + r8, b_c = (q >> 1) * 8;
-  for (int s = 0; s < kTz * kTx / 16; ++s) {  // 16 pixels per k-step: half a column
-    const int xx = s >> 1, zz0 = (s & 1) * 16;
-    unsigned a[MT][4];
+  const int ntz = Hz / kTz, ntiles = ntz * ((Wx + kTx - 1) / kTx);
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int z0 = (tile % ntz) * kTz, x0 = (tile / ntz) * kTx;
+    if (tile != static_cast<int>(blockIdx.x)) __syncthreads();  // the last tile has been read
+    load_tile<CIN>(x_in, Hz, Wx, z0, x0, s_x);
+    constexpr int CH = COUT / 8;
+    for (int k = threadIdx.x; k < kTz * kTx * CH; k += blockDim.x) {
+      const int ch = k % CH, pix = k / CH;
+      const int zz = pix % kTz, xx = pix / kTz;
+      const int x = x0 + xx;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (x < Wx) v = *reinterpret_cast<const uint4*>(dz + (static_cast<size_t>(x) * Hz + z0 + zz) * COUT + ch * 8);
+      *reinterpret_cast<uint4*>(s_dz + pix * CSZ + ch * 8) = v;
+    }
+    __syncthreads();
+    for (int s = 0; s < kTz * kTx / 16; ++s) {  // 16 pixels per k-step: half a column
+      const int xx = s >> 1, zz0 = (s & 1) * 16;
+      unsigned a[MT][4];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
-      ldmatrix_x4_trans(a[m], s_x + ((xx + kx) * kHz + zz0 + a_px + ky) * CSX + m * 16 + a_c);
+      for (int m = 0; m < MT; ++m)
+        ldmatrix_x4_trans(a[m], s_x + ((xx + kx) * kHz + zz0 + a_px + ky) * CSX + m * 16 + a_c);
 #pragma unroll
-    for (int nb = 0; nb < NT / 2; ++nb) {
-      unsigned b[4];
-      ldmatrix_x4_trans(b, s_dz + (xx * kTz + zz0 + b_px) * CSZ + nb * 16 + b_c);
+      for (int nb = 0; nb < NT / 2; ++nb) {
+        unsigned b[4];
+        ldmatrix_x4_trans(b, s_dz + (xx * kTz + zz0 + b_px) * CSZ + nb * 16 + b_c);
 #pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        mma_bf16(acc[m][2 * nb], a[m], b[0], b[1]);
-        mma_bf16(acc[m][2 * nb + 1], a[m], b[2], b[3]);
+        for (int m = 0; m < MT; ++m) {
+          mma_bf16(acc[m][2 * nb], a[m], b[0], b[1]);
+          mma_bf16(acc[m][2 * nb + 1], a[m], b[2], b[3]);
+        }
       }
     }
   }
-  float* out = part + static_cast<size_t>(blockIdx.y * gridDim.x + blockIdx.x) * 9 * CIN * COUT +
-               static_cast<size_t>(tap) * CIN * COUT;
+  float* out = part + static_cast<size_t>(blockIdx.x) * 9 * CIN * COUT + static_cast<size_t>(tap) * CIN * COUT;
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -557,13 +562,28 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad(const __nv_bfloat16* __re
     }
 }
 
-// out[i] = sum over b < nblocks of part[b * n + i], in block order.
-__global__ void k_reduce_partials(const float* __restrict__ part, int nblocks, int n, float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// out[i] = sum over b < nblocks of part[b * n + i] in a fixed order: warp w of
+// 8 sums the partials b = w, w + 8, ... of the block's 32 values, then the
+// eight sums are added in turn. (One thread per value ran n / 256 blocks with
+// one chain of nblocks loads each: 133 us on average over the twelve sums of a
+// 608 x 1600 backward pass.)
+constexpr int kRedWarps = 8;
+__global__ void __launch_bounds__(32 * kRedWarps) k_reduce_partials(const float* __restrict__ part, int nblocks, int n,
+                                                                    float* __restrict__ out) {
+  __shared__ float sh[kRedWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
   float s = 0.0f;
-  for (int b = 0; b < nblocks; ++b) s += part[static_cast<size_t>(b) * n + i];
-  out[i] = s;
+  if (i < n) {
+#pragma unroll 8
+    for (int b = w; b < nblocks; b += kRedWarps) s += part[static_cast<size_t>(b) * n + i];
+  }
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < n) {
+#pragma unroll
+    for (int k = 1; k < kRedWarps; ++k) s += sh[k][lane];
+    out[i] = s;
+  }
 }
 
 // Per-block partial sums over pixels of dZ[p][co] (bias gradient): block b
@@ -893,23 +913,41 @@ int fwigb_cnn_conv3x3(const void* x, int Hz, int Wx, int cin_pad, int cout_pad, 
   return e == cudaSuccess ? FWIGB_OK : FWIGB_ERR_CUDA;
 }
 
-int fwigb_cnn_wgrad_partials(const void* x, const void* dz, int Hz, int Wx, int cin_pad, int cout_pad,
-                             float* partials, void* stream) {
+static int wgrad(const void* x, const void* dz, int Hz, int Wx, int cin_pad, int cout_pad, int blocks,
+                 float* partials, void* stream) {
   cudaGetLastError();  // drop a stale non-sticky error of an earlier, unrelated call
   if (!x || !dz || !partials || Hz <= 0 || Wx <= 0 || Hz % kTz != 0) return FWIGB_ERR_ARG;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const dim3 grid(Hz / kTz, (Wx + kTx - 1) / kTx);
   const auto* xi = static_cast<const __nv_bfloat16*>(x);
   const auto* di = static_cast<const __nv_bfloat16*>(dz);
   if (cin_pad == 16 && cout_pad == 32)
-    k_conv3x3_wgrad<16, 32><<<grid, 288, 0, s>>>(xi, di, Hz, Wx, partials);
+    k_conv3x3_wgrad<16, 32><<<blocks, 288, 0, s>>>(xi, di, Hz, Wx, partials);
   else if (cin_pad == 32 && cout_pad == 32)
-    k_conv3x3_wgrad<32, 32><<<grid, 288, 0, s>>>(xi, di, Hz, Wx, partials);
+    k_conv3x3_wgrad<32, 32><<<blocks, 288, 0, s>>>(xi, di, Hz, Wx, partials);
   else if (cin_pad == 32 && cout_pad == 16)
-    k_conv3x3_wgrad<32, 16><<<grid, 288, 0, s>>>(xi, di, Hz, Wx, partials);
+    k_conv3x3_wgrad<32, 16><<<blocks, 288, 0, s>>>(xi, di, Hz, Wx, partials);
   else
     return FWIGB_ERR_UNSUPPORTED;
   return cudaGetLastError() == cudaSuccess ? FWIGB_OK : FWIGB_ERR_CUDA;
+}
+
+int fwigb_cnn_wgrad_partials(const void* x, const void* dz, int Hz, int Wx, int cin_pad, int cout_pad,
+                             float* partials, void* stream) {
+  return wgrad(x, dz, Hz, Wx, cin_pad, cout_pad, fwigb_cnn_tile_count(Hz, Wx), partials, stream);
+}
+
+// Blocks of a weight gradient: four resident per SM (47 KB of tiles each).
+int fwigb_cnn_wgrad_blocks(int Hz, int Wx) {
+  const int tiles = fwigb_cnn_tile_count(Hz, Wx);
+  return tiles < 608 ? tiles : 608;
+}
+
+int fwigb_cnn_wgrad(const void* x, const void* dz, int Hz, int Wx, int cin_pad, int cout_pad, float* partials,
+                    float* out, void* stream) {
+  if (!out) return FWIGB_ERR_ARG;
+  const int nb = fwigb_cnn_wgrad_blocks(Hz, Wx);
+  const int rc = wgrad(x, dz, Hz, Wx, cin_pad, cout_pad, nb, partials, stream);
+  return rc != FWIGB_OK ? rc : fwigb_cnn_reduce_partials(partials, nb, 9 * cin_pad * cout_pad, out, stream);
 }
 
 int fwigb_cnn_tile_count(int Hz, int Wx) { return (Hz / kTz) * ((Wx + kTx - 1) / kTx); }
@@ -965,7 +1003,7 @@ int fwigb_cnn_pack_weights_tc(const float* w, int cin, int cout, int cin_pad, in
 int fwigb_cnn_reduce_partials(const float* partials, int nblocks, int n, float* out, void* stream) {
   cudaGetLastError();  // drop a stale non-sticky error of an earlier, unrelated call
   if (!partials || !out || nblocks <= 0 || n <= 0) return FWIGB_ERR_ARG;
-  k_reduce_partials<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(partials, nblocks, n, out);
+  k_reduce_partials<<<(n + 31) / 32, 32 * kRedWarps, 0, static_cast<cudaStream_t>(stream)>>>(partials, nblocks, n, out);
   return cudaGetLastError() == cudaSuccess ? FWIGB_OK : FWIGB_ERR_CUDA;
 }
 

@@ -245,10 +245,8 @@ class CnnPreconditioner:
         for k in range(DEPTH - 1, -1, -1):
             _, _, cip, cop = self.LAYERS[k]
             xin = self.x0 if k == 0 else self.y[k - 1]
-            self._ck(self.lib.fwigb_cnn_wgrad_partials(self._p(xin), self._p(dz), self.Hz, self.Wx, cip, cop,
-                                                       self._p(self.part), s))
-            self._ck(self.lib.fwigb_cnn_reduce_partials(self._p(self.part), self.ntiles, 9 * cip * cop,
-                                                        self._p(self.gW[k]), s))
+            self._ck(self.lib.fwigb_cnn_wgrad(self._p(xin), self._p(dz), self.Hz, self.Wx, cip, cop,
+                                              self._p(self.part), self._p(self.gW[k]), s))
             self._ck(self.lib.fwigb_cnn_bias_partials(self._p(dz), self.npix, cop, self.chunk, self._p(self.bpart),
                                                       s))
             nb = (self.npix + self.chunk - 1) // self.chunk

@@ -284,7 +284,7 @@ int fwigb_cnn_tile_count(int Hz, int Wx);
  * dL/dW[tap][ci][co] = sum_p x(p + tap offset)[ci] dz(p)[co]. */
 int fwigb_cnn_wgrad_partials(const void *x, const void *dz, int Hz, int Wx, int cin_pad, int cout_pad,
                              float *partials, void *stream);
-/* out[i] = sum over blocks b (in order) of partials[b * n + i]. */
+/* out[i] = sum over blocks b (in a fixed order) of partials[b * n + i]. */
 int fwigb_cnn_reduce_partials(const float *partials, int nblocks, int n, float *out, void *stream);
 /* Per-chunk partial sums over pixels of dz[p][c] (bias gradient):
  * partials[ceil(npix / chunk)][c_pad]. */
@@ -297,6 +297,11 @@ int fwigb_cnn_adam(float *w, const float *grad, float *m1, float *m2, int n, flo
  * gradient: W'[tap][co][ci] = W[8 - tap][ci][co]. */
 int fwigb_cnn_pack_weights(const float *w, int cin, int cout, int cin_pad, int cout_pad, int transposed, void *frag,
                            void *stream);
+/* Weight gradient [9][cin_pad][cout_pad] (FP32); partials holds
+ * fwigb_cnn_wgrad_blocks() times as many floats of scratch. */
+int fwigb_cnn_wgrad_blocks(int Hz, int Wx);
+int fwigb_cnn_wgrad(const void *x, const void *dz, int Hz, int Wx, int cin_pad, int cout_pad, float *partials,
+                    float *out, void *stream);
 /* Model-shaped arrays (row-major double [c][nz][nx], on the device) to an
  * image: out[x * nz + z][c_pad] in FP32, rounded to BF16 when bf16; channels
  * past c are zero. c_pad at most 16. */
