@@ -1201,16 +1201,25 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   for (int k = 0; k < G; ++k) ctx->pack_nx[k / kPackShots] = std::max(ctx->pack_nx[k / kPackShots], slots[k].g.nx);
   // Launch extents: the widest member sub-grid, and rows down to the last
   // one a sweep touches (zact1, or the lowest source / receiver row).
-  ctx->pack_grid.assign(ctx->npacks, SweepGrid{0, 0});
+  ctx->pack_grid.assign(ctx->npacks, SweepGrid{0, 0, 0});
   for (int q = 0; q < ctx->npacks; ++q) ctx->pack_grid[q].nx = ctx->pack_nx[q];
   for (int k = 0; k < G; ++k) {
     const int rows = std::min(slots[k].g.nz, std::max(slots[k].g.zact1, slots[k].sh.rbz1) + 1);
     ctx->pack_grid[k / kPackShots].nz = std::max(ctx->pack_grid[k / kPackShots].nz, rows);
   }
+  // (Every sub-grid has the same rows, hence the same offset.) Variants w = 3 *
+  // (sweep, + 4 with two depths per thread) + tile width.
+  const int zoff = wide_tile_offset(slots[0].g);
+  for (SweepGrid& gr : ctx->pack_grid) gr.zoff = zoff;
+  auto split = [&](int w, int k) {
+    const bool wide = w / 3 >= 4;
+    return tile_split(slots[k].g, kTileXs[w % 3], wide ? kTileZFwd : kTileZ, wide ? zoff : 0);
+  };
   if (G == 1) {
     ctx->pack1.assign(kSweepVariants * 3, SweepPack<1>{});
     for (int w = 0; w < kSweepVariants * 3; ++w) {
       ctx->pack1[w].maps[0] = maps[static_cast<size_t>(w) * ctx->group_cap];
+      ctx->pack1[w].tiles[0] = split(w, 0);
       ctx->pack1[w].slots[0] = slots[0];
     }
   } else {
@@ -1219,6 +1228,7 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
       for (int k = 0; k < G; ++k) {
         SweepPack<kPackShots>& pk = ctx->packs[static_cast<size_t>(w) * ctx->npacks + k / kPackShots];
         pk.maps[k % kPackShots] = maps[static_cast<size_t>(w) * ctx->group_cap + k];
+        pk.tiles[k % kPackShots] = split(w, k);
         pk.slots[k % kPackShots] = slots[k];
       }
   }

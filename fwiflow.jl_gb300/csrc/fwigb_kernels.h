@@ -71,30 +71,38 @@ struct Geo {
   float dt, rdz, rdx;
 };
 
-// Split of a sub-grid's tiles (tz depths x tx columns, ntz x ntx in all)
-// into the fast tiles, the rectangle [ftz0, ftz1) x [ftx0, ftx1) of tiles
-// inside the fast box, the mid tiles, those of the rectangle [mtz0, mtz1) x
-// [mtx0, mtx1) inside the mid box that are not fast, and the edge tiles
-// around them.
+// Split of a sub-grid's tiles (tz depths x tx columns, from row zoff on) into
+// the fast tiles, the rectangle [ftz0, ftz1) x [ftx0, ftx1) of tiles inside the
+// fast box, the mid tiles, those of the rectangle [mtz0, mtz1) x [mtx0, mtx1)
+// inside the mid box that are not fast, and the edge tiles around them.
+// Computed on the host; the sweeps read it with their parameters.
 struct TileSplit {
-  int ntz, ntx, ftz0, ftz1, ftx0, ftx1, mtz0, mtz1, mtx0, mtx1;
+  int ftz0, ftz1, ftx0, ftx1, mtz0, mtz1, mtx0, mtx1;
+  int zoff;
 };
 
-__host__ __device__ inline TileSplit tile_split(const Geo& g, int tx, int tz) {
+inline TileSplit tile_split(const Geo& g, int tx, int tz, int zoff) {
   TileSplit s;
-  s.ntz = (g.nz + tz - 1) / tz;
-  s.ntx = (g.nx + tx - 1) / tx;
-  s.ftz0 = (g.fz0 + tz - 1) / tz;
-  s.ftz1 = (g.fz1 + 1) / tz;
-  s.ftx0 = (g.fx0 + tx - 1) / tx;
-  s.ftx1 = (g.fx1 + 1) / tx;
-  if (g.fz0 > g.fz1 || g.fx0 > g.fx1 || s.ftz1 <= s.ftz0 || s.ftx1 <= s.ftx0) s.ftz0 = s.ftz1 = s.ftx0 = s.ftx1 = 0;
-  s.mtz0 = (g.mz0 + tz - 1) / tz;
-  s.mtz1 = (g.mz1 + 1) / tz;
-  s.mtx0 = (g.mx0 + tx - 1) / tx;
-  s.mtx1 = (g.mx1 + 1) / tx;
-  if (g.mz0 > g.mz1 || g.mx0 > g.mx1 || s.mtz1 <= s.mtz0 || s.mtx1 <= s.mtx0) s.mtz0 = s.mtz1 = s.mtx0 = s.mtx1 = 0;
+  auto range = [](int lo, int hi, int t, int& a, int& b) {  // tiles of t inside [lo, hi]
+    a = (lo + t - 1) / t;
+    b = (hi + 1) / t;
+    return lo <= hi && a < b;
+  };
+  s.zoff = zoff;
+  const bool fz = range(g.fz0 - zoff, g.fz1 - zoff, tz, s.ftz0, s.ftz1), fx = range(g.fx0, g.fx1, tx, s.ftx0, s.ftx1);
+  if (!fz || !fx) s.ftz0 = s.ftz1 = s.ftx0 = s.ftx1 = 0;
+  const bool mz = range(g.mz0 - zoff, g.mz1 - zoff, tz, s.mtz0, s.mtz1), mx = range(g.mx0, g.mx1, tx, s.mtx0, s.mtx1);
+  if (!mz || !mx) s.mtz0 = s.mtz1 = s.mtx0 = s.mtx1 = 0;
   return s;
+}
+
+// First row of the 64-row tiles: 0, or -32 where that leaves more of them free
+// of CPML rows (608 rows with a 32-row CPML: 8 of 10 tiles instead of 7, and the
+// first of the other two half empty, so that 11 % of the rows run the edge
+// bodies instead of 22 %).
+inline int wide_tile_offset(const Geo& g) {
+  const TileSplit a = tile_split(g, 4, 64, 0), b = tile_split(g, 4, 64, -32);
+  return b.mtz1 - b.mtz0 > a.mtz1 - a.mtz0 ? -32 : 0;
 }
 
 struct Fields {
@@ -183,14 +191,15 @@ struct SweepMaps {
 constexpr int kSweepVariants = 8;
 
 // What one sweep launch reads for up to K shots, passed by value as a
-// __grid_constant__ kernel parameter: the block of shot k reads its slot and
-// tensor maps from the constant bank (no global-memory round trip before its
+// __grid_constant__ kernel parameter: the block of shot k reads its slot, tile split
+// and tensor maps from the constant bank (no global-memory round trip before its
 // first stencil load). K = 1 for a lone shot; kPackShots for a batch, which
 // keeps the parameter block under the 32 KB kernel-parameter limit.
 constexpr int kPackShots = 16;
 template <int K>
 struct SweepPack {
   TileMaps maps[K];
+  TileSplit tiles[K];
   ShotSlot slots[K];
 };
 static_assert(sizeof(SweepPack<kPackShots>) < 32000, "sweep pack exceeds the kernel parameter limit");
@@ -205,6 +214,7 @@ bool encode_sweep_maps(const Geo& g, const Fields& f, int tx, SweepMaps& out, co
 // Blocks past a shot's own grid leave at once.
 struct SweepGrid {
   int nz, nx;
+  int zoff;  // first row of the 64-row tiles (wide_tile_offset)
 };
 
 // ---- launchers (kernels.cu). One launch covers the first `nshots` (<= K)

@@ -88,10 +88,10 @@ __device__ __forceinline__ void tma_load_2d(float* dst, const CUtensorMap* tm, i
       : "memory");
 }
 
-// Starts staging NA arrays of the tile at (z0, x0) into shared memory: one
-// 2-D TMA copy each of the box [z0-4, z0-4+BOXZ) x [x0-2, x0+TX+2), zero
-// filled outside the grid. The leader initialises the mbarrier (fenced so the
-// copies see it) and issues the copies after the block has met the barrier's
+// Stages NA arrays of the tile at (z0, x0) into shared memory: one 2-D TMA
+// copy each of the box [z0-4, z0-4+BOXZ) x [x0-2, x0+TX+2), zero filled
+// outside the grid. The leader initialises the mbarrier (fenced so the copies
+// see it) and issues the copies after the block has met the barrier's
 // initialisation; the caller then loads its own-cell operands (which overlap
 // with the copies) and calls stage_wait.
 template <int NA, int TX, int BOXZ>
@@ -109,11 +109,6 @@ __device__ __forceinline__ void stage_init(uint64_t* bar) {
     fence_mbar_init();
   }
   __syncthreads();
-}
-template <int NA, int TX, int BOXZ>
-__device__ __forceinline__ void stage_begin(const TileMaps& mp, float* sm, uint64_t* bar, int z0, int x0) {
-  stage_init(bar);
-  stage_issue<NA, TX, BOXZ>(mp, sm, bar, z0, x0);
 }
 
 // Waits (bounded) for the staged tiles. On a timeout the error word is raised
@@ -162,10 +157,17 @@ __device__ __forceinline__ bool tile_meets_shot_box(const ShotD& sh, int z0, int
 // logic). The choice is uniform per block. Blocks past a narrower shot's grid
 // leave before staging anything, and so do blocks whose tile lies wholly
 // below row zact1 (the nPad rows, where no sweep reads or writes a cell of
-// its own) unless it holds the shot's source or a receiver. Block
-// (32, TX): lane threadIdx.x covers R adjacent depths (R = TZ / 32),
-// threadIdx.y the column; `b` is the index of its first cell in a staged box
-// (column stride BOXZ = TZ + 8).
+// its own) unless it holds the shot's source or a receiver.
+//
+// Work split. Block (32, TX): lane threadIdx.x covers R adjacent depths
+// (R = TZ / 32), threadIdx.y the column. The sweeps issue more integer than
+// floating-point instructions (F1: 27 FP32 and 57 integer of 164 per cell), so
+// the tile split comes with the parameters, and a thread's addresses are
+// block-uniform 64-bit bases plus one 32-bit byte offset: with the shifted
+// 64-row tiles, a gradient's sweeps on 608 x 1600 (500 steps) 24.4 -> 23.1 ms,
+// two shots of 352 x 832 (400 steps) 15.9 -> 15.1 ms, four of 1120 x 3152 (60
+// steps) 35.4 -> 34.5 ms, 16 of 352 x 832 unchanged.
+//
 // Programmatic dependent launch: a sweep lets the next sweep's blocks be
 // scheduled as soon as all of its own blocks have started, and waits
 // (pdl_wait) for the previous sweep to complete, and its writes to be
@@ -176,68 +178,61 @@ __device__ __forceinline__ bool tile_meets_shot_box(const ShotD& sh, int z0, int
 #define SWEEP_KERNEL_TILE(TZ_)                                                 \
   const int shot = K == 1 ? 0 : static_cast<int>(blockIdx.z);                  \
   const Geo& g0 = P.slots[shot].g;                                             \
-  const int z0 = blockIdx.x * (TZ_), x0 = blockIdx.y * TX;                     \
+  const TileSplit& ts = P.tiles[shot];                                         \
+  const int tz = blockIdx.x, tx = blockIdx.y;                                  \
+  const int z0 = tz * (TZ_) + ts.zoff, x0 = tx * TX;                           \
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");              \
   if (z0 >= g0.nz || x0 >= g0.nx) return;                                      \
   if (z0 > g0.zact1 && !tile_meets_shot_box(P.slots[shot].sh, z0, x0, (TZ_), TX)) return; \
-  const TileSplit ts = tile_split(g0, TX, (TZ_));                              \
-  const bool fast = static_cast<int>(blockIdx.x) >= ts.ftz0 &&                 \
-                    static_cast<int>(blockIdx.x) < ts.ftz1 &&                  \
-                    static_cast<int>(blockIdx.y) >= ts.ftx0 &&                 \
-                    static_cast<int>(blockIdx.y) < ts.ftx1;                    \
-  const bool mid = !fast && static_cast<int>(blockIdx.x) >= ts.mtz0 &&         \
-                   static_cast<int>(blockIdx.x) < ts.mtz1 &&                   \
-                   static_cast<int>(blockIdx.y) >= ts.mtx0 &&                  \
-                   static_cast<int>(blockIdx.y) < ts.mtx1;
+  const bool fast = tz >= ts.ftz0 && tz < ts.ftz1 && tx >= ts.ftx0 && tx < ts.ftx1; \
+  const bool mid = !fast && tz >= ts.mtz0 && tz < ts.mtz1 && tx >= ts.mtx0 && tx < ts.mtx1;
 
 #define SWEEP_BODY_SLOT()                                                      \
   const ShotSlot& S = P.slots[shot];                                           \
-  const Geo& g = S.g;
-
-// A fast tile lies wholly inside the grid. `special` marks the tiles that
-// meet the bounding box of the shot's receivers and source.
-#define SWEEP_FAST_SLOT(TZ_)                                                   \
-  SWEEP_BODY_SLOT()                                                            \
-  const ShotD& sh = S.sh;                                                      \
-  const bool special = !(z0 + (TZ_) - 1 < sh.rbz0 || z0 > sh.rbz1 ||           \
-                         x0 + TX - 1 < sh.rbx0 || x0 > sh.rbx1);
+  const Geo& g = S.g;                                                          \
+  const Fields& f = S.f;                                                       \
+  const MediaD& m = S.m;                                                       \
+  const ShotD& sh = S.sh;
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Fast tiles: the thread's first cell (z, x), its global index i and its box
-// index b (every cell of a fast tile is inside the grid).
-#define SWEEP_CELL(BOXZ_, R_)                                                  \
-  const Fields& f = S.f;                                                       \
-  const MediaD& m = S.m;                                                       \
-  const int z = z0 + (R_) * static_cast<int>(threadIdx.x), x = x0 + threadIdx.y; \
-  const size_t ldz = static_cast<size_t>(g.ldz);                               \
-  const size_t i = static_cast<size_t>(x) * ldz + z;                           \
-  const int b = (threadIdx.y + 2) * (BOXZ_) + (R_) * threadIdx.x + 4;
-
-// Fast tiles: the staging barrier is set up before the media loads and the
-// tile copies are issued right after pdl_wait (SWEEP_TMA).
-#define SWEEP_SMEM(BOXZ_)                                                      \
+// Fast and mid tiles lie wholly inside the grid: `base` is the byte offset of
+// the tile's first cell, `off` that of the thread's first cell from there and b
+// its index in a staged box. `special` marks the tiles that meet the bounding
+// box of the shot's receivers and source.
+#define SWEEP_FAST(TZ_, BOXZ_, R_)                                             \
+  SWEEP_BODY_SLOT()                                                            \
+  const bool special = tile_meets_shot_box(sh, z0, x0, (TZ_), TX);             \
   constexpr int N = (BOXZ_) * (TX + 4);                                        \
+  const size_t base = (static_cast<size_t>(x0) * g.ldz + z0) * sizeof(float);  \
+  const unsigned off =                                                         \
+      (threadIdx.y * static_cast<unsigned>(g.ldz) + (R_) * threadIdx.x) * static_cast<unsigned>(sizeof(float)); \
+  const int b = (threadIdx.y + 2) * (BOXZ_) + (R_) * threadIdx.x + 4;          \
+  const int z = z0 + (R_) * static_cast<int>(threadIdx.x), x = x0 + threadIdx.y; \
+  SWEEP_SMEM()
+
+#define SWEEP_SMEM()                                                           \
   extern __shared__ __align__(128) float sm[];                                 \
   __shared__ __align__(8) uint64_t bar;                                        \
   stage_init(&bar);
 #define SWEEP_TMA(NA, BOXZ_) stage_issue<NA, TX, (BOXZ_)>(P.maps[shot], sm, &bar, z0, x0);
 
-// Edge tiles: the thread's first cell (z, x), its global index i, its box
-// index b and whether the cell lies in the grid (`live`; a thread with no
-// cell in the grid takes part in the staging set-up only, and the tile's
-// first thread, which issues and awaits the copies, is always live).
-#define SWEEP_EDGE_CELL(BOXZ_, R_)                                             \
-  const Fields& f = S.f;                                                       \
-  const MediaD& m = S.m;                                                       \
+// Edge tiles: the thread's first cell (z, x), its global index i, its box index
+// b, whether it lies in the grid (`live`: depths may also lie above it, in a
+// shifted tile grid) and how many of its R depths do (rows_in). A thread with no
+// cell in the grid takes part in the staging set-up only.
+#define SWEEP_EDGE(BOXZ_, R_)                                                  \
+  SWEEP_BODY_SLOT()                                                            \
   const CpmlD& c = S.c;                                                        \
-  const int z = z0 + (R_) * static_cast<int>(threadIdx.x), x = x0 + threadIdx.y; \
-  const bool live = z < g.nz && x < g.nx;                                      \
-  const int rows_in = live ? g.nz - z : 0;                                     \
+  constexpr int N = (BOXZ_) * (TX + 4);                                        \
   const size_t ldz = static_cast<size_t>(g.ldz);                               \
+  const int z = z0 + (R_) * static_cast<int>(threadIdx.x), x = x0 + threadIdx.y; \
+  const bool live = z >= 0 && z < g.nz && x < g.nx;                            \
+  const int rows_in = live ? g.nz - z : 0;                                     \
   const size_t i = static_cast<size_t>(x) * ldz + z;                           \
-  const int b = (threadIdx.y + 2) * (BOXZ_) + (R_) * threadIdx.x + 4;           \
-  (void)rows_in;
+  const int b = (threadIdx.y + 2) * (BOXZ_) + (R_) * threadIdx.x + 4;          \
+  (void)rows_in;                                                               \
+  SWEEP_SMEM()
 
 // Values of the thread's R depths that lie in the grid (rows_in of them);
 // the others are left 0.
@@ -247,10 +242,49 @@ __device__ __forceinline__ void ldrows(const float* p, int rows_in, float (&v)[R
   for (int r = 0; r < R; ++r) v[r] = r < rows_in ? p[r] : 0.0f;
 }
 
-// Paired loads / stores of two adjacent depths (8-byte aligned: even depth,
-// ldz a multiple of 32, even box index).
+// Own-cell values of a thread's R adjacent depths at a byte offset from a
+// block-uniform pointer (8-byte paired when R == 2: even depth, ldz a
+// multiple of 32).
+template <int R>
+__device__ __forceinline__ void ldo(const float* p, size_t base, unsigned off, float (&v)[R]) {
+  const char* q = reinterpret_cast<const char*>(p) + base + off;
+  if constexpr (R == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(q);
+    v[0] = t.x;
+    v[1] = t.y;
+  } else {
+    v[0] = *reinterpret_cast<const float*>(q);
+  }
+}
+template <int R>
+__device__ __forceinline__ void sto(float* p, size_t base, unsigned off, const float (&v)[R]) {
+  char* q = reinterpret_cast<char*>(p) + base + off;
+  if constexpr (R == 2)
+    *reinterpret_cast<float2*>(q) = make_float2(v[0], v[1]);
+  else
+    *reinterpret_cast<float*>(q) = v[0];
+}
+
+// The media arrays are read by every sweep and, in a batched launch, by every
+// shot of the pack (their sub-grids are windows of the same model): their
+// loads carry an L2 evict-last policy so that the streamed fields do not push
+// them out of L2 (createpolicy / ld.global.L2::cache_hint).
+__device__ __forceinline__ uint64_t media_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+template <int R>
+__device__ __forceinline__ void ldm(const float* a, size_t base, unsigned off, float (&v)[R], uint64_t pol) {
+  const char* q = reinterpret_cast<const char*>(a) + base + off;
+  if constexpr (R == 2)
+    asm("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v[0]), "=f"(v[1]) : "l"(q), "l"(pol));
+  else
+    asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v[0]) : "l"(q), "l"(pol));
+}
+
+// Paired shared-memory loads of two adjacent depths (even box index).
 __device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
-__device__ __forceinline__ void st2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
 
 // 4th-order staggered difference from its four samples: (C1 (p - q) -
 // C2 (s - t)) r, the expression of sdm / sdp.
@@ -258,15 +292,67 @@ __device__ __forceinline__ float dd(float p, float q, float s, float t, float r)
   return (C1 * (p - q) - C2 * (s - t)) * r;
 }
 
+// The differences of a staged array at the thread's R depths: along z (Dm, Dp)
+// and along x. With two depths (b even) the float2 at b + o (o even) holds
+// both depths' samples at offset o, so a z stencil of both takes the pairs at
+// b - 2, b, b + 2 and an x stencil those at b + k BOXZ.
+template <int R>
+__device__ __forceinline__ void dmz(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdm(a, b, 1, r);
+  } else {
+    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
+    o[0] = dd(c.x, m.y, c.y, m.x, r);
+    o[1] = dd(c.y, c.x, p.x, m.y, r);
+  }
+}
+template <int R>
+__device__ __forceinline__ void dpz(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdp(a, b, 1, r);
+  } else {
+    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
+    o[0] = dd(c.y, c.x, p.x, m.y, r);
+    o[1] = dd(p.x, c.y, p.y, c.x, r);
+  }
+}
+template <int R, int BOXZ>
+__device__ __forceinline__ void dmx(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdm(a, b, BOXZ, r);
+  } else {
+    const float2 c = ld2(a + b), m = ld2(a + b - BOXZ), p = ld2(a + b + BOXZ), m2 = ld2(a + b - 2 * BOXZ);
+    o[0] = dd(c.x, m.x, p.x, m2.x, r);
+    o[1] = dd(c.y, m.y, p.y, m2.y, r);
+  }
+}
+template <int R, int BOXZ>
+__device__ __forceinline__ void dpx(const float* a, int b, float r, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = sdp(a, b, BOXZ, r);
+  } else {
+    const float2 c = ld2(a + b), p = ld2(a + b + BOXZ), p2 = ld2(a + b + 2 * BOXZ), m = ld2(a + b - BOXZ);
+    o[0] = dd(p.x, c.x, p2.x, m.x, r);
+    o[1] = dd(p.y, c.y, p2.y, m.y, r);
+  }
+}
+template <int R>
+__device__ __forceinline__ void own(const float* a, int b, float (&o)[R]) {
+  if constexpr (R == 1) {
+    o[0] = a[b];
+  } else {
+    const float2 c = ld2(a + b);
+    o[0] = c.x;
+    o[1] = c.y;
+  }
+}
+
 // Register budgets (measured on GB300 over the tile widths; the sweeps wait
 // on memory latency, so resident warps count for more than the bytes
-// spilled): forward sweeps 32 registers (64 warps per SM; with two cells per
-// thread 9 % faster than 40 registers on a 16-shot group). Backward sweeps:
+// spilled): forward sweeps 32 registers (64 warps per SM). Backward sweeps:
 // NT resident threads per SM, so 65536 / NT registers: with one cell per
-// thread 2048 (32 registers, 52-96 bytes spilled; 4 % faster than 40 on the
-// 64-shot workload) or 1536 (40 registers; 10 % faster on a lone 608 x 1600
-// shot, whose arrays stay partly in L2), picked by the autotuner; with two
-// cells 1024 (64 registers).
+// thread 2048 (32 registers) or 1536 (40 registers), picked by the autotuner;
+// with two cells 1024 (64 registers).
 #define FWD_BOUNDS __launch_bounds__(32 * TX, 2048 / (32 * TX))
 #define BWD_BOUNDS __launch_bounds__(32 * TX, (NT / (32 * TX)) > 0 ? (NT / (32 * TX)) : 1)
 
@@ -279,13 +365,10 @@ template <int TX, int K, int R>
 __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
-  SWEEP_BODY_SLOT()
-  SWEEP_EDGE_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_EDGE(BOXZ, R)
   pdl_wait();
   SWEEP_TMA(2, BOXZ)
   if (!live) return;
-  const ShotD& sh = S.sh;
   const bool rec_tile = tile_meets_shot_box(sh, z0, x0, 32 * R, TX);
   const StoreD& st = S.st;
   if (!stage_wait(&bar, err, inject)) return;
@@ -354,9 +437,8 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
 template <int TX, int K, int R>
 __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
-  SWEEP_BODY_SLOT()
-  SWEEP_EDGE_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_EDGE(BOXZ, R)
+  (void)sh;
   pdl_wait();
   SWEEP_TMA(3, BOXZ)
   if (!live) return;
@@ -418,9 +500,7 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
-  SWEEP_BODY_SLOT()
-  SWEEP_EDGE_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_EDGE(BOXZ, R)
   const Grads& gr = S.gr;
   float p_lam[R], p_l2m[R], p_amu[R];
   float p_szz[R], p_sxx[R], p_sxz[R], p_vza[R], p_vxa[R];
@@ -435,7 +515,6 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
   ldrows<R>(f.vz_a + i, rows_in, p_vza);
   ldrows<R>(f.vx_a + i, rows_in, p_vxa);
   if (!live) return;
-  const ShotD& sh = S.sh;
   const StoreD& st = S.st;
   const int it = S.nSteps - 2 - j;  // this shot's time step at backward iteration j
   const float dt = g.dt;
@@ -531,9 +610,7 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
 template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
-  SWEEP_BODY_SLOT()
-  SWEEP_EDGE_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_EDGE(BOXZ, R)
   const Grads& gr = S.gr;
   const int rev = S.nSteps - 2 - j >= 1;
   float p_bA[R], p_bB[R], p_amu[R], p_lam[R], p_l2m[R], p_sa[R], p_xa[R], p_za[R], p_vz[R], p_vx[R];
@@ -550,7 +627,6 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
   ldrows<R>(f.vz + i, rev ? rows_in : 0, p_vz);
   ldrows<R>(f.vx + i, rev ? rows_in : 0, p_vx);
   if (!live) return;
-  const ShotD& sh = S.sh;
   const StoreD& st = S.st;
   const bool rec_tile = tile_meets_shot_box(sh, z0, x0, 32 * R, TX);
   // Backward iteration j handles res_injection + el_stress_adj of step
@@ -638,314 +714,128 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
 // reference's CPML divisions by K are exact there (x / 1 = x) and are left
 // out, the memory-array updates and the ring are never reached, and the
 // source / receiver terms are evaluated only in tiles that meet the bounding
-// box of the shot's receivers and source. Operation order otherwise follows
-// the edge kernels.
+// box of the shot's receivers and source. Operation order of the fields'
+// updates otherwise follows the edge bodies.
+// MID: the tile is a mid tile (no CPML cell; it may hold ring cells).
+// Own-cell operands and results move as float2 with two depths per thread.
 
-// Forward fast bodies, one depth per thread (32-row tiles).
-// MID: the tile is a mid tile (no CPML cell; it may hold ring cells), and
-// the boundary ring of step it is saved when `save` is set.
-// The media arrays are read by every sweep and, in a batched launch, by every
-// shot of the pack (their sub-grids are windows of the same model): their
-// loads carry an L2 evict-last policy so that the streamed fields do not push
-// them out of L2 (createpolicy / ld.global.L2::cache_hint).
-__device__ __forceinline__ uint64_t media_policy() {
-  uint64_t p;
-  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ float ldm(const float* a, uint64_t pol) {
-  float v;
-  asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(a), "l"(pol));
-  return v;
-}
-__device__ __forceinline__ float2 ldm2(const float* a, uint64_t pol) {
-  float2 v;
-  asm("ld.global.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(a), "l"(pol));
-  return v;
-}
-template <int R>
-__device__ __forceinline__ void ldrm(const float* p, float (&v)[R], uint64_t pol) {
-  if constexpr (R == 2) {
-    const float2 t = ldm2(p, pol);
-    v[0] = t.x;
-    v[1] = t.y;
-  } else {
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = ldm(p + r, pol);
-  }
-}
-
-template <int TX, int K, bool MID>
-__device__ __forceinline__ void fwd_stress_fast1(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
-                                                 bool inject, unsigned* err) {
-  SWEEP_FAST_SLOT(kTileZ)
-  SWEEP_CELL(kBoxZ, 1)
-  SWEEP_SMEM(kBoxZ)
-  const uint64_t pol = media_policy();
-  const float lam = ldm(m.lam + i, pol), l2m = ldm(m.l2m + i, pol), amu = ldm(m.aveMu + i, pol);
-  pdl_wait();
-  SWEEP_TMA(2, kBoxZ)
-  float szz = f.szz[i], sxx = f.sxx[i];
-  const float sxz = f.sxz[i];
-  if (!stage_wait(&bar, err, inject)) return;
-  const float* s_vz = sm;
-  const float* s_vx = sm + N;
-  if constexpr (MID) {
-    if (save) ring_save(g, S.st, it, z, x, szz, sxz, sxx, s_vz[b], s_vx[b]);
-  } else {
-    (void)save;
-  }
-  const float dvz_dz = sdm(s_vz, b, 1, g.rdz);
-  const float dvx_dx = sdm(s_vx, b, kBoxZ, g.rdx);
-  const float dvx_dz = sdp(s_vx, b, 1, g.rdz);
-  const float dvz_dx = sdp(s_vz, b, kBoxZ, g.rdx);
-  szz += (l2m * dvz_dz + lam * dvx_dx) * g.dt;
-  sxx += (lam * dvz_dz + l2m * dvx_dx) * g.dt;
-  f.sxz[i] = sxz + amu * (dvx_dz + dvz_dx) * g.dt;
-  if (special) {
-    if (z == sh.src_z && x == sh.src_x) {
-      szz += sh.src_szz[it];
-      sxx += sh.src_sxx[it];
-    }
-    record(sh, it, first_receiver(sh, z, x), z, x, szz, sxx);
-  }
-  f.szz[i] = szz;
-  f.sxx[i] = sxx;
-}
-
-template <int TX, int K>
-__device__ __forceinline__ void fwd_velocity_fast1(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
-  SWEEP_FAST_SLOT(kTileZ)
-  (void)special;
-  SWEEP_CELL(kBoxZ, 1)
-  SWEEP_SMEM(kBoxZ)
-  const uint64_t pol = media_policy();
-  const float bA = ldm(m.bycA + i, pol), bB = ldm(m.bycB + i, pol);
-  pdl_wait();
-  SWEEP_TMA(3, kBoxZ)
-  const float vz = f.vz[i], vx = f.vx[i];
-  if (!stage_wait(&bar, err)) return;
-  const float* s_szz = sm;
-  const float* s_sxx = sm + N;
-  const float* s_sxz = sm + 2 * N;
-  const float dszz_dz = sdp(s_szz, b, 1, g.rdz);
-  const float dsxz_dx = sdm(s_sxz, b, kBoxZ, g.rdx);
-  const float dsxz_dz = sdm(s_sxz, b, 1, g.rdz);
-  const float dsxx_dx = sdp(s_sxx, b, kBoxZ, g.rdx);
-  const float nvz = vz + (dszz_dz + dsxz_dx) * bA * g.dt;
-  const float nvx = vx + (dsxz_dz + dsxx_dx) * bB * g.dt;
-  f.vz[i] = nvz;
-  f.vx[i] = nvx;
-  if (S.gr.illum) S.gr.illum[i] += nvz * nvz + nvx * nvx;
-}
-
-// Forward fast bodies, two adjacent depths per thread (R = 2): own-cell
-// operands and results move as float2, and the staged samples are read in
-// pairs (b-2, b-1), (b, b+1), (b+2, b+3) along z and (b, b+1) at each
-// column offset along x, which cover the stencils of both depths.
 template <int TX, int K, int R, bool MID>
-__device__ __forceinline__ void fwd_stress_fast2(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
-                                                 bool inject, unsigned* err) {
-  static_assert(R == 2, "the forward fast bodies handle two depths per thread");
+__device__ __forceinline__ void fwd_stress_fast(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
+                                                bool inject, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST_SLOT(TZ)
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_FAST(TZ, BOXZ, R)
   const uint64_t pol = media_policy();
-  const float2 lam = ldm2(m.lam + i, pol), l2m = ldm2(m.l2m + i, pol), amu = ldm2(m.aveMu + i, pol);
+  float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R];
+  ldm<R>(m.lam, base, off, lam, pol);
+  ldm<R>(m.l2m, base, off, l2m, pol);
+  ldm<R>(m.aveMu, base, off, amu, pol);
   pdl_wait();
   SWEEP_TMA(2, BOXZ)
-  const float2 szz = ld2(f.szz + i), sxx = ld2(f.sxx + i), sxz = ld2(f.sxz + i);
+  ldo<R>(f.szz, base, off, szz);
+  ldo<R>(f.sxx, base, off, sxx);
+  ldo<R>(f.sxz, base, off, sxz);
   if (!stage_wait(&bar, err, inject)) return;
   const float* s_vz = sm;
   const float* s_vx = sm + N;
+  const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
   if constexpr (MID) {
     if (save) {
-      ring_save(g, S.st, it, z, x, szz.x, sxz.x, sxx.x, s_vz[b], s_vx[b]);
-      ring_save(g, S.st, it, z + 1, x, szz.y, sxz.y, sxx.y, s_vz[b + 1], s_vx[b + 1]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) ring_save(g, S.st, it, z + r, x, szz[r], sxz[r], sxx[r], s_vz[b + r], s_vx[b + r]);
     }
   } else {
     (void)save;
   }
-  const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
-  const float2 zm = ld2(s_vz + b - 2), z0v = ld2(s_vz + b), zp = ld2(s_vz + b + 2);
-  const float2 xm = ld2(s_vx + b - 2), x0v = ld2(s_vx + b), xp = ld2(s_vx + b + 2);
-  const float2 zc1 = ld2(s_vz + b + BOXZ), zc2 = ld2(s_vz + b + 2 * BOXZ), zcm = ld2(s_vz + b - BOXZ);
-  const float2 xc1 = ld2(s_vx + b + BOXZ), xcm = ld2(s_vx + b - BOXZ), xcm2 = ld2(s_vx + b - 2 * BOXZ);
-  // depth z (.x): sdm_z(vz) = dd(a[b], a[b-1], a[b+1], a[b-2]); sdp_z(vx) = dd(a[b+1], a[b], a[b+2], a[b-1])
-  const float dvz_dz0 = dd(z0v.x, zm.y, z0v.y, zm.x, rdz), dvz_dz1 = dd(z0v.y, z0v.x, zp.x, zm.y, rdz);
-  const float dvx_dz0 = dd(x0v.y, x0v.x, xp.x, xm.y, rdz), dvx_dz1 = dd(xp.x, x0v.y, xp.y, x0v.x, rdz);
-  // along x: sdm_x(vx) = dd(a[b], a[b-B], a[b+B], a[b-2B]); sdp_x(vz) = dd(a[b+B], a[b], a[b+2B], a[b-B])
-  const float dvx_dx0 = dd(x0v.x, xcm.x, xc1.x, xcm2.x, rdx), dvx_dx1 = dd(x0v.y, xcm.y, xc1.y, xcm2.y, rdx);
-  const float dvz_dx0 = dd(zc1.x, z0v.x, zc2.x, zcm.x, rdx), dvz_dx1 = dd(zc1.y, z0v.y, zc2.y, zcm.y, rdx);
-  float szz0 = szz.x + (l2m.x * dvz_dz0 + lam.x * dvx_dx0) * dt;
-  float szz1 = szz.y + (l2m.y * dvz_dz1 + lam.y * dvx_dx1) * dt;
-  float sxx0 = sxx.x + (lam.x * dvz_dz0 + l2m.x * dvx_dx0) * dt;
-  float sxx1 = sxx.y + (lam.y * dvz_dz1 + l2m.y * dvx_dx1) * dt;
-  st2(f.sxz + i, sxz.x + amu.x * (dvx_dz0 + dvz_dx0) * dt, sxz.y + amu.y * (dvx_dz1 + dvz_dx1) * dt);
-  if (special) {
-    float* szr[2] = {&szz0, &szz1};
-    float* sxr[2] = {&sxx0, &sxx1};
+  float dvz_dz[R], dvx_dx[R], dvx_dz[R], dvz_dx[R];
+  dmz<R>(s_vz, b, rdz, dvz_dz);
+  dmx<R, BOXZ>(s_vx, b, rdx, dvx_dx);
+  dpz<R>(s_vx, b, rdz, dvx_dz);
+  dpx<R, BOXZ>(s_vz, b, rdx, dvz_dx);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int zr = z + r;
-      if (zr == sh.src_z && x == sh.src_x) {
-        *szr[r] += sh.src_szz[it];
-        *sxr[r] += sh.src_sxx[it];
+  for (int r = 0; r < R; ++r) {
+    szz[r] += (l2m[r] * dvz_dz[r] + lam[r] * dvx_dx[r]) * dt;
+    sxx[r] += (lam[r] * dvz_dz[r] + l2m[r] * dvx_dx[r]) * dt;
+    sxz[r] = sxz[r] + amu[r] * (dvx_dz[r] + dvz_dx[r]) * dt;
+  }
+  sto<R>(f.sxz, base, off, sxz);
+  if (special) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (z + r == sh.src_z && x == sh.src_x) {
+        szz[r] += sh.src_szz[it];
+        sxx[r] += sh.src_sxx[it];
       }
-      record(sh, it, first_receiver(sh, zr, x), zr, x, *szr[r], *sxr[r]);
+      record(sh, it, first_receiver(sh, z + r, x), z + r, x, szz[r], sxx[r]);
     }
   }
-  st2(f.szz + i, szz0, szz1);
-  st2(f.sxx + i, sxx0, sxx1);
+  sto<R>(f.szz, base, off, szz);
+  sto<R>(f.sxx, base, off, sxx);
 }
 
 template <int TX, int K, int R>
-__device__ __forceinline__ void fwd_velocity_fast2(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
-  static_assert(R == 2, "the forward fast bodies handle two depths per thread");
+__device__ __forceinline__ void fwd_velocity_fast(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST_SLOT(TZ)
+  SWEEP_FAST(TZ, BOXZ, R)
   (void)special;
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  (void)z;
+  (void)x;
   const uint64_t pol = media_policy();
-  const float2 bA = ldm2(m.bycA + i, pol), bB = ldm2(m.bycB + i, pol);
+  float bA[R], bB[R], vz[R], vx[R];
+  ldm<R>(m.bycA, base, off, bA, pol);
+  ldm<R>(m.bycB, base, off, bB, pol);
   pdl_wait();
   SWEEP_TMA(3, BOXZ)
-  const float2 vz = ld2(f.vz + i), vx = ld2(f.vx + i);
+  ldo<R>(f.vz, base, off, vz);
+  ldo<R>(f.vx, base, off, vx);
   if (!stage_wait(&bar, err)) return;
   const float* s_szz = sm;
   const float* s_sxx = sm + N;
   const float* s_sxz = sm + 2 * N;
   const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
-  const float2 pm = ld2(s_szz + b - 2), p0 = ld2(s_szz + b), pp = ld2(s_szz + b + 2);
-  const float2 qm = ld2(s_sxz + b - 2), q0 = ld2(s_sxz + b), qp = ld2(s_sxz + b + 2);
-  const float2 qcm = ld2(s_sxz + b - BOXZ), qc1 = ld2(s_sxz + b + BOXZ), qcm2 = ld2(s_sxz + b - 2 * BOXZ);
-  const float2 r0 = ld2(s_sxx + b), rc1 = ld2(s_sxx + b + BOXZ), rc2 = ld2(s_sxx + b + 2 * BOXZ),
-               rcm = ld2(s_sxx + b - BOXZ);
-  // sdp_z(szz) = dd(a[b+1], a[b], a[b+2], a[b-1]); sdm_x(sxz) = dd(a[b], a[b-B], a[b+B], a[b-2B]);
-  // sdm_z(sxz) = dd(a[b], a[b-1], a[b+1], a[b-2]); sdp_x(sxx) = dd(a[b+B], a[b], a[b+2B], a[b-B])
-  const float dszz_dz0 = dd(p0.y, p0.x, pp.x, pm.y, rdz), dszz_dz1 = dd(pp.x, p0.y, pp.y, p0.x, rdz);
-  const float dsxz_dx0 = dd(q0.x, qcm.x, qc1.x, qcm2.x, rdx), dsxz_dx1 = dd(q0.y, qcm.y, qc1.y, qcm2.y, rdx);
-  const float dsxz_dz0 = dd(q0.x, qm.y, q0.y, qm.x, rdz), dsxz_dz1 = dd(q0.y, q0.x, qp.x, qm.y, rdz);
-  const float dsxx_dx0 = dd(rc1.x, r0.x, rc2.x, rcm.x, rdx), dsxx_dx1 = dd(rc1.y, r0.y, rc2.y, rcm.y, rdx);
-  const float nvz0 = vz.x + (dszz_dz0 + dsxz_dx0) * bA.x * dt, nvz1 = vz.y + (dszz_dz1 + dsxz_dx1) * bA.y * dt;
-  const float nvx0 = vx.x + (dsxz_dz0 + dsxx_dx0) * bB.x * dt, nvx1 = vx.y + (dsxz_dz1 + dsxx_dx1) * bB.y * dt;
-  st2(f.vz + i, nvz0, nvz1);
-  st2(f.vx + i, nvx0, nvx1);
+  float dszz_dz[R], dsxz_dx[R], dsxz_dz[R], dsxx_dx[R];
+  dpz<R>(s_szz, b, rdz, dszz_dz);
+  dmx<R, BOXZ>(s_sxz, b, rdx, dsxz_dx);
+  dmz<R>(s_sxz, b, rdz, dsxz_dz);
+  dpx<R, BOXZ>(s_sxx, b, rdx, dsxx_dx);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    vz[r] = vz[r] + (dszz_dz[r] + dsxz_dx[r]) * bA[r] * dt;
+    vx[r] = vx[r] + (dsxz_dz[r] + dsxx_dx[r]) * bB[r] * dt;
+  }
+  sto<R>(f.vz, base, off, vz);
+  sto<R>(f.vx, base, off, vx);
   if (S.gr.illum) {
-    const float2 e = ld2(S.gr.illum + i);
-    st2(S.gr.illum + i, e.x + (nvz0 * nvz0 + nvx0 * nvx0), e.y + (nvz1 * nvz1 + nvx1 * nvx1));
-  }
-}
-
-// Own-cell values of a thread's R adjacent depths (8-byte paired when R == 2:
-// even depth, ldz a multiple of 32).
-template <int R>
-__device__ __forceinline__ void ldr(const float* p, float (&v)[R]) {
-  if constexpr (R == 2) {
-    const float2 t = ld2(p);
-    v[0] = t.x;
-    v[1] = t.y;
-  } else {
+    float e[R];
+    ldo<R>(S.gr.illum, base, off, e);
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = p[r];
-  }
-}
-template <int R>
-__device__ __forceinline__ void str(float* p, const float (&v)[R]) {
-  if constexpr (R == 2) {
-    st2(p, v[0], v[1]);
-  } else {
-#pragma unroll
-    for (int r = 0; r < R; ++r) p[r] = v[r];
+    for (int r = 0; r < R; ++r) e[r] += vz[r] * vz[r] + vx[r] * vx[r];
+    sto<R>(S.gr.illum, base, off, e);
   }
 }
 
-// Differences of a staged array at the thread's R depths: along z (Dm, Dp) and
-// along x. With two depths (b even) the float2 at b + o (o even) holds both
-// depths' samples at offset o, so a z stencil of both takes the pairs at
-// b - 2, b, b + 2 and an x stencil those at b + k BOXZ.
-template <int R>
-__device__ __forceinline__ void dmz(const float* a, int b, float r, float (&o)[R]) {
-  if constexpr (R == 1) {
-    o[0] = sdm(a, b, 1, r);
-  } else {
-    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
-    o[0] = dd(c.x, m.y, c.y, m.x, r);
-    o[1] = dd(c.y, c.x, p.x, m.y, r);
-  }
-}
-template <int R>
-__device__ __forceinline__ void dpz(const float* a, int b, float r, float (&o)[R]) {
-  if constexpr (R == 1) {
-    o[0] = sdp(a, b, 1, r);
-  } else {
-    const float2 m = ld2(a + b - 2), c = ld2(a + b), p = ld2(a + b + 2);
-    o[0] = dd(c.y, c.x, p.x, m.y, r);
-    o[1] = dd(p.x, c.y, p.y, c.x, r);
-  }
-}
-template <int R, int BOXZ>
-__device__ __forceinline__ void dmx(const float* a, int b, float r, float (&o)[R]) {
-  if constexpr (R == 1) {
-    o[0] = sdm(a, b, BOXZ, r);
-  } else {
-    const float2 c = ld2(a + b), m = ld2(a + b - BOXZ), p = ld2(a + b + BOXZ), m2 = ld2(a + b - 2 * BOXZ);
-    o[0] = dd(c.x, m.x, p.x, m2.x, r);
-    o[1] = dd(c.y, m.y, p.y, m2.y, r);
-  }
-}
-template <int R, int BOXZ>
-__device__ __forceinline__ void dpx(const float* a, int b, float r, float (&o)[R]) {
-  if constexpr (R == 1) {
-    o[0] = sdp(a, b, BOXZ, r);
-  } else {
-    const float2 c = ld2(a + b), p = ld2(a + b + BOXZ), p2 = ld2(a + b + 2 * BOXZ), m = ld2(a + b - BOXZ);
-    o[0] = dd(p.x, c.x, p2.x, m.x, r);
-    o[1] = dd(p.y, c.y, p2.y, m.y, r);
-  }
-}
-template <int R>
-__device__ __forceinline__ void own(const float* a, int b, float (&o)[R]) {
-  if constexpr (R == 1) {
-    o[0] = a[b];
-  } else {
-    const float2 c = ld2(a + b);
-    o[0] = c.x;
-    o[1] = c.y;
-  }
-}
-
-// Backward fast bodies, R adjacent depths per thread (tiles of 32 R rows):
-// the own-cell operands of all R depths are loaded before the staged tiles
-// are awaited.
-// MID: a mid tile (no CPML cell): the reverse stress update and the imaging
-// sums only at cells of the reverse-time interior, and the ring's stresses of
-// step it restored.
+// MID: the reverse stress update and the imaging sums only at cells of the
+// reverse-time interior, and the ring's stresses of step it restored.
 template <int TX, int K, int R, bool MID>
 __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST_SLOT(TZ)
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_FAST(TZ, BOXZ, R)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
   const uint64_t pol = media_policy();
   float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R], gl[R], gm[R], gt[R], va_z[R], va_x[R];
-  ldrm<R>(m.lam + i, lam, pol);
-  ldrm<R>(m.l2m + i, l2m, pol);
-  ldrm<R>(m.aveMu + i, amu, pol);
+  ldm<R>(m.lam, base, off, lam, pol);
+  ldm<R>(m.l2m, base, off, l2m, pol);
+  ldm<R>(m.aveMu, base, off, amu, pol);
   pdl_wait();
   SWEEP_TMA(5, BOXZ)
-  ldr<R>(f.szz + i, szz);
-  ldr<R>(f.sxx + i, sxx);
-  ldr<R>(f.sxz + i, sxz);
-  ldr<R>(gr.lam + i, gl);
-  ldr<R>(gr.mu + i, gm);
-  ldr<R>(gr.tau + i, gt);
-  ldr<R>(f.vz_a + i, va_z);
-  ldr<R>(f.vx_a + i, va_x);
+  ldo<R>(f.szz, base, off, szz);
+  ldo<R>(f.sxx, base, off, sxx);
+  ldo<R>(f.sxz, base, off, sxz);
+  ldo<R>(gr.lam, base, off, gl);
+  ldo<R>(gr.mu, base, off, gm);
+  ldo<R>(gr.tau, base, off, gt);
+  ldo<R>(f.vz_a, base, off, va_z);
+  ldo<R>(f.vx_a, base, off, va_x);
   if (!stage_wait(&bar, err)) return;
   const float* s_vz = sm;
   const float* s_vx = sm + N;
@@ -988,12 +878,12 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
       }
     }
   }
-  str<R>(f.szz + i, szz);
-  str<R>(f.sxx + i, sxx);
-  str<R>(f.sxz + i, sxz);
-  str<R>(gr.lam + i, gl);
-  str<R>(gr.mu + i, gm);
-  str<R>(gr.tau + i, gt);
+  sto<R>(f.szz, base, off, szz);
+  sto<R>(f.sxx, base, off, sxx);
+  sto<R>(f.sxz, base, off, sxz);
+  sto<R>(gr.lam, base, off, gl);
+  sto<R>(gr.mu, base, off, gm);
+  sto<R>(gr.tau, base, off, gt);
   // el_velocity_adj without the psi memory terms.
   {
     float d1[R], d2[R], d3[R];
@@ -1002,7 +892,7 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
     dmz<R>(s_sxz_a, b, rdz, d3);
 #pragma unroll
     for (int r = 0; r < R; ++r) va_x[r] -= (lam[r] * d1[r] + l2m[r] * d2[r] + amu[r] * d3[r]) * dt;
-    str<R>(f.vx_a + i, va_x);
+    sto<R>(f.vx_a, base, off, va_x);
   }
   {
     float d1[R], d2[R], d3[R];
@@ -1011,36 +901,34 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
     dmx<R, BOXZ>(s_sxz_a, b, rdx, d3);
 #pragma unroll
     for (int r = 0; r < R; ++r) va_z[r] -= (l2m[r] * d1[r] + lam[r] * d2[r] + amu[r] * d3[r]) * dt;
-    str<R>(f.vz_a + i, va_z);
+    sto<R>(f.vz_a, base, off, va_z);
   }
 }
 
-// MID: a mid tile (no CPML cell): the adjoint memory arrays updated in their
-// bands (el_stress_adj.cu:68-94, within 2 cells of the CPML), the reverse
-// velocity update and its imaging sums only at cells of the reverse-time
-// interior, and the ring's velocities of step it-1 restored.
+// MID: the adjoint memory arrays updated in their bands (el_stress_adj.cu:68-94,
+// within 2 cells of the CPML), the reverse velocity update and its imaging
+// sums only at cells of the reverse-time interior, and the ring's velocities
+// of step it-1 restored.
 template <int TX, int K, int R, bool MID>
 __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST_SLOT(TZ)
-  SWEEP_CELL(BOXZ, R)
-  SWEEP_SMEM(BOXZ)
+  SWEEP_FAST(TZ, BOXZ, R)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
   const bool rev = it >= 1;
   const uint64_t pol = media_policy();
   float bA[R], bB[R], sa[R], xa[R], za[R], vz[R], vx[R], ga[R], gb[R];
-  ldrm<R>(m.bycA + i, bA, pol);
-  ldrm<R>(m.bycB + i, bB, pol);
+  ldm<R>(m.bycA, base, off, bA, pol);
+  ldm<R>(m.bycB, base, off, bB, pol);
   pdl_wait();
   SWEEP_TMA(5, BOXZ)
-  ldr<R>(f.szz_a + i, sa);
-  ldr<R>(f.sxx_a + i, xa);
-  ldr<R>(f.sxz_a + i, za);
-  ldr<R>(f.vz + i, vz);
-  ldr<R>(f.vx + i, vx);
-  ldr<R>(gr.va + i, ga);
-  ldr<R>(gr.vb + i, gb);
+  ldo<R>(f.szz_a, base, off, sa);
+  ldo<R>(f.sxx_a, base, off, xa);
+  ldo<R>(f.sxz_a, base, off, za);
+  ldo<R>(f.vz, base, off, vz);
+  ldo<R>(f.vx, base, off, vx);
+  ldo<R>(gr.va, base, off, ga);
+  ldo<R>(gr.vb, base, off, gb);
   if (!stage_wait(&bar, err)) return;
   const float* s_vz_a = sm;
   const float* s_vx_a = sm + N;
@@ -1048,9 +936,9 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
   const float* s_sxx = sm + 3 * N;
   const float* s_sxz = sm + 4 * N;
   const float rdz = g.rdz, rdx = g.rdx, dt = g.dt;
+  if (special) {
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (special) inject_res(sh, it, first_receiver(sh, z + r, x), z + r, x, sa[r], xa[r]);
+    for (int r = 0; r < R; ++r) inject_res(sh, it, first_receiver(sh, z + r, x), z + r, x, sa[r], xa[r]);
   }
   {
     float d1[R], d2[R], d3[R], d4[R];
@@ -1073,7 +961,7 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
       const bool zb = (zr <= g.zband_lo) || (zr >= g.zband_hi);
       if (xb || zb) {
         const CpmlD& c = S.c;
-        const size_t ir = i + r;
+        const size_t ir = static_cast<size_t>(x) * g.ldz + zr;
         const float amu = m.aveMu[ir], lam = m.lam[ir], l2m = m.l2m[ir];
         if (xb) f.m_dvz_dx[ir] = c.b_xh[x] * f.m_dvz_dx[ir] + za[r] * amu * dt;
         if (zb) f.m_dvx_dz[ir] = c.b_zh[zr] * f.m_dvx_dz[ir] + za[r] * amu * dt;
@@ -1082,9 +970,9 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
       }
     }
   }
-  str<R>(f.sxz_a + i, za);
-  str<R>(f.szz_a + i, sa);
-  str<R>(f.sxx_a + i, xa);
+  sto<R>(f.sxz_a, base, off, za);
+  sto<R>(f.szz_a, base, off, sa);
+  sto<R>(f.sxx_a, base, off, xa);
   if (!rev) return;
   float ea[R], eb[R], t[R], wa[R], wb[R];
   dpz<R>(s_szz, b, rdz, ea);
@@ -1114,10 +1002,10 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
       }
     }
   }
-  str<R>(f.vz + i, vz);
-  str<R>(f.vx + i, vx);
-  str<R>(gr.va + i, ga);
-  str<R>(gr.vb + i, gb);
+  sto<R>(f.vz, base, off, vz);
+  sto<R>(f.vx, base, off, vx);
+  sto<R>(gr.va, base, off, ga);
+  sto<R>(gr.vb, base, off, gb);
 }
 
 // ---------------------------------------------------------------------------
@@ -1131,19 +1019,12 @@ template <int TX, int K, int R>
 __global__ void FWD_BOUNDS k_fwd_stress(const __grid_constant__ SweepPack<K> P, int it, int flags, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R)
   const bool inject = (flags & 2) != 0;
-  if (fast) {
-    if constexpr (R == 1)
-      fwd_stress_fast1<TX, K, false>(P, shot, z0, x0, it, 0, inject, err);
-    else
-      fwd_stress_fast2<TX, K, R, false>(P, shot, z0, x0, it, 0, inject, err);
-  } else if (mid) {
-    if constexpr (R == 1)
-      fwd_stress_fast1<TX, K, true>(P, shot, z0, x0, it, flags & 1, inject, err);
-    else
-      fwd_stress_fast2<TX, K, R, true>(P, shot, z0, x0, it, flags & 1, inject, err);
-  } else {
+  if (fast)
+    fwd_stress_fast<TX, K, R, false>(P, shot, z0, x0, it, 0, inject, err);
+  else if (mid)
+    fwd_stress_fast<TX, K, R, true>(P, shot, z0, x0, it, flags & 1, inject, err);
+  else
     fwd_stress_edge<TX, K, R>(P, shot, z0, x0, it, flags & 1, inject, err);
-  }
 }
 
 template <int TX, int K, int R>
@@ -1151,14 +1032,10 @@ __global__ void FWD_BOUNDS k_fwd_velocity(const __grid_constant__ SweepPack<K> P
   SWEEP_KERNEL_TILE(32 * R)
   // A mid tile of this sweep has nothing beyond the fast form: no CPML cell,
   // every cell in the stencil domain, and no ring or band work.
-  if (fast || mid) {
-    if constexpr (R == 1)
-      fwd_velocity_fast1<TX, K>(P, shot, z0, x0, err);
-    else
-      fwd_velocity_fast2<TX, K, R>(P, shot, z0, x0, err);
-  } else {
+  if (fast || mid)
+    fwd_velocity_fast<TX, K, R>(P, shot, z0, x0, err);
+  else
     fwd_velocity_edge<TX, K, R>(P, shot, z0, x0, err);
-  }
 }
 
 // Backward sweeps: R depths per thread (tiles of 32 R rows), R in {1, 2};
@@ -1166,25 +1043,23 @@ __global__ void FWD_BOUNDS k_fwd_velocity(const __grid_constant__ SweepPack<K> P
 template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R)
-  if (fast) {
+  if (fast)
     bwd_B_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
-  } else if (mid) {
+  else if (mid)
     bwd_B_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
-  } else {
+  else
     bwd_B_edge<TX, K, R>(P, shot, z0, x0, j, err);
-  }
 }
 
 template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_C(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R)
-  if (fast) {
+  if (fast)
     bwd_C_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
-  } else if (mid) {
+  else if (mid)
     bwd_C_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
-  } else {
+  else
     bwd_C_edge<TX, K, R>(P, shot, z0, x0, j, err);
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1696,7 +1571,7 @@ void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
 }
 
 dim3 sweep_grid(int tx, int tz, const SweepGrid& gr, int nshots) {
-  return dim3((gr.nz + tz - 1) / tz, (gr.nx + tx - 1) / tx, nshots);
+  return dim3((gr.nz - (tz == kTileZFwd ? gr.zoff : 0) + tz - 1) / tz, (gr.nx + tx - 1) / tx, nshots);
 }
 
 template <int K>
