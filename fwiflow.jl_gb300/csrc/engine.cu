@@ -1108,15 +1108,22 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // Whether the staged shots run as marching kernels (march.cu) rather than as
 // tile sweeps, one launch per sweep and step: small calls, of at most
 // kMarchCells cells in at most kPackShots shots (all shots of the call, so
-// that the grouping does not change the choice). Microseconds a step, marching
-// against tiles: 16k cells 9.2 / 21.1, 100k 13.0 / 22.7, 290k (one shot) 25.4 /
-// 25.2, 400k (4 and 8 shots) 31.7 / 34.8 and 33.3 / 37.6, 590k 40.0 / 39.7,
-// 970k 63 / 50.
+// that the grouping does not change the choice) of at most kMarchShotCells
+// each. Microseconds a step, marching against tiles:
+//   one shot    100k cells 11.9 / 22.1, 293k 21.2 / 25.0, 382k 26.3 / 28.8,
+//               511k 36.6 / 33.2, 970k 52.7 / 46.5
+//   2-12 shots  101k 13.3 / 24.5, 287k 22.4 / 29.2, 586k 34.0 / 38.1,
+//               608k (12 shots) 43.0 / 45.8, 684k 39.4 / 44.2
+//   16 shots    811k 54.4 / 54.4
 // Fixed tile shapes and per-sweep timing ask for the sweeps themselves.
-constexpr size_t kMarchCells = 400000;
+constexpr size_t kMarchCells = 700000, kMarchShotCells = 400000;
 bool marches(const fwigb_ctx* ctx) {
   size_t cells = 0;
-  for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
+  for (const ShotPlan& pl : ctx->plans) {
+    const size_t n = static_cast<size_t>(ctx->p.nz) * pl.nx;
+    if (n > kMarchShotCells) return false;
+    cells += n;
+  }
   return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
 }
 

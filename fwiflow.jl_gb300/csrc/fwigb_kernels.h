@@ -241,17 +241,22 @@ template <int K>
 int launch_bwd_C(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>& p, int nshots, const SweepGrid& gr,
                  int j, unsigned* err);
 // ---- marching kernels (march.cu): one launch per pass over time for up to
-// kPackShots shots. Block b belongs to the shot k with first[k] <= b <
+// kPackShots shots. Block b of a pass belongs to the shot k with first[k] <= b <
 // first[k + 1] and holds an even share of its columns.
-constexpr int kMarchThreads = 1024;
-struct MarchPack {
-  int nshots, threads, smem;
+constexpr int kMarchThreads = 512;  // threads of a block at most
+struct MarchSplit {
+  int threads, smem;
   int first[kPackShots + 1];
+};
+struct MarchPack {
+  int nshots;
+  int fwd_blocks;  // per SM in the forward pass: 1 or 2 (the backward pass: one)
+  MarchSplit fwd, bwd;
   ShotSlot slots[kPackShots];
 };
 static_assert(sizeof(MarchPack) < 32000, "march pack exceeds the kernel parameter limit");
-// Fills `first` and `threads` for a GPU of `sms` SMs (one block each); false
-// when the shots have more strips than that.
+// Fills `fwd` and `bwd` for a GPU of `sms` SMs, on which all blocks are resident
+// together; false where that cannot be.
 bool march_plan(MarchPack& p, int sms);
 // Bytes of the strips' flags; they are zeroed before each pass.
 size_t march_flag_bytes(const MarchPack& p);

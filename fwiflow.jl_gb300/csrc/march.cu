@@ -12,12 +12,22 @@
 // orders their writes before its reads, and their reads before its writes).
 // All blocks of a launch are resident together (a cooperative launch). The
 // hand-over costs 1.1 us of a sweep, the sweep itself 1-1.5 us at the smallest
-// sizes: a step of a 96 x 84 grid takes 9.1 us (21.1 with a launch per sweep),
-// of two 192 x 264 grids 15.1 us (23.8), of one 192 x 448 grid 13.0 us (22.7).
+// sizes: a step of two 96 x 84 grids takes 9.4 us (20.4 with a launch per sweep),
+// of two 192 x 264 grids 13.3 us (24.5), of one 224 x 448 grid 11.9 us (22.1), of
+// two 352 x 832 grids 34.0 us (38.1).
 //
-// A warp takes 32 depths of one column at a time and reads its stencil samples
-// from the fields themselves (L1 / L2): at these sizes the fields live in L2,
-// and staging would add its own latency.
+// A warp takes 64 depths of one column at a time, two adjacent ones a thread,
+// and reads its stencil samples from the fields themselves (L1 / L2): at these
+// sizes the fields live in L2, and staging would add its own latency. Where a
+// block's work takes several rounds of its warps it is bound by the instructions
+// of its loads and their addresses (about 150 loads a cell of a step), which
+// paired loads halve: one depth a thread took 20.1 us a step for two 224 x 448
+// grids (now 17.8) and 25.6 us for one 352 x 832 (now 21.2).
+// With several rounds the forward pass runs two blocks of 512 threads on each
+// SM, so that one works while the other waits for its neighbours (352 x 832:
+// 3.6 us for F1 and F2; 4.2 with one block). The backward pass has more operands in flight: one block with
+// 128 registers a thread (two 352 x 832 grids: 11.3 us; 13.1 with two blocks of
+// 64 registers, 12.6 with one of 640 threads).
 #include <algorithm>
 
 #include "fwigb_kernels.h"
@@ -26,6 +36,7 @@
 namespace fwigb {
 namespace {
 
+constexpr int R = 2;  // depths per thread
 constexpr unsigned kFlagStride = 32;  // words between flags: one 128-byte line each
 
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
@@ -62,21 +73,21 @@ struct Strip {
   int shot, xa, xb;        // columns [xa, xb) of the shot's sub-grid
   bool left, right;        // has a neighbour
   unsigned* flag;          // its own flag
-  int nch;                 // 32-depth chunks down to the last row a sweep touches
+  int nch;                 // 64-depth chunks down to the last row a sweep touches
 };
 
-__device__ __forceinline__ Strip strip_of(const MarchPack& P, unsigned* flags) {
+__device__ __forceinline__ Strip strip_of(const MarchPack& P, const MarchSplit& split, unsigned* flags) {
   Strip s;
   s.shot = 0;
-  while (s.shot + 1 < P.nshots && static_cast<int>(blockIdx.x) >= P.first[s.shot + 1]) ++s.shot;
-  const int j = blockIdx.x - P.first[s.shot], nb = P.first[s.shot + 1] - P.first[s.shot];
+  while (s.shot + 1 < P.nshots && static_cast<int>(blockIdx.x) >= split.first[s.shot + 1]) ++s.shot;
+  const int j = blockIdx.x - split.first[s.shot], nb = split.first[s.shot + 1] - split.first[s.shot];
   const Geo& g = P.slots[s.shot].g;
   s.xa = static_cast<int>(static_cast<long long>(j) * g.nx / nb);
   s.xb = static_cast<int>(static_cast<long long>(j + 1) * g.nx / nb);
   s.left = j > 0;
   s.right = j + 1 < nb;
   s.flag = flags + static_cast<size_t>(blockIdx.x) * kFlagStride;
-  s.nch = (min(g.nz, max(g.zact1, P.slots[s.shot].sh.rbz1) + 1) + 31) / 32;
+  s.nch = (min(g.nz, max(g.zact1, P.slots[s.shot].sh.rbz1) + 1) + 32 * R - 1) / (32 * R);
   return s;
 }
 
@@ -93,7 +104,7 @@ __device__ __forceinline__ bool strip_sync(const Strip& s, unsigned count, unsig
   return __syncthreads_and(ok);
 }
 
-// A warp's place in its block's list of work: part, then column, then 32-depth
+// A warp's place in its block's list of work: part, then column, then 64-depth
 // chunk (chunks fastest), every warp taking every blockDim.x / 32-th item.
 struct Item {
   int part, x, ch;
@@ -112,7 +123,7 @@ __device__ __forceinline__ void step_item(const Strip& s, Item& t, int n) {
 template <class F>
 __device__ __forceinline__ void for_items(const Strip& s, Item t, int parts, F fn) {
   while (t.part < parts) {
-    fn(t.part, t.ch * 32, t.x);
+    fn(t.part, t.ch * 32 * R, t.x);
     step_item(s, t, blockDim.x >> 5);
   }
 }
@@ -162,28 +173,55 @@ struct March {
   int n, mn, ldz;
   float dt, rdz, rdx;
   const float* prof;   // shared: kProfiles z profiles of nz values, then as many x profiles of w columns
-  const unsigned* info;  // shared: nch * 32 depths of each column
+  const unsigned* info;  // shared: the strip's cells, `depth` of each column
   int nz, w, xa, depth;
 };
 
-// The thread's cell of an item: its index, its depth, its column in the strip.
-struct Cell {
+// The thread's cells of an item (adjacent depths; the first one's index, depth
+// and column in the strip), what each of them is and what any of them is.
+struct Cells {
   int i, z, xl;
-  unsigned v;
+  unsigned v[R], any;
 };
-__device__ __forceinline__ Cell cell_at(const March& M, int z0, int x) {
-  Cell c;
-  c.z = z0 + (threadIdx.x & 31);
+__device__ __forceinline__ Cells cells_at(const March& M, int z0, int x) {
+  Cells c;
+  c.z = z0 + R * (threadIdx.x & 31);
   c.xl = x - M.xa;
   c.i = x * M.ldz + c.z;
-  c.v = M.info[c.xl * M.depth + c.z];
+  const unsigned* p = M.info + c.xl * M.depth + c.z;
+  const uint2 t = *reinterpret_cast<const uint2*>(p);
+  c.v[0] = t.x;
+  c.v[1] = t.y;
+  c.any = t.x | t.y;
   return c;
 }
-__device__ __forceinline__ float& fld(const March& M, const Cell& c, int q) { return M.f[c.i + q * M.n]; }
-__device__ __forceinline__ float med(const March& M, const Cell& c, int q) { return M.m[c.i + q * M.mn]; }
-__device__ __forceinline__ float& sum(const March& M, const Cell& c, int q) { return M.g[c.i + q * M.n]; }
-__device__ __forceinline__ float pz(const March& M, const Cell& c, int q) { return M.prof[q * M.nz + c.z]; }
-__device__ __forceinline__ float px(const March& M, const Cell& c, int q) { return M.prof[kProfiles * M.nz + q * M.w + c.xl]; }
+
+// Values at the thread's cells: one paired access (even depths, columns a
+// multiple of 32 floats apart).
+struct Vals {
+  float v[R];
+  __device__ __forceinline__ float& operator[](int r) { return v[r]; }
+  __device__ __forceinline__ float operator[](int r) const { return v[r]; }
+};
+__device__ __forceinline__ Vals load(const float* p) {
+  const float2 t = *reinterpret_cast<const float2*>(p);
+  return {{t.x, t.y}};
+}
+__device__ __forceinline__ Vals load_if(bool on, const float* p) {
+  Vals a{};
+  if (on) a = load(p);
+  return a;
+}
+__device__ __forceinline__ void store(float* p, const Vals& a) {
+  *reinterpret_cast<float2*>(p) = make_float2(a.v[0], a.v[1]);
+}
+__device__ __forceinline__ float* fld(const March& M, const Cells& c, int q) { return M.f + (c.i + q * M.n); }
+__device__ __forceinline__ const float* med(const March& M, const Cells& c, int q) { return M.m + (c.i + q * M.mn); }
+__device__ __forceinline__ float* sum(const March& M, const Cells& c, int q) { return M.g + (c.i + q * M.n); }
+__device__ __forceinline__ float pz(const March& M, const Cells& c, int r, int q) { return M.prof[q * M.nz + c.z + r]; }
+__device__ __forceinline__ float px(const March& M, const Cells& c, int q) {
+  return M.prof[kProfiles * M.nz + q * M.w + c.xl];
+}
 // a / K with r = 1 / K rounded: the quotient estimate a r corrected by its
 // residual, correctly rounded by Markstein's theorem (IBM J. Res. Dev. 34,
 // 1990) as the division is, without its range checks (K is in [1, 2]).
@@ -191,230 +229,322 @@ __device__ __forceinline__ float over(float a, float K, float r) {
   const float q = a * r;
   return fmaf(fmaf(-K, q, a), r, q);
 }
-__device__ __forceinline__ float over_z(const March& M, const Cell& c, float a, int h) {
-  return over(a, pz(M, c, h ? KH : K_), pz(M, c, h ? RKH : RK));
+__device__ __forceinline__ float over_z(const March& M, const Cells& c, int r, float a, int h) {
+  return over(a, pz(M, c, r, h ? KH : K_), pz(M, c, r, h ? RKH : RK));
 }
-__device__ __forceinline__ float over_x(const March& M, const Cell& c, float a, int h) {
+__device__ __forceinline__ float over_x(const March& M, const Cells& c, float a, int h) {
   return over(a, px(M, c, h ? KH : K_), px(M, c, h ? RKH : RK));
 }
-__device__ __forceinline__ float dmz(const March& M, const Cell& c, int q) { return sdm(M.f, c.i + q * M.n, 1, M.rdz); }
-__device__ __forceinline__ float dpz(const March& M, const Cell& c, int q) { return sdp(M.f, c.i + q * M.n, 1, M.rdz); }
-__device__ __forceinline__ float dmx(const March& M, const Cell& c, int q) { return sdm(M.f, c.i + q * M.n, M.ldz, M.rdx); }
-__device__ __forceinline__ float dpx(const March& M, const Cell& c, int q) { return sdp(M.f, c.i + q * M.n, M.ldz, M.rdx); }
-// The five saved values of ring row v & kRing of a step (szz, sxz, sxx, vz, vx).
-__device__ __forceinline__ float* ring_at(const March& M, const Cell& c, int it) {
-  return M.S->st.base + static_cast<size_t>(it) * 5 * M.S->g.ring_len + ((c.v & kRing) - 1);
+// Differences at the cells. Only where one of them is in the stencil domain:
+// the pair's samples then lie in the array (two columns follow the domain's last).
+__device__ __forceinline__ float diff(float p, float q, float s, float t, float r) {
+  return (C1 * (p - q) - C2 * (s - t)) * r;
+}
+__device__ __forceinline__ Vals dmz(const March& M, const Cells& c, int q) {
+  const float* a = fld(M, c, q);
+  const Vals m = load(a - 2), e = load(a), p = load(a + 2);
+  return {{diff(e[0], m[1], e[1], m[0], M.rdz), diff(e[1], e[0], p[0], m[1], M.rdz)}};
+}
+__device__ __forceinline__ Vals dpz(const March& M, const Cells& c, int q) {
+  const float* a = fld(M, c, q);
+  const Vals m = load(a - 2), e = load(a), p = load(a + 2);
+  return {{diff(e[1], e[0], p[0], m[1], M.rdz), diff(p[0], e[1], p[1], e[0], M.rdz)}};
+}
+__device__ __forceinline__ Vals dmx(const March& M, const Cells& c, int q) {
+  const float* a = fld(M, c, q);
+  const Vals e = load(a), m = load(a - M.ldz), p = load(a + M.ldz), n = load(a - 2 * M.ldz);
+  Vals o;
+#pragma unroll
+  for (int r = 0; r < R; ++r) o.v[r] = diff(e[r], m[r], p[r], n[r], M.rdx);
+  return o;
+}
+__device__ __forceinline__ Vals dpx(const March& M, const Cells& c, int q) {
+  const float* a = fld(M, c, q);
+  const Vals e = load(a), p = load(a + M.ldz), n = load(a + 2 * M.ldz), m = load(a - M.ldz);
+  Vals o;
+#pragma unroll
+  for (int r = 0; r < R; ++r) o.v[r] = diff(p[r], e[r], n[r], m[r], M.rdx);
+  return o;
+}
+// The five saved values of a cell in ring row v & kRing of a step (szz, sxz, sxx, vz, vx).
+__device__ __forceinline__ float* ring_at(const March& M, unsigned v, int it) {
+  return M.S->st.base + static_cast<size_t>(it) * 5 * M.S->g.ring_len + ((v & kRing) - 1);
 }
 
 // Each sweep is two or three independent parts (fields that no other part of
-// the sweep reads or writes), which different warps take: at these sizes a
-// sweep lasts as long as one warp's chain of dependent instructions. A part
+// the sweep reads or writes), which different warps take: at the smallest sizes
+// a sweep lasts as long as one warp's chain of dependent instructions. A part
 // loads everything it may need before it stores anything: the arrays do not
 // alias, which the compiler cannot know, and a load behind a store would cost
-// another L2 round trip.
+// another L2 round trip. A pair is loaded and stored whole when either cell
+// needs it; the other one's values go back as they came.
 
 // F1, normal stresses: szz, sxx, the source, recording, their ring samples and the velocities'.
 __device__ __forceinline__ void f1_normal(const March& M, int it, int save, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & (kDom | kRing | kSrc | kRec))) return;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & (kDom | kRing | kSrc | kRec))) return;
   const ShotD& sh = M.S->sh;
-  const bool dom = c.v & kDom, zp = c.v & kZp, xp = c.v & kXp, src = c.v & kSrc;
-  const int rec = c.v & kRec ? first_receiver(sh, c.z, x) : -1;
-  const float s1 = src ? sh.src_szz[it] : 0.0f, s2 = src ? sh.src_sxx[it] : 0.0f;
-  float szz = fld(M, c, SZZ), sxx = fld(M, c, SXX);
-  const float lam = med(M, c, LAM), l2m = med(M, c, L2M);
-  float mz = zp ? fld(M, c, M_VZ_Z) : 0.0f, mx = xp ? fld(M, c, M_VX_X) : 0.0f;
-  float dvz_dz = 0.0f, dvx_dx = 0.0f;
-  if (dom) {
-    dvz_dz = dmz(M, c, VZ);
-    dvx_dx = dmx(M, c, VX);
+  const bool zp = c.any & kZp, xp = c.any & kXp;
+  int rec[R];
+  float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+  for (int r = 0; r < R; ++r) rec[r] = c.v[r] & kRec ? first_receiver(sh, c.z + r, x) : -1;
+  if (c.any & kSrc) {
+    s1 = sh.src_szz[it];
+    s2 = sh.src_sxx[it];
   }
-  if (save && (c.v & kRing)) {
-    const float vz = fld(M, c, VZ), vx = fld(M, c, VX);
-    float* p = ring_at(M, c, it);
+  Vals szz = load(fld(M, c, SZZ)), sxx = load(fld(M, c, SXX));
+  const Vals lam = load(med(M, c, LAM)), l2m = load(med(M, c, L2M));
+  Vals mz = load_if(zp, fld(M, c, M_VZ_Z)), mx = load_if(xp, fld(M, c, M_VX_X));
+  Vals dz{}, dx{};
+  if (c.any & kDom) {
+    dz = dmz(M, c, VZ);
+    dx = dmx(M, c, VX);
+  }
+  if (save && (c.any & kRing)) {
+    const Vals vz = load(fld(M, c, VZ)), vx = load(fld(M, c, VX));
     const int len = M.S->g.ring_len;
-    p[0] = szz;
-    p[2 * len] = sxx;
-    p[3 * len] = vz;
-    p[4 * len] = vx;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c.v[r] & kRing) {
+        float* p = ring_at(M, c.v[r], it);
+        p[0] = szz[r];
+        p[2 * len] = sxx[r];
+        p[3 * len] = vz[r];
+        p[4 * len] = vx[r];
+      }
   }
-  if (zp) {
-    mz = pz(M, c, B_) * mz + pz(M, c, A_) * dvz_dz;
-    dvz_dz = over_z(M, c, dvz_dz, 0) + mz;
-    fld(M, c, M_VZ_Z) = mz;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (c.v[r] & kZp) {
+      mz[r] = pz(M, c, r, B_) * mz[r] + pz(M, c, r, A_) * dz[r];
+      dz[r] = over_z(M, c, r, dz[r], 0) + mz[r];
+    }
+    if (c.v[r] & kXp) {
+      mx[r] = px(M, c, B_) * mx[r] + px(M, c, A_) * dx[r];
+      dx[r] = over_x(M, c, dx[r], 0) + mx[r];
+    }
+    if (c.v[r] & kDom) {
+      szz[r] += (l2m[r] * dz[r] + lam[r] * dx[r]) * M.dt;
+      sxx[r] += (lam[r] * dz[r] + l2m[r] * dx[r]) * M.dt;
+    }
+    if (c.v[r] & kSrc) {
+      szz[r] += s1;
+      sxx[r] += s2;
+    }
   }
-  if (xp) {
-    mx = px(M, c, B_) * mx + px(M, c, A_) * dvx_dx;
-    dvx_dx = over_x(M, c, dvx_dx, 0) + mx;
-    fld(M, c, M_VX_X) = mx;
+  if (zp) store(fld(M, c, M_VZ_Z), mz);
+  if (xp) store(fld(M, c, M_VX_X), mx);
+  if (c.any & (kDom | kSrc)) {
+    store(fld(M, c, SZZ), szz);
+    store(fld(M, c, SXX), sxx);
   }
-  if (dom) {
-    szz += (l2m * dvz_dz + lam * dvx_dx) * M.dt;
-    sxx += (lam * dvz_dz + l2m * dvx_dx) * M.dt;
-  }
-  if (src) {
-    szz += s1;
-    sxx += s2;
-  }
-  if (dom || src) {
-    fld(M, c, SZZ) = szz;
-    fld(M, c, SXX) = sxx;
-  }
-  record(sh, it, rec, c.z, x, szz, sxx);
+#pragma unroll
+  for (int r = 0; r < R; ++r) record(sh, it, rec[r], c.z + r, x, szz[r], sxx[r]);
 }
 
 // F1, shear stress.
 __device__ __forceinline__ void f1_shear(const March& M, int it, int save, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & (kDom | kRing))) return;
-  const bool dom = c.v & kDom, zp = c.v & kZp, xp = c.v & kXp;
-  const float sxz = fld(M, c, SXZ), amu = med(M, c, AMU);
-  float mz = zp ? fld(M, c, M_VX_Z) : 0.0f, mx = xp ? fld(M, c, M_VZ_X) : 0.0f;
-  if (save && (c.v & kRing)) ring_at(M, c, it)[M.S->g.ring_len] = sxz;
-  if (!dom) return;
-  float dvx_dz = dpz(M, c, VX), dvz_dx = dpx(M, c, VZ);
-  if (zp) {
-    mz = pz(M, c, BH) * mz + pz(M, c, AH) * dvx_dz;
-    dvx_dz = over_z(M, c, dvx_dz, 1) + mz;
-    fld(M, c, M_VX_Z) = mz;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & (kDom | kRing))) return;
+  const bool zp = c.any & kZp, xp = c.any & kXp;
+  Vals sxz = load(fld(M, c, SXZ));
+  const Vals amu = load(med(M, c, AMU));
+  Vals mz = load_if(zp, fld(M, c, M_VX_Z)), mx = load_if(xp, fld(M, c, M_VZ_X));
+  if (save) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c.v[r] & kRing) ring_at(M, c.v[r], it)[M.S->g.ring_len] = sxz[r];
   }
-  if (xp) {
-    mx = px(M, c, BH) * mx + px(M, c, AH) * dvz_dx;
-    dvz_dx = over_x(M, c, dvz_dx, 1) + mx;
-    fld(M, c, M_VZ_X) = mx;
+  if (!(c.any & kDom)) return;
+  Vals dz = dpz(M, c, VX), dx = dpx(M, c, VZ);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (c.v[r] & kZp) {
+      mz[r] = pz(M, c, r, BH) * mz[r] + pz(M, c, r, AH) * dz[r];
+      dz[r] = over_z(M, c, r, dz[r], 1) + mz[r];
+    }
+    if (c.v[r] & kXp) {
+      mx[r] = px(M, c, BH) * mx[r] + px(M, c, AH) * dx[r];
+      dx[r] = over_x(M, c, dx[r], 1) + mx[r];
+    }
+    if (c.v[r] & kDom) sxz[r] = sxz[r] + amu[r] * (dz[r] + dx[r]) * M.dt;
   }
-  fld(M, c, SXZ) = sxz + amu * (dvx_dz + dvz_dx) * M.dt;
+  if (zp) store(fld(M, c, M_VX_Z), mz);
+  if (xp) store(fld(M, c, M_VZ_X), mx);
+  store(fld(M, c, SXZ), sxz);
 }
 
-// F2, one velocity component (0 outside the stencil domain): vz from dszz/dz (half-point profile) and dsxz/dx, or
-// vx from dsxz/dz and dsxx/dx (half-point profile).
+// F2, one velocity component: vz from dszz/dz (half-point profile) and dsxz/dx, or vx from dsxz/dz and dsxx/dx
+// (half-point profile). Only cells with one of the pair in the stencil domain.
 template <bool Z>
-__device__ __forceinline__ float f2_velocity(const March& M, const Cell& c) {
-  if (!(c.v & kDom)) return 0.0f;
-  const bool zp = c.v & kZp, xp = c.v & kXpV;
+__device__ __forceinline__ Vals f2_velocity(const March& M, const Cells& c) {
+  const bool zp = c.any & kZp, xp = c.any & kXpV;
   constexpr int V = Z ? VZ : VX, MZ = Z ? M_SZZ_Z : M_SXZ_Z, MX = Z ? M_SXZ_X : M_SXX_X;
   constexpr int hz = Z ? 3 : 0, hx = Z ? 0 : 3;  // half-point profiles
-  const float old = fld(M, c, V), by = med(M, c, Z ? BYA : BYB);
-  float mz = zp ? fld(M, c, MZ) : 0.0f, mx = xp ? fld(M, c, MX) : 0.0f;
-  float dz = Z ? dpz(M, c, SZZ) : dmz(M, c, SXZ);
-  float dx = Z ? dmx(M, c, SXZ) : dpx(M, c, SXX);
-  if (zp) {
-    mz = pz(M, c, B_ + hz) * mz + pz(M, c, A_ + hz) * dz;
-    dz = over_z(M, c, dz, hz) + mz;
-    fld(M, c, MZ) = mz;
+  Vals v = load(fld(M, c, V));
+  const Vals by = load(med(M, c, Z ? BYA : BYB));
+  Vals mz = load_if(zp, fld(M, c, MZ)), mx = load_if(xp, fld(M, c, MX));
+  Vals dz = Z ? dpz(M, c, SZZ) : dmz(M, c, SXZ);
+  Vals dx = Z ? dmx(M, c, SXZ) : dpx(M, c, SXX);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (c.v[r] & kZp) {
+      mz[r] = pz(M, c, r, B_ + hz) * mz[r] + pz(M, c, r, A_ + hz) * dz[r];
+      dz[r] = over_z(M, c, r, dz[r], hz) + mz[r];
+    }
+    if (c.v[r] & kXpV) {
+      mx[r] = px(M, c, B_ + hx) * mx[r] + px(M, c, A_ + hx) * dx[r];
+      dx[r] = over_x(M, c, dx[r], hx) + mx[r];
+    }
+    if (c.v[r] & kDom) v[r] = v[r] + (dz[r] + dx[r]) * by[r] * M.dt;
   }
-  if (xp) {
-    mx = px(M, c, B_ + hx) * mx + px(M, c, A_ + hx) * dx;
-    dx = over_x(M, c, dx, hx) + mx;
-    fld(M, c, MX) = mx;
-  }
-  const float v = old + (dz + dx) * by * M.dt;
-  fld(M, c, V) = v;
+  if (zp) store(fld(M, c, MZ), mz);
+  if (xp) store(fld(M, c, MX), mx);
+  store(fld(M, c, V), v);
   return v;
+}
+template <bool Z>
+__device__ __forceinline__ void f2_part(const March& M, int z0, int x) {
+  const Cells c = cells_at(M, z0, x);
+  if (c.any & kDom) f2_velocity<Z>(M, c);
 }
 
 // F2 with the illumination, which takes both components.
-__device__ __forceinline__ void f2_illum(const March& M, const Cell& c) {
-  if (!(c.v & kDom)) return;
-  const float e = sum(M, c, G_ILLUM);
-  const float nvz = f2_velocity<true>(M, c), nvx = f2_velocity<false>(M, c);
-  sum(M, c, G_ILLUM) = e + (nvz * nvz + nvx * nvx);
+__device__ __forceinline__ void f2_illum(const March& M, int z0, int x) {
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & kDom)) return;
+  Vals e = load(sum(M, c, G_ILLUM));
+  const Vals vz = f2_velocity<true>(M, c), vx = f2_velocity<false>(M, c);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (c.v[r] & kDom) e[r] = e[r] + (vz[r] * vz[r] + vx[r] * vx[r]);
+  store(sum(M, c, G_ILLUM), e);
 }
 
 // B, forward fields: source removal, reverse stresses, the sums of the lambda and mu kernels, the ring's stresses.
 __device__ __forceinline__ void b_stress(const March& M, int it, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & (kInner | kSrc | kRing))) return;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & (kInner | kSrc | kRing))) return;
   const ShotD& sh = M.S->sh;
-  const bool src = c.v & kSrc, ring = c.v & kRing;
-  const float s1 = src ? sh.src_szz_r[it] : 0.0f, s2 = src ? sh.src_sxx_r[it] : 0.0f;
-  float szz = fld(M, c, SZZ), sxx = fld(M, c, SXX), sxz = fld(M, c, SXZ), r0 = 0.0f, r1 = 0.0f, r2 = 0.0f;
-  if (ring) {
-    const float* p = ring_at(M, c, it);
-    const int len = M.S->g.ring_len;
-    r0 = p[0];
-    r1 = p[len];
-    r2 = p[2 * len];
+  float s1 = 0.0f, s2 = 0.0f, ring[3][R];
+  if (c.any & kSrc) {
+    s1 = sh.src_szz_r[it];
+    s2 = sh.src_sxx_r[it];
   }
-  if (src) {
-    szz -= s1;
-    sxx -= s2;
+  Vals szz = load(fld(M, c, SZZ)), sxx = load(fld(M, c, SXX)), sxz = load(fld(M, c, SXZ));
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (c.v[r] & kRing) {
+      const float* p = ring_at(M, c.v[r], it);
+      const int len = M.S->g.ring_len;
+      ring[0][r] = p[0];
+      ring[1][r] = p[len];
+      ring[2][r] = p[2 * len];
+    }
+  if (c.any & kInner) {
+    const float dt = M.dt;
+    const Vals lam = load(med(M, c, LAM)), l2m = load(med(M, c, L2M)), amu = load(med(M, c, AMU));
+    Vals gl = load(sum(M, c, G_LAM)), gm = load(sum(M, c, G_MU)), gt = load(sum(M, c, G_TAU));
+    const Vals sa = load(fld(M, c, SZZ_A)), xa = load(fld(M, c, SXX_A)), za = load(fld(M, c, SXZ_A));
+    const Vals a = dmz(M, c, VZ), b = dmx(M, c, VX), e1 = dpz(M, c, VX), e2 = dpx(M, c, VZ);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (c.v[r] & kSrc) {
+        szz[r] -= s1;
+        sxx[r] -= s2;
+      }
+      if (c.v[r] & kInner) {
+        const float e = e1[r] + e2[r];  // dvx_dz + dvz_dx
+        szz[r] -= (l2m[r] * a[r] + lam[r] * b[r]) * dt;
+        sxx[r] -= (lam[r] * a[r] + l2m[r] * b[r]) * dt;
+        sxz[r] -= amu[r] * e * dt;
+        gl[r] += (sa[r] + xa[r]) * (a[r] + b[r]);
+        gm[r] += sa[r] * a[r] + xa[r] * b[r];
+        gt[r] += za[r] * e;
+      }
+    }
+    store(sum(M, c, G_LAM), gl);
+    store(sum(M, c, G_MU), gm);
+    store(sum(M, c, G_TAU), gt);
+  } else if (c.any & kSrc) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c.v[r] & kSrc) {
+        szz[r] -= s1;
+        sxx[r] -= s2;
+      }
   }
-  if (c.v & kInner) {
-    const float lam = med(M, c, LAM), l2m = med(M, c, L2M), amu = med(M, c, AMU), dt = M.dt;
-    const float gl = sum(M, c, G_LAM), gm = sum(M, c, G_MU), gt = sum(M, c, G_TAU);
-    const float sa = fld(M, c, SZZ_A), xa = fld(M, c, SXX_A), za = fld(M, c, SXZ_A);
-    const float dvz_dz = dmz(M, c, VZ), dvx_dx = dmx(M, c, VX), e = dpz(M, c, VX) + dpx(M, c, VZ);
-    szz -= (l2m * dvz_dz + lam * dvx_dx) * dt;
-    sxx -= (lam * dvz_dz + l2m * dvx_dx) * dt;
-    sxz -= amu * e * dt;
-    sum(M, c, G_LAM) = gl + (sa + xa) * (dvz_dz + dvx_dx);
-    sum(M, c, G_MU) = gm + (sa * dvz_dz + xa * dvx_dx);
-    sum(M, c, G_TAU) = gt + za * e;
-  }
-  fld(M, c, SZZ) = ring ? r0 : szz;
-  fld(M, c, SXZ) = ring ? r1 : sxz;
-  fld(M, c, SXX) = ring ? r2 : sxx;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (c.v[r] & kRing) {
+      szz[r] = ring[0][r];
+      sxz[r] = ring[1][r];
+      sxx[r] = ring[2][r];
+    }
+  store(fld(M, c, SZZ), szz);
+  store(fld(M, c, SXZ), sxz);
+  store(fld(M, c, SXX), sxx);
 }
 
 // B, one adjoint velocity component (el_velocity_adj.cu:57-102) with the memory arrays it feeds; the psi memory terms
-// are read only where their CPML coefficient is non-zero. vx_a: normal stresses differ along x (a_x, K_x), the shear
-// stress along z (a_zh, K_zh); vz_a: along z (a_z, K_z) and x (a_xh, K_xh).
+// are read only where their CPML coefficient may be non-zero. vx_a: normal stresses differ along x (a_x, K_x), the
+// shear stress along z (a_zh, K_zh); vz_a: along z (a_z, K_z) and x (a_xh, K_xh).
 template <bool X>
 __device__ __forceinline__ void b_velocity(const March& M, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & kDom)) return;
-  const bool zp = c.v & kZp, xp = c.v & kXp;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & kDom)) return;
+  const bool zp = c.any & kZp, xp = c.any & kXp;
   constexpr int V = X ? VX_A : VZ_A, MX = X ? M_SXX_X : M_SXZ_X, MZ = X ? M_SXZ_Z : M_SZZ_Z;
-  const float dt = M.dt, lam = med(M, c, LAM), l2m = med(M, c, L2M), amu = med(M, c, AMU);
-  const float mx = xp ? fld(M, c, MX) : 0.0f, mz = zp ? fld(M, c, MZ) : 0.0f;
-  const float by = xp || zp ? med(M, c, X ? BYB : BYA) : 0.0f;
-  float v = fld(M, c, V), q1 = 0.0f, q2 = 0.0f;
-  const bool band = c.v & (kXb | kZb);  // (a = 0 and K = 1 outside the bands)
-  if (c.v & (X ? kXb : kZb)) q1 = X ? dpx(M, c, M_VX_X) : dpz(M, c, M_VZ_Z);
-  if (c.v & (X ? kZb : kXb)) q2 = X ? dmz(M, c, M_VX_Z) : dmx(M, c, M_VZ_X);
-  const float dzz = X ? dpx(M, c, SZZ_A) : dpz(M, c, SZZ_A);
-  const float dxx = X ? dpx(M, c, SXX_A) : dpz(M, c, SXX_A);
-  const float dxz = X ? dmz(M, c, SXZ_A) : dmx(M, c, SXZ_A);
-  float tn = (X ? lam * dzz + l2m * dxx : l2m * dzz + lam * dxx), ts = amu * dxz, t = 0.0f;
-  if (band) {
-    const float an = X ? px(M, c, A_) : pz(M, c, A_), as = X ? pz(M, c, AH) : px(M, c, AH);
-    t = (an != 0.0f ? an * q1 : 0.0f) + (as != 0.0f ? as * q2 : 0.0f);
-    tn = X ? over_x(M, c, tn, 0) : over_z(M, c, tn, 0);
-    ts = X ? over_z(M, c, ts, 1) : over_x(M, c, ts, 1);
+  const float dt = M.dt;
+  const Vals lam = load(med(M, c, LAM)), l2m = load(med(M, c, L2M)), amu = load(med(M, c, AMU));
+  Vals mx = load_if(xp, fld(M, c, MX)), mz = load_if(zp, fld(M, c, MZ));
+  const Vals by = load_if(xp || zp, med(M, c, X ? BYB : BYA));
+  Vals v = load(fld(M, c, V)), q1{}, q2{};
+  if (c.any & (X ? kXb : kZb)) q1 = X ? dpx(M, c, M_VX_X) : dpz(M, c, M_VZ_Z);
+  if (c.any & (X ? kZb : kXb)) q2 = X ? dmz(M, c, M_VX_Z) : dmx(M, c, M_VZ_X);
+  const Vals dzz = X ? dpx(M, c, SZZ_A) : dpz(M, c, SZZ_A);
+  const Vals dxx = X ? dpx(M, c, SXX_A) : dpz(M, c, SXX_A);
+  const Vals dxz = X ? dmz(M, c, SXZ_A) : dmx(M, c, SXZ_A);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (!(c.v[r] & kDom)) continue;
+    float tn = X ? lam[r] * dzz[r] + l2m[r] * dxx[r] : l2m[r] * dzz[r] + lam[r] * dxx[r];
+    float ts = amu[r] * dxz[r], t = 0.0f;
+    if (c.v[r] & (kXb | kZb)) {  // (a = 0 and K = 1 outside the bands)
+      const float an = X ? px(M, c, A_) : pz(M, c, r, A_), as = X ? pz(M, c, r, AH) : px(M, c, AH);
+      t = (an != 0.0f ? an * q1[r] : 0.0f) + (as != 0.0f ? as * q2[r] : 0.0f);
+      tn = X ? over_x(M, c, tn, 0) : over_z(M, c, r, tn, 0);
+      ts = X ? over_z(M, c, r, ts, 1) : over_x(M, c, ts, 1);
+    }
+    v[r] -= (tn + ts) * dt + t;
+    if (c.v[r] & kXp) mx[r] = px(M, c, X ? BH : B_) * mx[r] + by[r] * v[r] * dt;
+    if (c.v[r] & kZp) mz[r] = pz(M, c, r, X ? B_ : BH) * mz[r] + by[r] * v[r] * dt;
   }
-  v -= (tn + ts) * dt + t;
-  fld(M, c, V) = v;
-  if (xp) fld(M, c, MX) = px(M, c, X ? BH : B_) * mx + by * v * dt;
-  if (zp) fld(M, c, MZ) = pz(M, c, X ? B_ : BH) * mz + by * v * dt;
+  store(fld(M, c, V), v);
+  if (xp) store(fld(M, c, MX), mx);
+  if (zp) store(fld(M, c, MZ), mz);
 }
 
 // C, adjoint stresses: residual injection, el_stress_adj.cu:53-97 with the memory arrays in their bands (within two
 // cells of the CPML), and the source gradient.
 __device__ __forceinline__ void c_stress(const March& M, int it, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & (kDom | kRec))) return;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & (kDom | kRec))) return;
   const ShotD& sh = M.S->sh;
-  const bool dom = c.v & kDom, xb = c.v & kXb, zb = c.v & kZb;
-  const int rec = c.v & kRec ? first_receiver(sh, c.z, x) : -1;
-  float sa = fld(M, c, SZZ_A), xa = fld(M, c, SXX_A), za = fld(M, c, SXZ_A);
-  const float bA = med(M, c, BYA), bB = med(M, c, BYB), dt = M.dt;
-  float m1 = 0.0f, m2 = 0.0f, m3 = 0.0f, m4 = 0.0f, amu = 0.0f, lam = 0.0f, l2m = 0.0f;
-  if (xb) {
-    m1 = fld(M, c, M_VZ_X);
-    m2 = fld(M, c, M_VX_X);
-  }
-  if (zb) {
-    m3 = fld(M, c, M_VX_Z);
-    m4 = fld(M, c, M_VZ_Z);
-  }
-  if (xb || zb) {
-    amu = med(M, c, AMU);
-    lam = med(M, c, LAM);
-    l2m = med(M, c, L2M);
-  }
-  if (dom) {
-    float q1 = 0.0f, q2 = 0.0f, q3 = 0.0f, q4 = 0.0f;
+  const bool xb = c.any & kXb, zb = c.any & kZb;
+  int rec[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) rec[r] = c.v[r] & kRec ? first_receiver(sh, c.z + r, x) : -1;
+  Vals sa = load(fld(M, c, SZZ_A)), xa = load(fld(M, c, SXX_A)), za = load(fld(M, c, SXZ_A));
+  const Vals bA = load(med(M, c, BYA)), bB = load(med(M, c, BYB));
+  const float dt = M.dt;
+  Vals m1 = load_if(xb, fld(M, c, M_VZ_X)), m2 = load_if(xb, fld(M, c, M_VX_X));
+  Vals m3 = load_if(zb, fld(M, c, M_VX_Z)), m4 = load_if(zb, fld(M, c, M_VZ_Z));
+  const Vals amu = load_if(xb || zb, med(M, c, AMU)), lam = load_if(xb || zb, med(M, c, LAM)),
+                l2m = load_if(xb || zb, med(M, c, L2M));
+  Vals d1{}, d2{}, d3{}, d4{}, q1{}, q2{}, q3{}, q4{};
+  if (c.any & kDom) {
     if (xb) {
       q1 = dpx(M, c, M_SXZ_X);
       q3 = dmx(M, c, M_SXX_X);
@@ -423,55 +553,84 @@ __device__ __forceinline__ void c_stress(const March& M, int it, int z0, int x) 
       q2 = dpz(M, c, M_SXZ_Z);
       q4 = dmz(M, c, M_SZZ_Z);
     }
-    float d1 = dpx(M, c, VZ_A), d2 = dpz(M, c, VX_A), d3 = dmx(M, c, VX_A), d4 = dmz(M, c, VZ_A);
-    float t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
-    if (xb || zb) {
-      const float ax = px(M, c, A_), az = pz(M, c, A_), axh = px(M, c, AH), azh = pz(M, c, AH);
-      t1 = (ax != 0.0f ? ax * q1 : 0.0f) + (az != 0.0f ? az * q2 : 0.0f);
-      t2 = axh != 0.0f ? axh * q3 : 0.0f;
-      t3 = azh != 0.0f ? azh * q4 : 0.0f;
-      d1 = over_x(M, c, d1, 0);
-      d2 = over_z(M, c, d2, 0);
-      d3 = over_x(M, c, d3, 1);
-      d4 = over_z(M, c, d4, 1);
-    }
-    inject_res(sh, it, rec, c.z, x, sa, xa);
-    za -= (d1 * bA + d2 * bB) * dt + t1;
-    xa -= bB * d3 * dt + t2;
-    sa -= bA * d4 * dt + t3;
-    if (xb) {
-      fld(M, c, M_VZ_X) = px(M, c, BH) * m1 + za * amu * dt;
-      fld(M, c, M_VX_X) = px(M, c, B_) * m2 + (lam * sa + l2m * xa) * dt;
-    }
-    if (zb) {
-      fld(M, c, M_VX_Z) = pz(M, c, BH) * m3 + za * amu * dt;
-      fld(M, c, M_VZ_Z) = pz(M, c, B_) * m4 + (l2m * sa + lam * xa) * dt;
-    }
-    fld(M, c, SXZ_A) = za;
-  } else {
-    inject_res(sh, it, rec, c.z, x, sa, xa);
+    d1 = dpx(M, c, VZ_A);
+    d2 = dpz(M, c, VX_A);
+    d3 = dmx(M, c, VX_A);
+    d4 = dmz(M, c, VZ_A);
   }
-  fld(M, c, SZZ_A) = sa;
-  fld(M, c, SXX_A) = xa;
-  if (it >= 1 && (c.v & kSrc)) sh.gstf[it - 1] = -(sa + 3.0f * xa) * dt;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    inject_res(sh, it, rec[r], c.z + r, x, sa[r], xa[r]);
+    if (!(c.v[r] & kDom)) continue;
+    float t1 = 0.0f, t2 = 0.0f, t3 = 0.0f;
+    if (c.v[r] & (kXb | kZb)) {
+      const float ax = px(M, c, A_), az = pz(M, c, r, A_), axh = px(M, c, AH), azh = pz(M, c, r, AH);
+      t1 = (ax != 0.0f ? ax * q1[r] : 0.0f) + (az != 0.0f ? az * q2[r] : 0.0f);
+      t2 = axh != 0.0f ? axh * q3[r] : 0.0f;
+      t3 = azh != 0.0f ? azh * q4[r] : 0.0f;
+      d1[r] = over_x(M, c, d1[r], 0);
+      d2[r] = over_z(M, c, r, d2[r], 0);
+      d3[r] = over_x(M, c, d3[r], 1);
+      d4[r] = over_z(M, c, r, d4[r], 1);
+    }
+    za[r] -= (d1[r] * bA[r] + d2[r] * bB[r]) * dt + t1;
+    xa[r] -= bB[r] * d3[r] * dt + t2;
+    sa[r] -= bA[r] * d4[r] * dt + t3;
+    if (c.v[r] & kXb) {
+      m1[r] = px(M, c, BH) * m1[r] + za[r] * amu[r] * dt;
+      m2[r] = px(M, c, B_) * m2[r] + (lam[r] * sa[r] + l2m[r] * xa[r]) * dt;
+    }
+    if (c.v[r] & kZb) {
+      m3[r] = pz(M, c, r, BH) * m3[r] + za[r] * amu[r] * dt;
+      m4[r] = pz(M, c, r, B_) * m4[r] + (l2m[r] * sa[r] + lam[r] * xa[r]) * dt;
+    }
+  }
+  if (xb) {
+    store(fld(M, c, M_VZ_X), m1);
+    store(fld(M, c, M_VX_X), m2);
+  }
+  if (zb) {
+    store(fld(M, c, M_VX_Z), m3);
+    store(fld(M, c, M_VZ_Z), m4);
+  }
+  if (c.any & kDom) store(fld(M, c, SXZ_A), za);
+  store(fld(M, c, SZZ_A), sa);
+  store(fld(M, c, SXX_A), xa);
+  if (it >= 1 && (c.any & kSrc)) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c.v[r] & kSrc) sh.gstf[it - 1] = -(sa[r] + 3.0f * xa[r]) * dt;
+  }
 }
 
 // C, one forward velocity component taken back to step it - 1 (it >= 1) with its sum of the rho kernel and the ring.
 template <bool Z>
 __device__ __forceinline__ void c_velocity(const March& M, int it, int z0, int x) {
-  const Cell c = cell_at(M, z0, x);
-  if (!(c.v & (kInner | kRing))) return;
-  const bool ring = c.v & kRing;
-  constexpr int V = Z ? VZ : VX;
-  float v = fld(M, c, V), r = 0.0f;
-  if (ring) r = ring_at(M, c, it - 1)[(Z ? 3 : 4) * M.S->g.ring_len];
-  if (c.v & kInner) {
-    const float by = med(M, c, Z ? BYA : BYB), w = fld(M, c, Z ? VZ_A : VX_A), a = sum(M, c, Z ? G_VA : G_VB);
-    const float e = Z ? dpz(M, c, SZZ) + dmx(M, c, SXZ) : dmz(M, c, SXZ) + dpx(M, c, SXX);
-    v -= e * by * M.dt;
-    sum(M, c, Z ? G_VA : G_VB) = a + w * e;
+  const Cells c = cells_at(M, z0, x);
+  if (!(c.any & (kInner | kRing))) return;
+  constexpr int V = Z ? VZ : VX, G = Z ? G_VA : G_VB;
+  Vals v = load(fld(M, c, V));
+  float ring[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (c.v[r] & kRing) ring[r] = ring_at(M, c.v[r], it - 1)[(Z ? 3 : 4) * M.S->g.ring_len];
+  if (c.any & kInner) {
+    const Vals by = load(med(M, c, Z ? BYA : BYB)), w = load(fld(M, c, Z ? VZ_A : VX_A));
+    Vals a = load(sum(M, c, G));
+    const Vals e1 = Z ? dpz(M, c, SZZ) : dmz(M, c, SXZ), e2 = Z ? dmx(M, c, SXZ) : dpx(M, c, SXX);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (c.v[r] & kInner) {
+        const float e = e1[r] + e2[r];
+        v[r] -= e * by[r] * M.dt;
+        a[r] += w[r] * e;
+      }
+    store(sum(M, c, G), a);
   }
-  fld(M, c, V) = ring ? r : v;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (c.v[r] & kRing) v[r] = ring[r];
+  store(fld(M, c, V), v);
 }
 
 // Sets a block up: its strip's CPML profiles (which would otherwise come from
@@ -491,11 +650,11 @@ __device__ __forceinline__ March set_up(const ShotSlot& S, const Strip& s, float
   M.nz = S.g.nz;
   M.w = s.xb - s.xa;
   M.xa = s.xa;
-  M.depth = s.nch * 32;
+  M.depth = s.nch * 32 * R;
   const float* gz[6] = {S.c.K_z, S.c.a_z, S.c.b_z, S.c.K_zh, S.c.a_zh, S.c.b_zh};
   const float* gx[6] = {S.c.K_x, S.c.a_x, S.c.b_x, S.c.K_xh, S.c.a_xh, S.c.b_xh};
   float* sx = sm + kProfiles * M.nz;
-  unsigned* info = reinterpret_cast<unsigned*>(sx + kProfiles * M.w);
+  unsigned* info = reinterpret_cast<unsigned*>(sm + (kProfiles * (M.nz + M.w) + 1) / 2 * 2);  // (8-byte aligned)
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
     for (int i = threadIdx.x; i < M.nz; i += blockDim.x) sm[q * M.nz + i] = gz[q][i];
@@ -515,12 +674,13 @@ __device__ __forceinline__ March set_up(const ShotSlot& S, const Strip& s, float
 
 // One forward pass of every shot of the pack over its own record. flags: bit 0
 // saves the boundary ring, bit 1 is the timeout test hook (the first block
-// gives up its first wait and raises err; the others follow).
-__global__ void __launch_bounds__(kMarchThreads, 1)
+// gives up its first wait and raises err; the others follow). B: blocks per SM.
+template <int B>
+__global__ void __launch_bounds__(kMarchThreads, B)
     k_march_fwd(const __grid_constant__ MarchPack P, int flags, unsigned* done, unsigned* err) {
-  const Strip s = strip_of(P, done);
+  const Strip s = strip_of(P, P.fwd, done);
   const ShotSlot& S = P.slots[s.shot];
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const March M = set_up(S, s, sm);
   const int n = S.nSteps;
   Item first{0, s.xa, 0};
@@ -538,13 +698,13 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
     }
     if (!strip_sync(s, 2 * it + 1, err)) return;
     if (S.gr.illum)
-      for_items(s, first, 1, [&](int, int z0, int x) { f2_illum(M, cell_at(M, z0, x)); });
+      for_items(s, first, 1, [&](int, int z0, int x) { f2_illum(M, z0, x); });
     else
       for_items(s, first, 2, [&](int part, int z0, int x) {
         if (part == 0)
-          f2_velocity<true>(M, cell_at(M, z0, x));
+          f2_part<true>(M, z0, x);
         else
-          f2_velocity<false>(M, cell_at(M, z0, x));
+          f2_part<false>(M, z0, x);
       });
     if (!strip_sync(s, 2 * it + 2, err)) return;
   }
@@ -554,9 +714,9 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
 // to the first (backward iteration j: step nSteps - 2 - j).
 __global__ void __launch_bounds__(kMarchThreads, 1)
     k_march_bwd(const __grid_constant__ MarchPack P, unsigned* done, unsigned* err) {
-  const Strip s = strip_of(P, done);
+  const Strip s = strip_of(P, P.bwd, done);
   const ShotSlot& S = P.slots[s.shot];
-  extern __shared__ float sm[];
+  extern __shared__ __align__(16) float sm[];
   const March M = set_up(S, s, sm);
   const int n = S.nSteps;
   Item first{0, s.xa, 0};
@@ -592,55 +752,72 @@ __global__ void __launch_bounds__(kMarchThreads, 1)
 }  // namespace
 
 size_t march_flag_bytes(const MarchPack& p) {
-  return static_cast<size_t>(p.first[p.nshots]) * kFlagStride * sizeof(unsigned);
+  return static_cast<size_t>(std::max(p.fwd.first[p.nshots], p.bwd.first[p.nshots])) * kFlagStride * sizeof(unsigned);
 }
 
-bool march_plan(MarchPack& p, int sms) {
-  // The narrowest strips that are all resident with one block per SM; at least
-  // 2 columns, because a stencil reaches two into the next strip. (A 96 x 84
-  // grid takes 9.1 / 9.8 / 10.5 / 13.7 us a step with strips of 2 / 3 / 4 / 6.)
-  int total = 0, chunks = 1;
+namespace {
+// Cuts the shots into at most `blocks` strips, the narrowest such ones; at
+// least 2 columns, because a stencil reaches two into the next strip. (A
+// 96 x 84 grid takes 9.1 / 9.8 / 10.5 / 13.7 us a step with strips of
+// 2 / 3 / 4 / 6.) Returns the rounds of a block's warps in a sweep; 0 when
+// there are more shots than that or a strip's flags and profiles do not fit
+// its shared memory.
+int split_shots(const MarchPack& p, int blocks, int parts, MarchSplit& split) {
+  int total = 0, rows = 1;
   for (int k = 0; k < p.nshots; ++k) {
     const Geo& g = p.slots[k].g;
     total += g.nx;
-    chunks = std::max(chunks, (std::min(g.nz, std::max(g.zact1, p.slots[k].sh.rbz1) + 1) + 31) / 32);
+    rows = std::max(rows, std::min(g.nz, std::max(g.zact1, p.slots[k].sh.rbz1) + 1));
+  }
+  for (int w = 2; w <= total; ++w) {
+    int n = 0, widest = 0;
+    for (int k = 0; k < p.nshots; ++k) {
+      const int nx = p.slots[k].g.nx, nb = std::max(1, nx / w);  // (widths w or more)
+      split.first[k] = n;
+      n += nb;
+      widest = std::max(widest, (nx + nb - 1) / nb);
+    }
+    split.first[p.nshots] = n;
+    if (n > blocks) continue;
+    const int chunks = (rows + 32 * R - 1) / (32 * R);
+    const int items = parts * widest * chunks, warps = std::max(4, std::min(kMarchThreads / 32, items));
+    split.threads = 32 * warps;
+    split.smem = static_cast<int>((kProfiles * (p.slots[0].g.nz + widest) + 1 + widest * chunks * 32 * R) *
+                                  sizeof(float));
+    return split.smem <= 48 * 1024 ? (items + warps - 1) / warps : 0;
+  }
+  return 0;
+}
+}  // namespace
+
+bool march_plan(MarchPack& p, int sms) {
+  for (int k = 0; k < p.nshots; ++k) {
     // Ring rows and offsets from the bases fit their 21 and 31 bits.
+    const Geo& g = p.slots[k].g;
     const long long media = p.slots[k].m.aveMu - p.slots[k].m.l2m;
     if (g.ring_len >= 1 << 21 || 18ll * g.ldz * g.nx >= 1ll << 31 || 8 * media >= 1ll << 31) return false;
   }
-  for (int w = 2; w <= total; ++w) {
-    int n = 0;
-    for (int k = 0; k < p.nshots; ++k) {
-      p.first[k] = n;
-      n += std::max(1, p.slots[k].g.nx / w);  // (widths w or more)
-    }
-    p.first[p.nshots] = n;
-    if (n > sms) continue;
-    int widest = 0;
-    for (int k = 0; k < p.nshots; ++k) {
-      const int nb = p.first[k + 1] - p.first[k];
-      widest = std::max(widest, (p.slots[k].g.nx + nb - 1) / nb);
-    }
-    p.threads = 32 * std::max(4, std::min(kMarchThreads / 32, 3 * widest * chunks));
-    p.smem = static_cast<int>((kProfiles * (p.slots[0].g.nz + widest) + widest * chunks * 32) * sizeof(float));
-    return p.smem <= 48 * 1024;
-  }
-  return false;
+  // Two blocks per SM in the forward pass, unless one of more registers has a
+  // single round (a sweep of two 96 x 84 grids: 1.02 us; 1.05 with 64 registers).
+  p.fwd_blocks = split_shots(p, sms, 2, p.fwd) == 1 ? 1 : 2;
+  return (p.fwd_blocks == 1 || split_shots(p, 2 * sms, 2, p.fwd)) && split_shots(p, sms, 3, p.bwd);
 }
 
 cudaError_t launch_march(cudaStream_t s, const MarchPack& p, bool backward, int flags, unsigned* done, unsigned* err) {
+  const MarchSplit& split = backward ? p.bwd : p.fwd;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.first[p.nshots]);
-  cfg.blockDim = dim3(p.threads);
-  cfg.dynamicSmemBytes = p.smem;
+  cfg.gridDim = dim3(split.first[p.nshots]);
+  cfg.blockDim = dim3(split.threads);
+  cfg.dynamicSmemBytes = split.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return backward ? cudaLaunchKernelEx(&cfg, k_march_bwd, p, done, err)
-                  : cudaLaunchKernelEx(&cfg, k_march_fwd, p, flags, done, err);
+  if (backward) return cudaLaunchKernelEx(&cfg, k_march_bwd, p, done, err);
+  return p.fwd_blocks == 1 ? cudaLaunchKernelEx(&cfg, k_march_fwd<1>, p, flags, done, err)
+                           : cudaLaunchKernelEx(&cfg, k_march_fwd<2>, p, flags, done, err);
 }
 
 }  // namespace fwigb
