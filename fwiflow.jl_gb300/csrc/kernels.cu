@@ -172,9 +172,9 @@ __device__ __forceinline__ bool tile_meets_shot_box(const ShotD& sh, int z0, int
 // scheduled as soon as all of its own blocks have started, and waits
 // (pdl_wait) for the previous sweep to complete, and its writes to be
 // visible, before it touches any field. The parameter reads, the tile
-// classification, the staging-barrier set-up and, in fast tiles and backward
-// edge tiles, the loads of the media (which no sweep writes) come before the
-// wait and overlap the previous sweep's last blocks.
+// classification, the staging-barrier set-up and the loads of the media (which
+// no sweep writes) come before the wait and overlap the previous sweep's last
+// blocks.
 #define SWEEP_KERNEL_TILE(TZ_)                                                 \
   const int shot = K == 1 ? 0 : static_cast<int>(blockIdx.z);                  \
   const Geo& g0 = P.slots[shot].g;                                             \
@@ -234,6 +234,23 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
   (void)rows_in;                                                               \
   SWEEP_SMEM()
 
+// Forward edge bodies: which of the thread's cells are in the stencil domain
+// (dom) and in the CPML along z (zc), and their address as in fast tiles (live
+// threads: even depths, so a pair lies in the padded column).
+#define SWEEP_EDGE_FWD(R_)                                                     \
+  const size_t base =                                                          \
+      static_cast<size_t>((static_cast<long long>(x0) * g.ldz + z0) * static_cast<long long>(sizeof(float))); \
+  const unsigned off =                                                         \
+      (threadIdx.y * static_cast<unsigned>(g.ldz) + (R_) * threadIdx.x) * static_cast<unsigned>(sizeof(float)); \
+  bool dom[R_], zc[R_], any_dom = false, any_z = false;                        \
+  _Pragma("unroll") for (int r = 0; r < (R_); ++r) {                           \
+    dom[r] = in_box(z + r, x, g.zs0, g.zs1, g.xs0, g.xs1);                     \
+    zc[r] = dom[r] && (z + r < g.nPml || z + r > g.zpml_hi);                   \
+    any_dom |= dom[r];                                                         \
+    any_z |= zc[r];                                                            \
+  }                                                                            \
+  (void)i;
+
 // Values of the thread's R depths that lie in the grid (rows_in of them);
 // the others are left 0.
 template <int R>
@@ -264,6 +281,16 @@ __device__ __forceinline__ void sto(float* p, size_t base, unsigned off, const f
   else
     *reinterpret_cast<float*>(q) = v[0];
 }
+
+// Asynchronous copy of a thread's own values into its place in shared memory,
+// and the wait for the thread's own copies (each thread reads only what it
+// copied, so there is no barrier).
+template <int R>
+__device__ __forceinline__ void ldasync(float* dst, const float* p, size_t base, unsigned off) {
+  const char* q = reinterpret_cast<const char*>(p) + base + off;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(q), "n"(4 * R) : "memory");
+}
+__device__ __forceinline__ void ldasync_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The media arrays are read by every sweep and, in a batched launch, by every
 // shot of the pack (their sub-grids are windows of the same model): their
@@ -356,81 +383,127 @@ __device__ __forceinline__ void own(const float* a, int b, float (&o)[R]) {
 #define FWD_BOUNDS __launch_bounds__(32 * TX, 2048 / (32 * TX))
 #define BWD_BOUNDS __launch_bounds__(32 * TX, (NT / (32 * TX)) > 0 ? (NT / (32 * TX)) : 1)
 
+// One CPML convolution (el_stress.cu:64-85): the memory value and the derivative.
+__device__ __forceinline__ void cpml_fwd(float bq, float aq, float K, float& mm, float& d) {
+  mm = bq * mm + aq * d;
+  d = d / K + mm;
+}
+
 // ---------------------------------------------------------------------------
 // F1: el_stress (el_stress.cu:50-88) + add_source (utilities.cu:521-541) +
 // recording (utilities.cu:557-567) + from_bnd of the 5 fields (Boundary.cu:55-76).
-// Staged: vz, vx. Edge body: the per-cell code for each of the thread's R
-// depths (after the staged tiles have landed).
+// Staged: vz, vx.
+//
+// Forward edge bodies. A load behind a store cannot be moved ahead of it (the
+// arrays might alias), so a body of one cell after the other makes up to ten
+// dependent trips to memory. Here a thread asks for the own values and the CPML
+// memory values of its R depths, as pairs, before it waits for the staged
+// tiles; a cell with CPML along both directions reads the x values when it is
+// done with those along z. F2 keeps the memory values in flight by cp.async
+// into shared memory, which holds no register. F1, which takes more registers
+// a cell, loads them into registers, the shear stress first: the shared memory
+// would come out of its L1 (on 1120 x 3152 grids 101 us; 97 this way).
+// us a sweep, one cell after the other / this: 16 shots of 352 x 832 F1 40.8 /
+// 38.2, F2 32.0 / 29.0; 608-row windows of 24 shots F1 116.3 / 111.0, F2 102.9
+// / 94.8; one 608 x 1600 shot F1 8.7 / 8.4, F2 7.6 / 7.1; four 1120 x 3152
+// shots F1 96.9 / 97.1, F2 80.7 / 78.1. (F2 with registers: 30.0, 97.6, 7.4,
+// 78.4.)
 template <int TX, int K, int R>
 __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
+  SWEEP_EDGE_FWD(R)
+  const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_s);
+  float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R], m1[R], m2[R];
+  if (live) {
+    ldo<R>(m.lam, base, off, lam);
+    ldo<R>(m.l2m, base, off, l2m);
+    ldo<R>(m.aveMu, base, off, amu);
+  }
   pdl_wait();
   SWEEP_TMA(2, BOXZ)
   if (!live) return;
-  const bool rec_tile = tile_meets_shot_box(sh, z0, x0, 32 * R, TX);
-  const StoreD& st = S.st;
+  ldo<R>(f.szz, base, off, szz);
+  ldo<R>(f.sxx, base, off, sxx);
+  ldo<R>(f.sxz, base, off, sxz);
+  if (any_z) {
+    ldo<R>(f.m_dvz_dz, base, off, m1);
+    ldo<R>(f.m_dvx_dz, base, off, m2);
+  } else if (xc) {
+    ldo<R>(f.m_dvx_dx, base, off, m1);
+    ldo<R>(f.m_dvz_dx, base, off, m2);
+  }
+  const bool special = tile_meets_shot_box(sh, z0, x0, 32 * R, TX);
   if (!stage_wait(&bar, err, inject)) return;
   const float* s_vz = sm;
   const float* s_vx = sm + N;
-  auto cell = [&](const int z, const size_t i, const int b) {
-    float szz = f.szz[i], sxx = f.sxx[i];
-    const float sxz = f.sxz[i];
-    const float lam = m.lam[i], l2m = m.l2m[i], amu = m.aveMu[i];
-    if (save) {
-      const int k = ring_index(g, z, x);
-      if (k >= 0) {
-        float* p = st.base + static_cast<size_t>(it) * 5 * g.ring_len + k;
-        p[0] = szz;
-        p[g.ring_len] = sxz;
-        p[2 * g.ring_len] = sxx;
-        p[3 * g.ring_len] = s_vz[b];
-        p[4 * g.ring_len] = s_vx[b];
+  if (save) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) ring_save(g, S.st, it, z + r, x, szz[r], sxz[r], sxx[r], s_vz[b + r], s_vx[b + r]);
+  }
+  if (any_dom) {
+    {
+      float dz[R], dx[R];
+      dpz<R>(s_vx, b, g.rdz, dz);
+      dpx<R, BOXZ>(s_vz, b, g.rdx, dx);
+      if (any_z) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (zc[r]) cpml_fwd(__ldg(c.b_zh + z + r), __ldg(c.a_zh + z + r), __ldg(c.K_zh + z + r), m2[r], dz[r]);
+        sto<R>(f.m_dvx_dz, base, off, m2);
+        if (xc) ldo<R>(f.m_dvz_dx, base, off, m2);
       }
-    }
-    const bool dom = in_box(z, x, g.zs0, g.zs1, g.xs0, g.xs1);
-    const bool src = (z == sh.src_z && x == sh.src_x);
-    if (dom) {
-      float dvz_dz = sdm(s_vz, b, 1, g.rdz);
-      float dvx_dx = sdm(s_vx, b, BOXZ, g.rdx);
-      float dvx_dz = sdp(s_vx, b, 1, g.rdz);
-      float dvz_dx = sdp(s_vz, b, BOXZ, g.rdx);
-      if ((z < g.nPml) || (z > g.zpml_hi)) {
-        float mm = c.b_z[z] * f.m_dvz_dz[i] + c.a_z[z] * dvz_dz;
-        f.m_dvz_dz[i] = mm;
-        dvz_dz = dvz_dz / c.K_z[z] + mm;
-        mm = c.b_zh[z] * f.m_dvx_dz[i] + c.a_zh[z] * dvx_dz;
-        f.m_dvx_dz[i] = mm;
-        dvx_dz = dvx_dz / c.K_zh[z] + mm;
+      if (xc) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (dom[r]) cpml_fwd(__ldg(c.b_xh + x), __ldg(c.a_xh + x), __ldg(c.K_xh + x), m2[r], dx[r]);
+        sto<R>(f.m_dvz_dx, base, off, m2);
       }
-      if ((x < g.nPml) || (x > g.xpml_hi_s)) {
-        float mm = c.b_x[x] * f.m_dvx_dx[i] + c.a_x[x] * dvx_dx;
-        f.m_dvx_dx[i] = mm;
-        dvx_dx = dvx_dx / c.K_x[x] + mm;
-        mm = c.b_xh[x] * f.m_dvz_dx[i] + c.a_xh[x] * dvz_dx;
-        f.m_dvz_dx[i] = mm;
-        dvz_dx = dvz_dx / c.K_xh[x] + mm;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (dom[r]) sxz[r] = sxz[r] + amu[r] * (dz[r] + dx[r]) * g.dt;
+      sto<R>(f.sxz, base, off, sxz);
+    }
+    float dz[R], dx[R];
+    dmz<R>(s_vz, b, g.rdz, dz);
+    dmx<R, BOXZ>(s_vx, b, g.rdx, dx);
+    if (any_z) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (zc[r]) cpml_fwd(__ldg(c.b_z + z + r), __ldg(c.a_z + z + r), __ldg(c.K_z + z + r), m1[r], dz[r]);
+      sto<R>(f.m_dvz_dz, base, off, m1);
+      if (xc) ldo<R>(f.m_dvx_dx, base, off, m1);
+    }
+    if (xc) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (dom[r]) cpml_fwd(__ldg(c.b_x + x), __ldg(c.a_x + x), __ldg(c.K_x + x), m1[r], dx[r]);
+      sto<R>(f.m_dvx_dx, base, off, m1);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        szz[r] += (l2m[r] * dz[r] + lam[r] * dx[r]) * g.dt;
+        sxx[r] += (lam[r] * dz[r] + l2m[r] * dx[r]) * g.dt;
       }
-      szz += (l2m * dvz_dz + lam * dvx_dx) * g.dt;
-      sxx += (lam * dvz_dz + l2m * dvx_dx) * g.dt;
-      f.sxz[i] = sxz + amu * (dvx_dz + dvz_dx) * g.dt;
-    }
-    if (src) {
-      szz += sh.src_szz[it];
-      sxx += sh.src_sxx[it];
-    }
-    if (dom || src) {
-      f.szz[i] = szz;
-      f.sxx[i] = sxx;
-    }
+  }
+  if (special) {
     // The velocity sweep that follows does not change the stresses, so the
     // sample of step it+1 is taken here.
-    if (rec_tile) record(sh, it, first_receiver(sh, z, x), z, x, szz, sxx);
-  };
 #pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (z + r < g.nz) cell(z + r, i + r, b + r);
+    for (int r = 0; r < R; ++r) {
+      if (z + r == sh.src_z && x == sh.src_x) {
+        szz[r] += sh.src_szz[it];
+        sxx[r] += sh.src_sxx[it];
+      }
+      record(sh, it, first_receiver(sh, z + r, x), z + r, x, szz[r], sxx[r]);
+    }
+  }
+  if (any_dom || special) {
+    sto<R>(f.szz, base, off, szz);
+    sto<R>(f.sxx, base, off, sxx);
+  }
 }
 
 // F2: el_velocity, isFor = true (el_velocity.cu:45-82). Staged: szz, sxx, sxz.
@@ -438,46 +511,83 @@ template <int TX, int K, int R>
 __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
+  SWEEP_EDGE_FWD(R)
+  constexpr int M = 32 * TX * R;  // floats between the thread's places in the shared arrays behind the staged ones
+  float* mem = sm + 3 * N + R * (threadIdx.y * 32 + threadIdx.x);
   (void)sh;
+  const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_v);
+  float bA[R], bB[R], vz[R], vx[R];
+  if (any_dom) {
+    ldo<R>(m.bycA, base, off, bA);
+    ldo<R>(m.bycB, base, off, bB);
+  }
   pdl_wait();
   SWEEP_TMA(3, BOXZ)
   if (!live) return;
-  if (!stage_wait(&bar, err)) return;
+  if (any_z) {
+    ldasync<R>(mem, f.m_dszz_dz, base, off);
+    ldasync<R>(mem + M, f.m_dsxz_dz, base, off);
+  }
+  if (xc) {
+    ldasync<R>(mem + 2 * M, f.m_dsxz_dx, base, off);
+    ldasync<R>(mem + 3 * M, f.m_dsxx_dx, base, off);
+  }
+  if (any_dom) {
+    ldo<R>(f.vz, base, off, vz);
+    ldo<R>(f.vx, base, off, vx);
+  }
+  ldasync_wait();
+  if (!stage_wait(&bar, err) || !any_dom) return;
   const float* s_szz = sm;
   const float* s_sxx = sm + N;
   const float* s_sxz = sm + 2 * N;
-  auto cell = [&](const int z, const size_t i, const int b) {
-    if (!in_box(z, x, g.zs0, g.zs1, g.xs0, g.xs1)) return;
-    const float vz = f.vz[i], vx = f.vx[i], bA = m.bycA[i], bB = m.bycB[i];
-    float dszz_dz = sdp(s_szz, b, 1, g.rdz);
-    float dsxz_dx = sdm(s_sxz, b, BOXZ, g.rdx);
-    float dsxz_dz = sdm(s_sxz, b, 1, g.rdz);
-    float dsxx_dx = sdp(s_sxx, b, BOXZ, g.rdx);
-    if ((z < g.nPml) || (z > g.zpml_hi)) {
-      float mm = c.b_zh[z] * f.m_dszz_dz[i] + c.a_zh[z] * dszz_dz;
-      f.m_dszz_dz[i] = mm;
-      dszz_dz = dszz_dz / c.K_zh[z] + mm;
-      mm = c.b_z[z] * f.m_dsxz_dz[i] + c.a_z[z] * dsxz_dz;
-      f.m_dsxz_dz[i] = mm;
-      dsxz_dz = dsxz_dz / c.K_z[z] + mm;
-    }
-    if ((x < g.nPml) || (x > g.xpml_hi_v)) {
-      float mm = c.b_x[x] * f.m_dsxz_dx[i] + c.a_x[x] * dsxz_dx;
-      f.m_dsxz_dx[i] = mm;
-      dsxz_dx = dsxz_dx / c.K_x[x] + mm;
-      mm = c.b_xh[x] * f.m_dsxx_dx[i] + c.a_xh[x] * dsxx_dx;
-      f.m_dsxx_dx[i] = mm;
-      dsxx_dx = dsxx_dx / c.K_xh[x] + mm;
-    }
-    const float nvz = vz + (dszz_dz + dsxz_dx) * bA * g.dt;
-    const float nvx = vx + (dsxz_dz + dsxx_dx) * bB * g.dt;
-    f.vz[i] = nvz;
-    f.vx[i] = nvx;
-    if (S.gr.illum) S.gr.illum[i] += nvz * nvz + nvx * nvx;
-  };
+  float dszz_dz[R], dsxz_dx[R], dsxz_dz[R], dsxx_dx[R];
+  dpz<R>(s_szz, b, g.rdz, dszz_dz);
+  dmx<R, BOXZ>(s_sxz, b, g.rdx, dsxz_dx);
+  dmz<R>(s_sxz, b, g.rdz, dsxz_dz);
+  dpx<R, BOXZ>(s_sxx, b, g.rdx, dsxx_dx);
+  if (any_z) {
+    float m1[R], m2[R];
+    own<R>(mem, 0, m1);
+    own<R>(mem + M, 0, m2);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (zc[r]) {
+        cpml_fwd(__ldg(c.b_zh + z + r), __ldg(c.a_zh + z + r), __ldg(c.K_zh + z + r), m1[r], dszz_dz[r]);
+        cpml_fwd(__ldg(c.b_z + z + r), __ldg(c.a_z + z + r), __ldg(c.K_z + z + r), m2[r], dsxz_dz[r]);
+      }
+    sto<R>(f.m_dszz_dz, base, off, m1);
+    sto<R>(f.m_dsxz_dz, base, off, m2);
+  }
+  if (xc) {
+    float m1[R], m2[R];
+    own<R>(mem + 2 * M, 0, m1);
+    own<R>(mem + 3 * M, 0, m2);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        cpml_fwd(__ldg(c.b_x + x), __ldg(c.a_x + x), __ldg(c.K_x + x), m1[r], dsxz_dx[r]);
+        cpml_fwd(__ldg(c.b_xh + x), __ldg(c.a_xh + x), __ldg(c.K_xh + x), m2[r], dsxx_dx[r]);
+      }
+    sto<R>(f.m_dsxz_dx, base, off, m1);
+    sto<R>(f.m_dsxx_dx, base, off, m2);
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r)
-    if (z + r < g.nz) cell(z + r, i + r, b + r);
+    if (dom[r]) {
+      vz[r] = vz[r] + (dszz_dz[r] + dsxz_dx[r]) * bA[r] * g.dt;
+      vx[r] = vx[r] + (dsxz_dz[r] + dsxx_dx[r]) * bB[r] * g.dt;
+    }
+  sto<R>(f.vz, base, off, vz);
+  sto<R>(f.vx, base, off, vx);
+  if (S.gr.illum) {
+    float e[R];
+    ldo<R>(S.gr.illum, base, off, e);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) e[r] += vz[r] * vz[r] + vx[r] * vx[r];
+    sto<R>(S.gr.illum, base, off, e);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1531,6 +1641,11 @@ template <int TX, int BOXZ>
 constexpr size_t smem_bytes(int na) {
   return static_cast<size_t>(na) * BOXZ * (TX + 4) * sizeof(float);
 }
+// Sweep F2: na staged arrays and the edge body's four arrays of memory values.
+template <int TX, int R>
+constexpr size_t smem_f2(int na) {
+  return smem_bytes<TX, 32 * R + 8>(na) + 4 * 32 * TX * R * sizeof(float);
+}
 }  // namespace
 
 #define FWIGB_DISPATCH_TX(tx, ...) \
@@ -1592,10 +1707,10 @@ int launch_fwd_velocity(cudaStream_t s, int tx, int rows, const SweepPack<K>& p,
                         unsigned* err) {
   if (rows == 2)
     FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 2>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
-                                     smem_bytes<TX, kBoxZFwd>(3), s, p, err))
+                                     smem_f2<TX, 2>(3), s, p, err))
   else
     FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 1>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
-                                     smem_bytes<TX, kBoxZ>(3), s, p, err))
+                                     smem_f2<TX, 1>(3), s, p, err))
   return 1;
 }
 
