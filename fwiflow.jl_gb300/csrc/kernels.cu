@@ -94,13 +94,13 @@ __device__ __forceinline__ void tma_load_2d(float* dst, const CUtensorMap* tm, i
 // see it) and issues the copies after the block has met the barrier's
 // initialisation; the caller then loads its own-cell operands (which overlap
 // with the copies) and calls stage_wait.
-template <int NA, int TX, int BOXZ>
+template <int NA, int TX, int BOXZ, int FIRST = 0>
 __device__ __forceinline__ void stage_issue(const TileMaps& mp, float* sm, uint64_t* bar, int z0, int x0) {
   constexpr int N = BOXZ * (TX + 4);
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     mbar_expect_tx(bar, NA * N * static_cast<unsigned>(sizeof(float)));
 #pragma unroll
-    for (int a = 0; a < NA; ++a) tma_load_2d(sm + a * N, &mp.t[a], z0 - 4, x0 - 2, bar);
+    for (int a = 0; a < NA; ++a) tma_load_2d(sm + a * N, &mp.t[FIRST + a], z0 - 4, x0 - 2, bar);
   }
 }
 __device__ __forceinline__ void stage_init(uint64_t* bar) {
@@ -147,17 +147,25 @@ __device__ __forceinline__ bool tile_meets_shot_box(const ShotD& sh, int z0, int
   return !(z0 + tz - 1 < sh.rbz0 || z0 > sh.rbz1 || x0 + tx - 1 < sh.rbx0 || x0 > sh.rbx1);
 }
 
+// An edge tile without a cell of the reverse-time interior, the source or a receiver.
+__device__ __forceinline__ bool outer_tile(const ShotSlot& S, int z0, int x0, int tz, int tx) {
+  const Geo& g = S.g;
+  const bool inner = z0 + tz > g.zi0 && z0 <= g.zi1 && x0 + tx > g.xi0 && x0 <= g.xi1;
+  return !inner && !tile_meets_shot_box(S.sh, z0, x0, tz, tx);
+}
+
 // Every sweep is one launch per time step for a pack of shots: blockIdx.z is
 // the shot (its slot holds its sub-grid, fields, source, receivers and TMA
 // maps), blockIdx.x / blockIdx.y the tile of TZ depths x TX columns. A tile
 // inside the shot's fast rectangle runs the sweep's fast body (the interior
 // form of the reference kernels); a tile inside the mid rectangle (no CPML
 // cell) runs the fast body with per-cell ring, band and guard handling; any
-// other tile runs its edge body (the full CPML / boundary-ring / band
-// logic). The choice is uniform per block. Blocks past a narrower shot's grid
-// leave before staging anything, and so do blocks whose tile lies wholly
-// below row zact1 (the nPad rows, where no sweep reads or writes a cell of
-// its own) unless it holds the shot's source or a receiver.
+// other tile runs its edge body (the full CPML / boundary-ring / band logic),
+// in the backward sweeps the shorter body of an outer tile where it can. The
+// choice is uniform per block. Blocks past a narrower shot's grid leave before
+// staging anything, and so do blocks whose tile lies wholly below row zact1
+// (the nPad rows, where no sweep reads or writes a cell of its own) unless it
+// holds the shot's source or a receiver.
 //
 // Work split. Block (32, TX): lane threadIdx.x covers R adjacent depths
 // (R = TZ / 32), threadIdx.y the column. The sweeps issue more integer than
@@ -234,10 +242,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
   (void)rows_in;                                                               \
   SWEEP_SMEM()
 
-// Forward edge bodies: which of the thread's cells are in the stencil domain
+// Which of an edge thread's cells are in the stencil domain
 // (dom) and in the CPML along z (zc), and their address as in fast tiles (live
 // threads: even depths, so a pair lies in the padded column).
-#define SWEEP_EDGE_FWD(R_)                                                     \
+#define SWEEP_EDGE_CELLS(R_)                                                     \
   const size_t base =                                                          \
       static_cast<size_t>((static_cast<long long>(x0) * g.ldz + z0) * static_cast<long long>(sizeof(float))); \
   const unsigned off =                                                         \
@@ -383,6 +391,27 @@ __device__ __forceinline__ void own(const float* a, int b, float (&o)[R]) {
 #define FWD_BOUNDS __launch_bounds__(32 * TX, 2048 / (32 * TX))
 #define BWD_BOUNDS __launch_bounds__(32 * TX, (NT / (32 * TX)) > 0 ? (NT / (32 * TX)) : 1)
 
+// psi differences of two memory arrays at the thread's cells in the stencil domain: Dm of the first and Dp of the
+// second along z; Dp of the first and Dm of the second along x.
+template <int R>
+__device__ __forceinline__ void psi_z(const float* a, const float* d, const bool (&dom)[R], size_t i, float r,
+                                      float (&pa)[R], float (&pd)[R]) {
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    pa[k] = dom[k] ? gdm(a, i + k, 1, r) : 0.0f;
+    pd[k] = dom[k] ? gdp(d, i + k, 1, r) : 0.0f;
+  }
+}
+template <int R>
+__device__ __forceinline__ void psi_x(const float* a, const float* d, const bool (&dom)[R], size_t i, size_t ldz,
+                                      float r, float (&pa)[R], float (&pd)[R]) {
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    pa[k] = dom[k] ? gdp(a, i + k, ldz, r) : 0.0f;
+    pd[k] = dom[k] ? gdm(d, i + k, ldz, r) : 0.0f;
+  }
+}
+
 // One CPML convolution (el_stress.cu:64-85): the memory value and the derivative.
 __device__ __forceinline__ void cpml_fwd(float bq, float aq, float K, float& mm, float& d) {
   mm = bq * mm + aq * d;
@@ -413,7 +442,7 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
                                                 bool inject, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_FWD(R)
+  SWEEP_EDGE_CELLS(R)
   const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_s);
   float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R], m1[R], m2[R];
   if (live) {
@@ -511,7 +540,7 @@ template <int TX, int K, int R>
 __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_FWD(R)
+  SWEEP_EDGE_CELLS(R)
   constexpr int M = 32 * TX * R;  // floats between the thread's places in the shared arrays behind the staged ones
   float* mem = sm + 3 * N + R * (threadIdx.y * 32 + threadIdx.x);
   (void)sh;
@@ -713,6 +742,129 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
     if (z + r < g.nz) cell(r, z + r, i + r, b + r);
 }
 
+// B of an outer tile: an edge tile without a cell of the reverse-time interior,
+// the source or a receiver, so that of the forward fields only the ring's
+// stresses are restored and only the adjoint stresses are staged. With an absorbing
+// layer as thick as a tile these are all tiles of the CPML but the few around
+// the source and receivers. They are bound by their memory trips as the forward
+// edge tiles are: all values but the x ones of the corners are asked for before
+// the staged tiles are waited for, which this body's fewer operands leave
+// registers for. us a sweep, edge body / this: 16 shots of 352 x 832 B 68.8 /
+// 66.1, C 71.5 / 67.9; 608-row windows of 24 shots B 224.1 / 220.2, C 226.1 /
+// 219.7; one 608 x 1600 shot B 13.5 / 13.1, C 13.8 / 12.6; four 1120 x 3152
+// shots B 202.4 / 203.8, C 185.9 / 183.9.
+template <int TX, int K, int R>
+__device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
+  constexpr int BOXZ = 32 * R + 8;
+  SWEEP_EDGE(BOXZ, R)
+  SWEEP_EDGE_CELLS(R)
+  (void)sh;
+  const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_s);
+  // Where there is something to read along x and z: in the CPML, and where a psi coefficient may not be zero.
+  const bool xq = xc || (any_dom && (x <= g.xband_lo || x >= g.xband_hi));
+  const bool zq = any_z || (any_dom && (z <= g.zband_lo || z + R - 1 >= g.zband_hi));
+  float lam[R], l2m[R], amu[R], bA[R], bB[R], va_x[R], va_z[R], p1[R], p2[R], m1[R], m2[R];
+  if (any_dom) {
+    ldo<R>(m.lam, base, off, lam);
+    ldo<R>(m.l2m, base, off, l2m);
+    ldo<R>(m.aveMu, base, off, amu);
+    ldo<R>(m.bycA, base, off, bA);
+    ldo<R>(m.bycB, base, off, bB);
+  }
+  pdl_wait();
+  stage_issue<3, TX, BOXZ, 2>(P.maps[shot], sm, &bar, z0, x0);
+  if (!live) return;
+  // The psi terms' differences and the memory values, along z, or along x where there are none along z.
+  if (zq) {
+    psi_z<R>(f.m_dvx_dz, f.m_dvz_dz, dom, i, g.rdz, p1, p2);
+    ldo<R>(f.m_dsxz_dz, base, off, m1);
+    ldo<R>(f.m_dszz_dz, base, off, m2);
+  } else if (xq) {
+    psi_x<R>(f.m_dvx_dx, f.m_dvz_dx, dom, i, ldz, g.rdx, p1, p2);
+    ldo<R>(f.m_dsxx_dx, base, off, m1);
+    ldo<R>(f.m_dsxz_dx, base, off, m2);
+  }
+  if (any_dom) {
+    ldo<R>(f.vx_a, base, off, va_x);
+    ldo<R>(f.vz_a, base, off, va_z);
+  }
+  const float* ring = S.st.base + static_cast<size_t>(S.nSteps - 2 - j) * 5 * g.ring_len;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int k = ring_index(g, z + r, x);
+    if (k >= 0) {
+      const float s1 = ring[k], s2 = ring[k + g.ring_len], s3 = ring[k + 2 * g.ring_len];
+      f.szz[i + r] = s1;
+      f.sxz[i + r] = s2;
+      f.sxx[i + r] = s3;
+    }
+  }
+  if (!stage_wait(&bar, err) || !any_dom) return;
+  const float* s_szz_a = sm;
+  const float* s_sxx_a = sm + N;
+  const float* s_sxz_a = sm + 2 * N;
+  const float dt = g.dt;
+  // el_velocity_adj (el_velocity_adj.cu:57-102); a psi term counts only where its CPML coefficient is not zero.
+  {
+    float d1[R], d2[R], d3[R], q1[R], n1[R];
+    dpx<R, BOXZ>(s_szz_a, b, g.rdx, d1);
+    dpx<R, BOXZ>(s_sxx_a, b, g.rdx, d2);
+    dmz<R>(s_sxz_a, b, g.rdz, d3);
+    if (xq && zq) {
+      ldo<R>(f.m_dsxx_dx, base, off, n1);
+#pragma unroll
+      for (int r = 0; r < R; ++r) q1[r] = dom[r] ? gdp(f.m_dvx_dx, i + r, ldz, g.rdx) : 0.0f;
+    }
+    const float Kx = __ldg(c.K_x + x), ax = __ldg(c.a_x + x);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        float t = 0.0f;
+        if (xq && ax != 0.0f) t += ax * (zq ? q1[r] : p1[r]);
+        const float azh = __ldg(c.a_zh + z + r);
+        if (zq && azh != 0.0f) t += azh * p1[r];
+        va_x[r] -= (kdiv(lam[r] * d1[r] + l2m[r] * d2[r], Kx) + kdiv(amu[r] * d3[r], __ldg(c.K_zh + z + r))) * dt + t;
+        const float add = bB[r] * va_x[r] * dt;
+        if (xc && !zq) m1[r] = __ldg(c.b_xh + x) * m1[r] + add;
+        if (xc && zq) n1[r] = __ldg(c.b_xh + x) * n1[r] + add;
+        if (zc[r]) m1[r] = __ldg(c.b_z + z + r) * m1[r] + add;
+      }
+    sto<R>(f.vx_a, base, off, va_x);
+    if (any_z) sto<R>(f.m_dsxz_dz, base, off, m1);
+    if (xc && !zq) sto<R>(f.m_dsxx_dx, base, off, m1);
+    if (xc && zq) sto<R>(f.m_dsxx_dx, base, off, n1);
+  }
+  {
+    float d1[R], d2[R], d3[R], q2[R], n2[R];
+    dpz<R>(s_szz_a, b, g.rdz, d1);
+    dpz<R>(s_sxx_a, b, g.rdz, d2);
+    dmx<R, BOXZ>(s_sxz_a, b, g.rdx, d3);
+    if (xq && zq) {
+      ldo<R>(f.m_dsxz_dx, base, off, n2);
+#pragma unroll
+      for (int r = 0; r < R; ++r) q2[r] = dom[r] ? gdm(f.m_dvz_dx, i + r, ldz, g.rdx) : 0.0f;
+    }
+    const float Kxh = __ldg(c.K_xh + x), axh = __ldg(c.a_xh + x);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        float t = 0.0f;
+        const float az = __ldg(c.a_z + z + r);
+        if (zq && az != 0.0f) t += az * p2[r];
+        if (xq && axh != 0.0f) t += axh * (zq ? q2[r] : p2[r]);
+        va_z[r] -= (kdiv(l2m[r] * d1[r] + lam[r] * d2[r], __ldg(c.K_z + z + r)) + kdiv(amu[r] * d3[r], Kxh)) * dt + t;
+        const float add = bA[r] * va_z[r] * dt;
+        if (xc && !zq) m2[r] = __ldg(c.b_x + x) * m2[r] + add;
+        if (xc && zq) n2[r] = __ldg(c.b_x + x) * n2[r] + add;
+        if (zc[r]) m2[r] = __ldg(c.b_zh + z + r) * m2[r] + add;
+      }
+    sto<R>(f.vz_a, base, off, va_z);
+    if (any_z) sto<R>(f.m_dszz_dz, base, off, m2);
+    if (xc && !zq) sto<R>(f.m_dsxz_dx, base, off, m2);
+    if (xc && zq) sto<R>(f.m_dsxz_dx, base, off, n2);
+  }
+}
+
 // C: res_injection (utilities.cu:569-580) + el_stress_adj (el_stress_adj.cu:53-97)
 //    + source_grad (utilities.cu:582-593) + el_velocity(isFor=false) with the
 //    sums of the density kernel (el_velocity.cu:84-117) + to_bnd(velocity).
@@ -815,6 +967,121 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (z + r < g.nz) cell(r, z + r, i + r, b + r);
+}
+
+// C of an outer tile (bwd_B_outer): of the forward fields only the ring's
+// velocities of step it - 1 are restored; only the adjoint velocities are staged.
+template <int TX, int K, int R>
+__device__ __forceinline__ void bwd_C_outer(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
+  constexpr int BOXZ = 32 * R + 8;
+  SWEEP_EDGE(BOXZ, R)
+  SWEEP_EDGE_CELLS(R)
+  (void)sh;
+  (void)zc;
+  (void)any_z;
+  const bool xq = any_dom && (x <= g.xband_lo || x >= g.xband_hi);
+  const bool zq = any_dom && (z <= g.zband_lo || z + R - 1 >= g.zband_hi);
+  float bA[R], bB[R], lam[R], l2m[R], amu[R], sa[R], xa[R], za[R], p1[R], p2[R], m1[R], m2[R];
+  if (any_dom) {
+    ldo<R>(m.bycA, base, off, bA);
+    ldo<R>(m.bycB, base, off, bB);
+    ldo<R>(m.aveMu, base, off, amu);
+    ldo<R>(m.lam, base, off, lam);
+    ldo<R>(m.l2m, base, off, l2m);
+  }
+  pdl_wait();
+  stage_issue<2, TX, BOXZ>(P.maps[shot], sm, &bar, z0, x0);
+  if (!live) return;
+  if (zq) {
+    psi_z<R>(f.m_dszz_dz, f.m_dsxz_dz, dom, i, g.rdz, p1, p2);
+    ldo<R>(f.m_dvz_dz, base, off, m1);
+    ldo<R>(f.m_dvx_dz, base, off, m2);
+  } else if (xq) {
+    psi_x<R>(f.m_dsxz_dx, f.m_dsxx_dx, dom, i, ldz, g.rdx, p2, p1);
+    ldo<R>(f.m_dvx_dx, base, off, m1);
+    ldo<R>(f.m_dvz_dx, base, off, m2);
+  }
+  if (any_dom) {
+    ldo<R>(f.szz_a, base, off, sa);
+    ldo<R>(f.sxx_a, base, off, xa);
+    ldo<R>(f.sxz_a, base, off, za);
+  }
+  const int it = S.nSteps - 2 - j;
+  if (it >= 1) {
+    const float* ring = S.st.base + static_cast<size_t>(it - 1) * 5 * g.ring_len + 3 * g.ring_len;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int k = ring_index(g, z + r, x);
+      if (k >= 0) {
+        const float v1 = ring[k], v2 = ring[k + g.ring_len];
+        f.vz[i + r] = v1;
+        f.vx[i + r] = v2;
+      }
+    }
+  }
+  if (!stage_wait(&bar, err) || !any_dom) return;
+  const float* s_vz_a = sm;
+  const float* s_vx_a = sm + N;
+  const float dt = g.dt;
+  {  // shear stress: psi terms p2 (along z, else x), memory values m2
+    float d1[R], d2[R], q[R], n[R];
+    dpx<R, BOXZ>(s_vz_a, b, g.rdx, d1);
+    dpz<R>(s_vx_a, b, g.rdz, d2);
+    if (xq && zq) {
+      ldo<R>(f.m_dvz_dx, base, off, n);
+#pragma unroll
+      for (int r = 0; r < R; ++r) q[r] = dom[r] ? gdp(f.m_dsxz_dx, i + r, ldz, g.rdx) : 0.0f;
+    }
+    const float Kx = __ldg(c.K_x + x), ax = __ldg(c.a_x + x);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        float t = 0.0f;
+        if (xq && ax != 0.0f) t += ax * (zq ? q[r] : p2[r]);
+        const float az = __ldg(c.a_z + z + r);
+        if (zq && az != 0.0f) t += az * p2[r];
+        za[r] -= (kdiv(d1[r], Kx) * bA[r] + kdiv(d2[r], __ldg(c.K_z + z + r)) * bB[r]) * dt + t;
+        const float add = za[r] * amu[r] * dt;
+        if (xq && !zq) m2[r] = __ldg(c.b_xh + x) * m2[r] + add;
+        if (xq && zq) n[r] = __ldg(c.b_xh + x) * n[r] + add;
+        if (zq && (z + r <= g.zband_lo || z + r >= g.zband_hi)) m2[r] = __ldg(c.b_zh + z + r) * m2[r] + add;
+      }
+    sto<R>(f.sxz_a, base, off, za);
+    if (zq) sto<R>(f.m_dvx_dz, base, off, m2);
+    if (xq && !zq) sto<R>(f.m_dvz_dx, base, off, m2);
+    if (xq && zq) sto<R>(f.m_dvz_dx, base, off, n);
+  }
+  {  // normal stresses
+    float d3[R], d4[R], q[R], n[R];
+    dmx<R, BOXZ>(s_vx_a, b, g.rdx, d3);
+    dmz<R>(s_vz_a, b, g.rdz, d4);
+    if (xq && zq) {
+      ldo<R>(f.m_dvx_dx, base, off, n);
+#pragma unroll
+      for (int r = 0; r < R; ++r) q[r] = dom[r] ? gdm(f.m_dsxx_dx, i + r, ldz, g.rdx) : 0.0f;
+    }
+    const float Kxh = __ldg(c.K_xh + x), axh = __ldg(c.a_xh + x);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (dom[r]) {
+        float tx = kdiv(bB[r] * d3[r], Kxh) * dt, tz = kdiv(bA[r] * d4[r], __ldg(c.K_zh + z + r)) * dt;
+        if (xq && axh != 0.0f) tx += axh * (zq ? q[r] : p1[r]);
+        const float azh = __ldg(c.a_zh + z + r);
+        if (zq && azh != 0.0f) tz += azh * p1[r];
+        xa[r] -= tx;
+        sa[r] -= tz;
+        const float ex = (lam[r] * sa[r] + l2m[r] * xa[r]) * dt;
+        if (xq && !zq) m1[r] = __ldg(c.b_x + x) * m1[r] + ex;
+        if (xq && zq) n[r] = __ldg(c.b_x + x) * n[r] + ex;
+        if (zq && (z + r <= g.zband_lo || z + r >= g.zband_hi))
+          m1[r] = __ldg(c.b_z + z + r) * m1[r] + (l2m[r] * sa[r] + lam[r] * xa[r]) * dt;
+      }
+    sto<R>(f.szz_a, base, off, sa);
+    sto<R>(f.sxx_a, base, off, xa);
+    if (zq) sto<R>(f.m_dvz_dz, base, off, m1);
+    if (xq && !zq) sto<R>(f.m_dvx_dx, base, off, m1);
+    if (xq && zq) sto<R>(f.m_dvx_dx, base, off, n);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1157,6 +1424,8 @@ __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j
     bwd_B_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   else if (mid)
     bwd_B_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
+  else if (outer_tile(P.slots[shot], z0, x0, 32 * R, TX))
+    bwd_B_outer<TX, K, R>(P, shot, z0, x0, j, err);
   else
     bwd_B_edge<TX, K, R>(P, shot, z0, x0, j, err);
 }
@@ -1168,6 +1437,8 @@ __global__ void BWD_BOUNDS k_bwd_C(const __grid_constant__ SweepPack<K> P, int j
     bwd_C_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   else if (mid)
     bwd_C_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
+  else if (outer_tile(P.slots[shot], z0, x0, 32 * R, TX))
+    bwd_C_outer<TX, K, R>(P, shot, z0, x0, j, err);
   else
     bwd_C_edge<TX, K, R>(P, shot, z0, x0, j, err);
 }
