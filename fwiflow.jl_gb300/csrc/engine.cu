@@ -1100,8 +1100,12 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
   const SweepGrid* grids = ctx->pack_grid.data();
   if (ctx->group_size == 1) return go(ctx->pack1[base], 1, grids[0]);
   int n = 0;
-  for (int q = 0; q * kPackShots < a; ++q)
+  const int np = (a + kPackShots - 1) / kPackShots;
+  const bool back = (w == 1 && (grids[0].order & kBackF2)) || (w == 3 && (grids[0].order & kBackC));
+  for (int k = 0; k < np; ++k) {
+    const int q = back ? np - 1 - k : k;
     n += go(ctx->packs[base * ctx->npacks + q], std::min(kPackShots, a - q * kPackShots), grids[q]);
+  }
   return n;
 }
 
@@ -1125,6 +1129,32 @@ bool marches(const fwigb_ctx* ctx) {
     cells += n;
   }
   return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
+}
+
+// Order of the sweeps' blocks (TileSplit::order).
+// kBackF2, kBackC: where the fields that a sweep shares with the one before it
+// (5 of F1 and F2, 13 of B and C) are larger than nearly half the L2, going back
+// over them finds their last part there; smaller ones are there anyway. ms a
+// pass over time, ahead / back (at 5 fields 57 MB are 2.9M cells, at 13 1.1M):
+//   F1 + F2  0.97M cells 8.0 / 8.0, 1.4M 4.18 / 4.43, 2.3M 7.92 / 7.85, 3.1M
+//            4.80 / 4.62, 3.5M (one shot) 5.36 / 5.13, 4.7M 14.68 / 14.25
+//   B + C    0.97M 13.6 / 13.8, 1.4M 10.1 / 9.3, 2.3M 15.6 / 14.6, 3.1M 10.5 /
+//            10.1, 3.5M 11.1 / 10.6, 4.7M 28.8 / 28.0
+// kByTile: the shots of a launch share the media (8 arrays of the model); where
+// these take more than a sixth of the L2, the shots of one tile follow each
+// other, so that they are read from memory once. ms a gradient, shot by shot /
+// tile by tile: model of 0.29M cells 42.1 / 43.9 (16 shots), 0.51M 36.3 / 36.6
+// (16) and 14.7 / 14.6 (6), 0.97M 107.8 / 104.7 (24), 1.4M 18.4 / 18.1 (3), 3.5M
+// 33.9 / 32.4 (4) and 17.6 / 17.1 (2).
+int block_order(const fwigb_ctx* ctx, const std::vector<ShotSlot>& slots) {
+  constexpr size_t l2 = 126u << 20;
+  size_t cells = 0;
+  for (const ShotSlot& s : slots) cells += static_cast<size_t>(s.g.nz) * s.g.nx;
+  int order = 0;
+  if (cells * 5 * sizeof(float) > l2 / 20 * 9) order |= kBackF2;
+  if (cells * 13 * sizeof(float) > l2 / 20 * 9) order |= kBackC;
+  if (slots.size() > 1 && ctx->cells * 8 * sizeof(float) > l2 / 6) order |= kByTile;
+  return order;
 }
 
 // Builds and uploads the slots and tensor maps of a group's members.
@@ -1208,7 +1238,7 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   for (int k = 0; k < G; ++k) ctx->pack_nx[k / kPackShots] = std::max(ctx->pack_nx[k / kPackShots], slots[k].g.nx);
   // Launch extents: the widest member sub-grid, and rows down to the last
   // one a sweep touches (zact1, or the lowest source / receiver row).
-  ctx->pack_grid.assign(ctx->npacks, SweepGrid{0, 0, 0});
+  ctx->pack_grid.assign(ctx->npacks, SweepGrid{});
   for (int q = 0; q < ctx->npacks; ++q) ctx->pack_grid[q].nx = ctx->pack_nx[q];
   for (int k = 0; k < G; ++k) {
     const int rows = std::min(slots[k].g.nz, std::max(slots[k].g.zact1, slots[k].sh.rbz1) + 1);
@@ -1217,10 +1247,16 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   // (Every sub-grid has the same rows, hence the same offset.) Variants w = 3 *
   // (sweep, + 4 with two depths per thread) + tile width.
   const int zoff = wide_tile_offset(slots[0].g);
-  for (SweepGrid& gr : ctx->pack_grid) gr.zoff = zoff;
+  const int order = block_order(ctx, slots);
+  for (SweepGrid& gr : ctx->pack_grid) {
+    gr.zoff = zoff;
+    gr.order = order;
+  }
   auto split = [&](int w, int k) {
     const bool wide = w / 3 >= 4;
-    return tile_split(slots[k].g, kTileXs[w % 3], wide ? kTileZFwd : kTileZ, wide ? zoff : 0);
+    TileSplit ts = tile_split(slots[k].g, kTileXs[w % 3], wide ? kTileZFwd : kTileZ, wide ? zoff : 0);
+    ts.order = order;
+    return ts;
   };
   if (G == 1) {
     ctx->pack1.assign(kSweepVariants * 3, SweepPack<1>{});

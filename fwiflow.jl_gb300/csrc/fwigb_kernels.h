@@ -71,6 +71,12 @@ struct Geo {
   float dt, rdz, rdx;
 };
 
+// Order of a launch's blocks (bits). kByTile: the shots of one tile follow each
+// other, else the tiles of one shot. kBackF2, kBackC: sweep F2, C goes through
+// columns (and shots) from the last to the first, so that it starts on what the
+// sweep before it left in L2.
+constexpr int kByTile = 1, kBackF2 = 2, kBackC = 4;
+
 // Split of a sub-grid's tiles (tz depths x tx columns, from row zoff on) into
 // the fast tiles, the rectangle [ftz0, ftz1) x [ftx0, ftx1) of tiles inside the
 // fast box, the mid tiles, those of the rectangle [mtz0, mtz1) x [mtx0, mtx1)
@@ -79,6 +85,7 @@ struct Geo {
 struct TileSplit {
   int ftz0, ftz1, ftx0, ftx1, mtz0, mtz1, mtx0, mtx1;
   int zoff;
+  int order;  // of the launch's blocks (kByTile, kBackF2, kBackC); the first shot's counts
 };
 
 inline TileSplit tile_split(const Geo& g, int tx, int tz, int zoff) {
@@ -215,6 +222,7 @@ bool encode_sweep_maps(const Geo& g, const Fields& f, int tx, SweepMaps& out, co
 struct SweepGrid {
   int nz, nx;
   int zoff;  // first row of the 64-row tiles (wide_tile_offset)
+  int order;  // TileSplit::order
 };
 
 // ---- launchers (kernels.cu). One launch covers the first `nshots` (<= K)

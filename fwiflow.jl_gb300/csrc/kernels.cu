@@ -154,18 +154,18 @@ __device__ __forceinline__ bool outer_tile(const ShotSlot& S, int z0, int x0, in
   return !inner && !tile_meets_shot_box(S.sh, z0, x0, tz, tx);
 }
 
-// Every sweep is one launch per time step for a pack of shots: blockIdx.z is
-// the shot (its slot holds its sub-grid, fields, source, receivers and TMA
-// maps), blockIdx.x / blockIdx.y the tile of TZ depths x TX columns. A tile
-// inside the shot's fast rectangle runs the sweep's fast body (the interior
-// form of the reference kernels); a tile inside the mid rectangle (no CPML
-// cell) runs the fast body with per-cell ring, band and guard handling; any
-// other tile runs its edge body (the full CPML / boundary-ring / band logic),
-// in the backward sweeps the shorter body of an outer tile where it can. The
-// choice is uniform per block. Blocks past a narrower shot's grid leave before
-// staging anything, and so do blocks whose tile lies wholly below row zact1
-// (the nPad rows, where no sweep reads or writes a cell of its own) unless it
-// holds the shot's source or a receiver.
+// Every sweep is one launch per time step for a pack of shots: a block takes a
+// tile of TZ depths x TX columns of one shot (whose slot holds its sub-grid,
+// fields, source, receivers and TMA maps), in the order that the host picks
+// (TileSplit::order). A tile inside the shot's fast rectangle runs the sweep's
+// fast body (the interior form of the reference kernels); a tile inside the mid
+// rectangle (no CPML cell) runs the fast body with per-cell ring, band and guard
+// handling; any other tile runs its edge body (the full CPML / boundary-ring /
+// band logic), in the backward sweeps the shorter body of an outer tile where it
+// can. The choice is uniform per block. Blocks past a narrower shot's grid leave
+// before staging anything, and so do blocks whose tile lies wholly below row
+// zact1 (the nPad rows, where no sweep reads or writes a cell of its own) unless
+// it holds the shot's source or a receiver.
 //
 // Work split. Block (32, TX): lane threadIdx.x covers R adjacent depths
 // (R = TZ / 32), threadIdx.y the column. The sweeps issue more integer than
@@ -183,11 +183,15 @@ __device__ __forceinline__ bool outer_tile(const ShotSlot& S, int z0, int x0, in
 // classification, the staging-barrier set-up and the loads of the media (which
 // no sweep writes) come before the wait and overlap the previous sweep's last
 // blocks.
-#define SWEEP_KERNEL_TILE(TZ_)                                                 \
-  const int shot = K == 1 ? 0 : static_cast<int>(blockIdx.z);                  \
+#define SWEEP_KERNEL_TILE(TZ_, BACK_)                                          \
+  const int order = P.tiles[0].order;                                          \
+  const bool by_tile = K > 1 && (order & kByTile);                             \
+  const bool back = order & (BACK_);                                           \
+  const int ntx = by_tile ? gridDim.z : gridDim.y, q = by_tile ? blockIdx.z : blockIdx.y; \
+  const int tz = by_tile ? blockIdx.y : blockIdx.x, tx = back ? ntx - 1 - q : q; \
+  const int shot = K == 1 ? 0 : by_tile ? blockIdx.x : back ? gridDim.z - 1 - blockIdx.z : blockIdx.z; \
   const Geo& g0 = P.slots[shot].g;                                             \
   const TileSplit& ts = P.tiles[shot];                                         \
-  const int tz = blockIdx.x, tx = blockIdx.y;                                  \
   const int z0 = tz * (TZ_) + ts.zoff, x0 = tx * TX;                           \
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");              \
   if (z0 >= g0.nz || x0 >= g0.nx) return;                                      \
@@ -1394,7 +1398,7 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
 // (stage_wait's `inject`).
 template <int TX, int K, int R>
 __global__ void FWD_BOUNDS k_fwd_stress(const __grid_constant__ SweepPack<K> P, int it, int flags, unsigned* err) {
-  SWEEP_KERNEL_TILE(32 * R)
+  SWEEP_KERNEL_TILE(32 * R, 0)
   const bool inject = (flags & 2) != 0;
   if (fast)
     fwd_stress_fast<TX, K, R, false>(P, shot, z0, x0, it, 0, inject, err);
@@ -1406,7 +1410,7 @@ __global__ void FWD_BOUNDS k_fwd_stress(const __grid_constant__ SweepPack<K> P, 
 
 template <int TX, int K, int R>
 __global__ void FWD_BOUNDS k_fwd_velocity(const __grid_constant__ SweepPack<K> P, unsigned* err) {
-  SWEEP_KERNEL_TILE(32 * R)
+  SWEEP_KERNEL_TILE(32 * R, kBackF2)
   // A mid tile of this sweep has nothing beyond the fast form: no CPML cell,
   // every cell in the stencil domain, and no ring or band work.
   if (fast || mid)
@@ -1419,7 +1423,7 @@ __global__ void FWD_BOUNDS k_fwd_velocity(const __grid_constant__ SweepPack<K> P
 // NT resident threads per SM (the register budget, BWD_BOUNDS).
 template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
-  SWEEP_KERNEL_TILE(32 * R)
+  SWEEP_KERNEL_TILE(32 * R, 0)
   if (fast)
     bwd_B_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   else if (mid)
@@ -1432,7 +1436,7 @@ __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j
 
 template <int TX, int K, int R, int NT>
 __global__ void BWD_BOUNDS k_bwd_C(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
-  SWEEP_KERNEL_TILE(32 * R)
+  SWEEP_KERNEL_TILE(32 * R, kBackC)
   if (fast)
     bwd_C_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
   else if (mid)
@@ -1957,7 +1961,8 @@ void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
 }
 
 dim3 sweep_grid(int tx, int tz, const SweepGrid& gr, int nshots) {
-  return dim3((gr.nz - (tz == kTileZFwd ? gr.zoff : 0) + tz - 1) / tz, (gr.nx + tx - 1) / tx, nshots);
+  const int ntz = (gr.nz - (tz == kTileZFwd ? gr.zoff : 0) + tz - 1) / tz, ntx = (gr.nx + tx - 1) / tx;
+  return gr.order & kByTile ? dim3(nshots, ntz, ntx) : dim3(ntz, ntx, nshots);
 }
 
 template <int K>
