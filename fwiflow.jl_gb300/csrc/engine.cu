@@ -643,17 +643,29 @@ Geo make_geo(const Params& p, int nx, const float* zprof, const float* xprof) {
   return g;
 }
 
+// Floats of an axis' CPML profiles of length n: K, a, b and their half-point
+// values, and packed behind them (16-byte aligned) {K, a, b, 1 / K} of both.
+size_t cpml_floats(int n) { return (static_cast<size_t>(6) * n + 3) / 4 * 4 + 8 * static_cast<size_t>(n); }
+
+void cpml_axis(int N, int n, int nPml, float dh, float f0, float dt, float* p) {
+  cpml_profile(N, n, nPml, dh, f0, dt, p, p + n, p + 2 * n, p + 3 * n, p + 4 * n, p + 5 * n);
+  float* q = p + (static_cast<size_t>(6) * n + 3) / 4 * 4;
+  for (int h = 0; h < 2; ++h)
+    for (int i = 0; i < n; ++i, q += 4) {
+      for (int k = 0; k < 3; ++k) q[k] = p[(3 * h + k) * n + i];
+      q[3] = 1.0f / q[0];
+    }
+}
+
 int setup_geometry(fwigb_ctx* ctx) {
   const Params& p = ctx->p;
   // CPML profiles: z (length nz, profile over nz - nPad, Cpml.cu:46-48) and x
   // of the full width; shots with an aperture window get their own x profiles.
-  std::vector<float> h(6 * p.nz + 6 * p.nx);
+  std::vector<float> h(cpml_floats(p.nz) + cpml_floats(p.nx));
   float* z = h.data();
-  float* x = h.data() + 6 * p.nz;
-  cpml_profile(p.nz - p.nPad, p.nz, p.nPml, p.dz, p.f0, p.dt, z, z + p.nz, z + 2 * p.nz, z + 3 * p.nz, z + 4 * p.nz,
-               z + 5 * p.nz);
-  cpml_profile(p.nx, p.nx, p.nPml, p.dx, p.f0, p.dt, x, x + p.nx, x + 2 * p.nx, x + 3 * p.nx, x + 4 * p.nx,
-               x + 5 * p.nx);
+  float* x = h.data() + cpml_floats(p.nz);
+  cpml_axis(p.nz - p.nPad, p.nz, p.nPml, p.dz, p.f0, p.dt, z);
+  cpml_axis(p.nx, p.nx, p.nPml, p.dx, p.f0, p.dt, x);
   ctx->geo = make_geo(p, p.nx, z, x);
   ctx->cells = static_cast<size_t>(ctx->geo.ldz) * p.nx;
   ctx->ncell = static_cast<size_t>(p.nz) * p.nx;
@@ -853,7 +865,7 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
       n_supd += SupdLayout(pl.nSteps).size;
     }
     pl.cpmlx_off = n_cpmlx;
-    n_cpmlx += 6 * static_cast<size_t>(pl.nx);
+    n_cpmlx += cpml_floats(pl.nx);
     ctx->plans.push_back(pl);
   }
   // Band-pass impulse responses, one per distinct record length.
@@ -876,9 +888,8 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
   std::vector<float> hsrc(n_src), htaper(n_taper, 1.0f), hcpml(n_cpmlx), hsupd(n_supd, 0.0f);
   std::vector<int> hrec(n_rec), hblk(n_blk, 0);
   const float* zprof = nullptr;
-  std::vector<float> zh(6 * p.nz);
-  cpml_profile(p.nz - p.nPad, p.nz, p.nPml, p.dz, p.f0, p.dt, zh.data(), zh.data() + p.nz, zh.data() + 2 * p.nz,
-               zh.data() + 3 * p.nz, zh.data() + 4 * p.nz, zh.data() + 5 * p.nz);
+  std::vector<float> zh(cpml_floats(p.nz));
+  cpml_axis(p.nz - p.nPad, p.nz, p.nPml, p.dz, p.f0, p.dt, zh.data());
   zprof = zh.data();
   const float scale = 2250000.0f;  // pow(1500.0, 2) (utilities.cu:528)
   ctx->nSteps_max = 0;
@@ -887,8 +898,7 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
     ctx->nSteps_max = std::max(ctx->nSteps_max, nt);
     // CPML x profiles of the sub-grid and its geometry.
     float* x = hcpml.data() + pl.cpmlx_off;
-    cpml_profile(pl.nx, pl.nx, p.nPml, p.dx, p.f0, p.dt, x, x + pl.nx, x + 2 * pl.nx, x + 3 * pl.nx, x + 4 * pl.nx,
-                 x + 5 * pl.nx);
+    cpml_axis(pl.nx, pl.nx, p.nPml, p.dx, p.f0, p.dt, x);
     pl.g = make_geo(p, pl.nx, zprof, x);
     // Source: taper 0.001 (Src_Rec.cu:140) and the add_source scale (utilities.cu:528-538).
     std::vector<float> w(nt);
@@ -1112,22 +1122,15 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // Whether the staged shots run as marching kernels (march.cu) rather than as
 // tile sweeps, one launch per sweep and step: small calls, of at most
 // kMarchCells cells in at most kPackShots shots (all shots of the call, so
-// that the grouping does not change the choice) of at most kMarchShotCells
-// each. Microseconds a step, marching against tiles:
-//   one shot    100k cells 11.9 / 22.1, 293k 21.2 / 25.0, 382k 26.3 / 28.8,
-//               511k 36.6 / 33.2, 970k 52.7 / 46.5
-//   2-12 shots  101k 13.3 / 24.5, 287k 22.4 / 29.2, 586k 34.0 / 38.1,
-//               608k (12 shots) 43.0 / 45.8, 684k 39.4 / 44.2
-//   16 shots    811k 54.4 / 54.4
+// that the grouping does not change the choice). Microseconds a step, marching
+// against tiles: 16k cells 9.2 / 16.1, 51k 11.7 / 12.4, 100k (one shot) 11.9 /
+// 13.7, 101k (two) 13.4 / 19.3, 118k 13.5 / 15.2, 200k 17.5 / 16.7, 287k (four)
+// 22.1 / 18.5, 293k (one) 21.4 / 17.8.
 // Fixed tile shapes and per-sweep timing ask for the sweeps themselves.
-constexpr size_t kMarchCells = 700000, kMarchShotCells = 400000;
+constexpr size_t kMarchCells = 150000;
 bool marches(const fwigb_ctx* ctx) {
   size_t cells = 0;
-  for (const ShotPlan& pl : ctx->plans) {
-    const size_t n = static_cast<size_t>(ctx->p.nz) * pl.nx;
-    if (n > kMarchShotCells) return false;
-    cells += n;
-  }
+  for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
   return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
 }
 
@@ -1167,6 +1170,9 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   nx_max = 0;
   const float* cz = ctx->cpml.as<float>();
   const int nz = ctx->p.nz;
+  auto packed = [](const float* p, int n) {
+    return reinterpret_cast<const float4*>(p + (static_cast<size_t>(6) * n + 3) / 4 * 4);
+  };
   for (size_t k = 0; k < members.size(); ++k) {
     const ShotPlan& pl = ctx->plans[members[k]];
     nx_max = std::max(nx_max, pl.nx);
@@ -1182,7 +1188,8 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
     sl.m = media_view(ctx, pl.x_off);
     const float* cx = ctx->shot_cpmlx.as<float>(pl.cpmlx_off);
     sl.c = CpmlD{cz,      cz + nz,      cz + 2 * nz,      cz + 3 * nz,      cz + 4 * nz,      cz + 5 * nz,
-                 cx,      cx + pl.nx,   cx + 2 * pl.nx,   cx + 3 * pl.nx,   cx + 4 * pl.nx,   cx + 5 * pl.nx};
+                 cx,      cx + pl.nx,   cx + 2 * pl.nx,   cx + 3 * pl.nx,   cx + 4 * pl.nx,   cx + 5 * pl.nx,
+                 packed(cz, nz), packed(cz, nz) + nz, packed(cx, pl.nx), packed(cx, pl.nx) + pl.nx};
     ShotD& sh = sl.sh;
     sh.src_z = pl.geom->z_src;
     sh.src_x = pl.geom->x_src - pl.x_off;

@@ -417,9 +417,9 @@ __device__ __forceinline__ void psi_x(const float* a, const float* d, const bool
 }
 
 // One CPML convolution (el_stress.cu:64-85): the memory value and the derivative.
-__device__ __forceinline__ void cpml_fwd(float bq, float aq, float K, float& mm, float& d) {
-  mm = bq * mm + aq * d;
-  d = d / K + mm;
+__device__ __forceinline__ void cpml_fwd(const float4& q, float& mm, float& d) {
+  mm = q.z * mm + q.y * d;
+  d = over(d, q.x, q.w) + mm;
 }
 
 // ---------------------------------------------------------------------------
@@ -483,14 +483,14 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
       if (any_z) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
-          if (zc[r]) cpml_fwd(__ldg(c.b_zh + z + r), __ldg(c.a_zh + z + r), __ldg(c.K_zh + z + r), m2[r], dz[r]);
+          if (zc[r]) cpml_fwd(__ldg(c.q_zh + z + r), m2[r], dz[r]);
         sto<R>(f.m_dvx_dz, base, off, m2);
         if (xc) ldo<R>(f.m_dvz_dx, base, off, m2);
       }
       if (xc) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
-          if (dom[r]) cpml_fwd(__ldg(c.b_xh + x), __ldg(c.a_xh + x), __ldg(c.K_xh + x), m2[r], dx[r]);
+          if (dom[r]) cpml_fwd(__ldg(c.q_xh + x), m2[r], dx[r]);
         sto<R>(f.m_dvz_dx, base, off, m2);
       }
 #pragma unroll
@@ -504,14 +504,14 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
     if (any_z) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (zc[r]) cpml_fwd(__ldg(c.b_z + z + r), __ldg(c.a_z + z + r), __ldg(c.K_z + z + r), m1[r], dz[r]);
+        if (zc[r]) cpml_fwd(__ldg(c.q_z + z + r), m1[r], dz[r]);
       sto<R>(f.m_dvz_dz, base, off, m1);
       if (xc) ldo<R>(f.m_dvx_dx, base, off, m1);
     }
     if (xc) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (dom[r]) cpml_fwd(__ldg(c.b_x + x), __ldg(c.a_x + x), __ldg(c.K_x + x), m1[r], dx[r]);
+        if (dom[r]) cpml_fwd(__ldg(c.q_x + x), m1[r], dx[r]);
       sto<R>(f.m_dvx_dx, base, off, m1);
     }
 #pragma unroll
@@ -586,8 +586,8 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (zc[r]) {
-        cpml_fwd(__ldg(c.b_zh + z + r), __ldg(c.a_zh + z + r), __ldg(c.K_zh + z + r), m1[r], dszz_dz[r]);
-        cpml_fwd(__ldg(c.b_z + z + r), __ldg(c.a_z + z + r), __ldg(c.K_z + z + r), m2[r], dsxz_dz[r]);
+        cpml_fwd(__ldg(c.q_zh + z + r), m1[r], dszz_dz[r]);
+        cpml_fwd(__ldg(c.q_z + z + r), m2[r], dsxz_dz[r]);
       }
     sto<R>(f.m_dszz_dz, base, off, m1);
     sto<R>(f.m_dsxz_dz, base, off, m2);
@@ -599,8 +599,8 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
-        cpml_fwd(__ldg(c.b_x + x), __ldg(c.a_x + x), __ldg(c.K_x + x), m1[r], dsxz_dx[r]);
-        cpml_fwd(__ldg(c.b_xh + x), __ldg(c.a_xh + x), __ldg(c.K_xh + x), m2[r], dsxx_dx[r]);
+        cpml_fwd(__ldg(c.q_x + x), m1[r], dsxz_dx[r]);
+        cpml_fwd(__ldg(c.q_xh + x), m2[r], dsxx_dx[r]);
       }
     sto<R>(f.m_dsxz_dx, base, off, m1);
     sto<R>(f.m_dsxx_dx, base, off, m2);
@@ -707,14 +707,14 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
   const bool zp = (z < g.nPml) || (z > g.zpml_hi);
   const bool xp = (x < g.nPml) || (x > g.xpml_hi_s);
   {
-    const float Kx = c.K_x[x], Kzh = c.K_zh[z];
+    const float4 cx = __ldg(c.q_x + x), czh = __ldg(c.q_zh + z);  // {K, a, b, 1 / K}
     const float dszz_dx = -sdp(s_szz_a, b, BOXZ, g.rdx);
     const float dsxx_dx = -sdp(s_sxx_a, b, BOXZ, g.rdx);
     const float dsxz_dz = -sdm(s_sxz_a, b, 1, g.rdz);
-    float t = kdiv(lam * dszz_dx, Kx) * dt + kdiv(l2m * dsxx_dx, Kx) * dt + kdiv(amu, Kzh) * dsxz_dz * dt;
-    const float ax = c.a_x[x], azh = c.a_zh[z];
-    if (ax != 0.0f) t += ax * (-gdp(f.m_dvx_dx, i, ldz, g.rdx));
-    if (azh != 0.0f) t += azh * (-gdm(f.m_dvx_dz, i, 1, g.rdz));
+    float t = over(lam * dszz_dx, cx.x, cx.w) * dt + over(l2m * dsxx_dx, cx.x, cx.w) * dt +
+              over(amu, czh.x, czh.w) * dsxz_dz * dt;
+    if (cx.y != 0.0f) t += cx.y * (-gdp(f.m_dvx_dx, i, ldz, g.rdx));
+    if (czh.y != 0.0f) t += czh.y * (-gdm(f.m_dvx_dz, i, 1, g.rdz));
     const float v = va_x + t;
     f.vx_a[i] = v;
     if (xp || zp) {
@@ -724,14 +724,14 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
     }
   }
   {
-    const float Kz = c.K_z[z], Kxh = c.K_xh[x];
+    const float4 cz = __ldg(c.q_z + z), cxh = __ldg(c.q_xh + x);
     const float dszz_dz = -sdp(s_szz_a, b, 1, g.rdz);
     const float dsxx_dz = -sdp(s_sxx_a, b, 1, g.rdz);
     const float dsxz_dx = -sdm(s_sxz_a, b, BOXZ, g.rdx);
-    float t = kdiv(l2m * dszz_dz, Kz) * dt + kdiv(lam * dsxx_dz, Kz) * dt + kdiv(amu, Kxh) * dsxz_dx * dt;
-    const float az = c.a_z[z], axh = c.a_xh[x];
-    if (az != 0.0f) t += az * (-gdp(f.m_dvz_dz, i, 1, g.rdz));
-    if (axh != 0.0f) t += axh * (-gdm(f.m_dvz_dx, i, ldz, g.rdx));
+    float t = over(l2m * dszz_dz, cz.x, cz.w) * dt + over(lam * dsxx_dz, cz.x, cz.w) * dt +
+              over(amu, cxh.x, cxh.w) * dsxz_dx * dt;
+    if (cz.y != 0.0f) t += cz.y * (-gdp(f.m_dvz_dz, i, 1, g.rdz));
+    if (cxh.y != 0.0f) t += cxh.y * (-gdm(f.m_dvz_dx, i, ldz, g.rdx));
     const float v = va_z + t;
     f.vz_a[i] = v;
     if (xp || zp) {
@@ -819,18 +819,19 @@ __device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int
 #pragma unroll
       for (int r = 0; r < R; ++r) q1[r] = dom[r] ? gdp(f.m_dvx_dx, i + r, ldz, g.rdx) : 0.0f;
     }
-    const float Kx = __ldg(c.K_x + x), ax = __ldg(c.a_x + x);
+    const float4 cx = __ldg(c.q_x + x);  // {K, a, b, 1 / K}
+    const float bxh = xc ? __ldg(c.b_xh + x) : 0.0f;
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
         float t = 0.0f;
-        if (xq && ax != 0.0f) t += ax * (zq ? q1[r] : p1[r]);
-        const float azh = __ldg(c.a_zh + z + r);
-        if (zq && azh != 0.0f) t += azh * p1[r];
-        va_x[r] -= (kdiv(lam[r] * d1[r] + l2m[r] * d2[r], Kx) + kdiv(amu[r] * d3[r], __ldg(c.K_zh + z + r))) * dt + t;
+        const float4 czh = __ldg(c.q_zh + z + r);
+        if (xq && cx.y != 0.0f) t += cx.y * (zq ? q1[r] : p1[r]);
+        if (zq && czh.y != 0.0f) t += czh.y * p1[r];
+        va_x[r] -= (over(lam[r] * d1[r] + l2m[r] * d2[r], cx.x, cx.w) + over(amu[r] * d3[r], czh.x, czh.w)) * dt + t;
         const float add = bB[r] * va_x[r] * dt;
-        if (xc && !zq) m1[r] = __ldg(c.b_xh + x) * m1[r] + add;
-        if (xc && zq) n1[r] = __ldg(c.b_xh + x) * n1[r] + add;
+        if (xc && !zq) m1[r] = bxh * m1[r] + add;
+        if (xc && zq) n1[r] = bxh * n1[r] + add;
         if (zc[r]) m1[r] = __ldg(c.b_z + z + r) * m1[r] + add;
       }
     sto<R>(f.vx_a, base, off, va_x);
@@ -848,18 +849,19 @@ __device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int
 #pragma unroll
       for (int r = 0; r < R; ++r) q2[r] = dom[r] ? gdm(f.m_dvz_dx, i + r, ldz, g.rdx) : 0.0f;
     }
-    const float Kxh = __ldg(c.K_xh + x), axh = __ldg(c.a_xh + x);
+    const float4 cxh = __ldg(c.q_xh + x);
+    const float bx = xc ? __ldg(c.b_x + x) : 0.0f;
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
         float t = 0.0f;
-        const float az = __ldg(c.a_z + z + r);
-        if (zq && az != 0.0f) t += az * p2[r];
-        if (xq && axh != 0.0f) t += axh * (zq ? q2[r] : p2[r]);
-        va_z[r] -= (kdiv(l2m[r] * d1[r] + lam[r] * d2[r], __ldg(c.K_z + z + r)) + kdiv(amu[r] * d3[r], Kxh)) * dt + t;
+        const float4 cz = __ldg(c.q_z + z + r);
+        if (zq && cz.y != 0.0f) t += cz.y * p2[r];
+        if (xq && cxh.y != 0.0f) t += cxh.y * (zq ? q2[r] : p2[r]);
+        va_z[r] -= (over(l2m[r] * d1[r] + lam[r] * d2[r], cz.x, cz.w) + over(amu[r] * d3[r], cxh.x, cxh.w)) * dt + t;
         const float add = bA[r] * va_z[r] * dt;
-        if (xc && !zq) m2[r] = __ldg(c.b_x + x) * m2[r] + add;
-        if (xc && zq) n2[r] = __ldg(c.b_x + x) * n2[r] + add;
+        if (xc && !zq) m2[r] = bx * m2[r] + add;
+        if (xc && zq) n2[r] = bx * n2[r] + add;
         if (zc[r]) m2[r] = __ldg(c.b_zh + z + r) * m2[r] + add;
       }
     sto<R>(f.vz_a, base, off, va_z);
@@ -917,10 +919,10 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
     {
       const float dvz_dx = -sdp(s_vz_a, b, BOXZ, g.rdx);
       const float dvx_dz = -sdp(s_vx_a, b, 1, g.rdz);
-      float t = kdiv(dvz_dx, c.K_x[x]) * bA * dt + kdiv(dvx_dz, c.K_z[z]) * bB * dt;
-      const float ax = c.a_x[x], az = c.a_z[z];
-      if (ax != 0.0f) t += ax * (-gdp(f.m_dsxz_dx, i, ldz, g.rdx));
-      if (az != 0.0f) t += az * (-gdp(f.m_dsxz_dz, i, 1, g.rdz));
+      const float4 cx = __ldg(c.q_x + x), cz = __ldg(c.q_z + z);
+      float t = over(dvz_dx, cx.x, cx.w) * bA * dt + over(dvx_dz, cz.x, cz.w) * bB * dt;
+      if (cx.y != 0.0f) t += cx.y * (-gdp(f.m_dsxz_dx, i, ldz, g.rdx));
+      if (cz.y != 0.0f) t += cz.y * (-gdp(f.m_dsxz_dz, i, 1, g.rdz));
       za += t;
       f.sxz_a[i] = za;
     }
@@ -931,11 +933,11 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
     {
       const float dvx_dx = -sdm(s_vx_a, b, BOXZ, g.rdx);
       const float dvz_dz = -sdm(s_vz_a, b, 1, g.rdz);
-      float tx = kdiv(bB * dvx_dx, c.K_xh[x]) * dt;
-      float tz = kdiv(bA * dvz_dz, c.K_zh[z]) * dt;
-      const float axh = c.a_xh[x], azh = c.a_zh[z];
-      if (axh != 0.0f) tx += axh * (-gdm(f.m_dsxx_dx, i, ldz, g.rdx));
-      if (azh != 0.0f) tz += azh * (-gdm(f.m_dszz_dz, i, 1, g.rdz));
+      const float4 cxh = __ldg(c.q_xh + x), czh = __ldg(c.q_zh + z);
+      float tx = over(bB * dvx_dx, cxh.x, cxh.w) * dt;
+      float tz = over(bA * dvz_dz, czh.x, czh.w) * dt;
+      if (cxh.y != 0.0f) tx += cxh.y * (-gdm(f.m_dsxx_dx, i, ldz, g.rdx));
+      if (czh.y != 0.0f) tz += czh.y * (-gdm(f.m_dszz_dz, i, 1, g.rdz));
       xa += tx;
       sa += tz;
     }
@@ -1036,18 +1038,19 @@ __device__ __forceinline__ void bwd_C_outer(const SweepPack<K>& P, int shot, int
 #pragma unroll
       for (int r = 0; r < R; ++r) q[r] = dom[r] ? gdp(f.m_dsxz_dx, i + r, ldz, g.rdx) : 0.0f;
     }
-    const float Kx = __ldg(c.K_x + x), ax = __ldg(c.a_x + x);
+    const float4 cx = __ldg(c.q_x + x);
+    const float bxh = __ldg(c.b_xh + x);
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
         float t = 0.0f;
-        if (xq && ax != 0.0f) t += ax * (zq ? q[r] : p2[r]);
-        const float az = __ldg(c.a_z + z + r);
-        if (zq && az != 0.0f) t += az * p2[r];
-        za[r] -= (kdiv(d1[r], Kx) * bA[r] + kdiv(d2[r], __ldg(c.K_z + z + r)) * bB[r]) * dt + t;
+        const float4 cz = __ldg(c.q_z + z + r);
+        if (xq && cx.y != 0.0f) t += cx.y * (zq ? q[r] : p2[r]);
+        if (zq && cz.y != 0.0f) t += cz.y * p2[r];
+        za[r] -= (over(d1[r], cx.x, cx.w) * bA[r] + over(d2[r], cz.x, cz.w) * bB[r]) * dt + t;
         const float add = za[r] * amu[r] * dt;
-        if (xq && !zq) m2[r] = __ldg(c.b_xh + x) * m2[r] + add;
-        if (xq && zq) n[r] = __ldg(c.b_xh + x) * n[r] + add;
+        if (xq && !zq) m2[r] = bxh * m2[r] + add;
+        if (xq && zq) n[r] = bxh * n[r] + add;
         if (zq && (z + r <= g.zband_lo || z + r >= g.zband_hi)) m2[r] = __ldg(c.b_zh + z + r) * m2[r] + add;
       }
     sto<R>(f.sxz_a, base, off, za);
@@ -1064,19 +1067,20 @@ __device__ __forceinline__ void bwd_C_outer(const SweepPack<K>& P, int shot, int
 #pragma unroll
       for (int r = 0; r < R; ++r) q[r] = dom[r] ? gdm(f.m_dsxx_dx, i + r, ldz, g.rdx) : 0.0f;
     }
-    const float Kxh = __ldg(c.K_xh + x), axh = __ldg(c.a_xh + x);
+    const float4 cxh = __ldg(c.q_xh + x);
+    const float bx = __ldg(c.b_x + x);
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
-        float tx = kdiv(bB[r] * d3[r], Kxh) * dt, tz = kdiv(bA[r] * d4[r], __ldg(c.K_zh + z + r)) * dt;
-        if (xq && axh != 0.0f) tx += axh * (zq ? q[r] : p1[r]);
-        const float azh = __ldg(c.a_zh + z + r);
-        if (zq && azh != 0.0f) tz += azh * p1[r];
+        const float4 czh = __ldg(c.q_zh + z + r);
+        float tx = over(bB[r] * d3[r], cxh.x, cxh.w) * dt, tz = over(bA[r] * d4[r], czh.x, czh.w) * dt;
+        if (xq && cxh.y != 0.0f) tx += cxh.y * (zq ? q[r] : p1[r]);
+        if (zq && czh.y != 0.0f) tz += czh.y * p1[r];
         xa[r] -= tx;
         sa[r] -= tz;
         const float ex = (lam[r] * sa[r] + l2m[r] * xa[r]) * dt;
-        if (xq && !zq) m1[r] = __ldg(c.b_x + x) * m1[r] + ex;
-        if (xq && zq) n[r] = __ldg(c.b_x + x) * n[r] + ex;
+        if (xq && !zq) m1[r] = bx * m1[r] + ex;
+        if (xq && zq) n[r] = bx * n[r] + ex;
         if (zq && (z + r <= g.zband_lo || z + r >= g.zband_hi))
           m1[r] = __ldg(c.b_z + z + r) * m1[r] + (l2m[r] * sa[r] + lam[r] * xa[r]) * dt;
       }

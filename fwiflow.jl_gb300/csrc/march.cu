@@ -222,13 +222,6 @@ __device__ __forceinline__ float pz(const March& M, const Cells& c, int r, int q
 __device__ __forceinline__ float px(const March& M, const Cells& c, int q) {
   return M.prof[kProfiles * M.nz + q * M.w + c.xl];
 }
-// a / K with r = 1 / K rounded: the quotient estimate a r corrected by its
-// residual, correctly rounded by Markstein's theorem (IBM J. Res. Dev. 34,
-// 1990) as the division is, without its range checks (K is in [1, 2]).
-__device__ __forceinline__ float over(float a, float K, float r) {
-  const float q = a * r;
-  return fmaf(fmaf(-K, q, a), r, q);
-}
 __device__ __forceinline__ float over_z(const March& M, const Cells& c, int r, float a, int h) {
   return over(a, pz(M, c, r, h ? KH : K_), pz(M, c, r, h ? RKH : RK));
 }

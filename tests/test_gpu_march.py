@@ -19,7 +19,7 @@ CASES = {
     # chunks and strips without any CPML cell
     "interior": dict(nz=110, nx=150, nPml=12, nSteps=150, n_shots=2),
     # several rounds of a block's warps, strips of different widths in the two passes
-    "rounds": dict(nz=277, nx=401, nPml=16, nSteps=70, n_shots=2),
+    "rounds": dict(nz=177, nx=233, nPml=16, nSteps=70, n_shots=2),
     # as many shots as a pack holds
     "sixteen": dict(nz=40, nx=48, nPml=10, nSteps=80, n_shots=16),
 }
