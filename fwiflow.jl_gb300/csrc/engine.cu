@@ -1096,6 +1096,10 @@ int plan_groups(fwigb_ctx* ctx, bool adj, std::vector<std::vector<int>>& groups)
 // Returns the number of launches.
 int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int flags, unsigned* d_err) {
   cudaStream_t s = ctx->stream;
+  if (ctx->pack_grid[0].wide) {
+    tx = kWideTx;
+    rows = 1;
+  }
   const int variant = rows == 2 ? w + 4 : w;
   const size_t base = static_cast<size_t>(variant * 3 + tx_slot(tx));
   auto go = [&](const auto& pk, int n, const SweepGrid& gr) {
@@ -1123,9 +1127,12 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // tile sweeps, one launch per sweep and step: small calls, of at most
 // kMarchCells cells in at most kPackShots shots (all shots of the call, so
 // that the grouping does not change the choice). Microseconds a step, marching
-// against tiles: 16k cells 9.2 / 16.1, 51k 11.7 / 12.4, 100k (one shot) 11.9 /
-// 13.7, 101k (two) 13.4 / 19.3, 118k 13.5 / 15.2, 200k 17.5 / 16.7, 287k (four)
-// 22.1 / 18.5, 293k (one) 21.4 / 17.8.
+// against tiles, with an absorbing layer of 32 cells: 51k cells 11.7 / 12.4,
+// 100k (one shot) 11.9 / 13.7, 101k (two) 13.4 / 18.0, 171k 19.1 / 18.8, 200k
+// 17.5 / 16.7, 287k (four) 22.1 / 18.5, 293k (one) 21.4 / 17.8; with one of
+// 12-20 cells: 16k 9.2 / 16.1, 129k (16 shots) 14.7 / 22.9, 137k 16.7 / 19.3,
+// 170k (one) 16.2 / 16.7, 206k 20.7 / 20.3, 274k 24.1 / 22.6, 343k (five) 27.0
+// / 28.1, 380k (three) 29.1 / 26.6.
 // Fixed tile shapes and per-sweep timing ask for the sweeps themselves.
 constexpr size_t kMarchCells = 150000;
 bool marches(const fwigb_ctx* ctx) {
@@ -1133,6 +1140,9 @@ bool marches(const fwigb_ctx* ctx) {
   for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
   return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
 }
+
+// Arrays of this many bytes need 64-bit offsets in the sweeps.
+constexpr size_t kWideBytes = size_t{1} << 32;
 
 // Order of the sweeps' blocks (TileSplit::order).
 // kBackF2, kBackC: where the fields that a sweep shares with the one before it
@@ -1258,6 +1268,8 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
   for (SweepGrid& gr : ctx->pack_grid) {
     gr.zoff = zoff;
     gr.order = order;
+    for (const ShotSlot& sl : slots)
+      gr.wide |= static_cast<size_t>(sl.g.ldz) * sl.g.nx * sizeof(float) >= kWideBytes;
   }
   auto split = [&](int w, int k) {
     const bool wide = w / 3 >= 4;

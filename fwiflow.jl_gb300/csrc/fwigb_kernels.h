@@ -32,6 +32,7 @@ constexpr int kBinX = 8;
 constexpr int kBoxZ = kTileZ + 8;
 constexpr int kBoxZFwd = kTileZFwd + 8;
 constexpr int kTileXs[3] = {4, 8, 16};
+constexpr int kWideTx = 8;
 
 // Tensor maps of the (up to 5) arrays a sweep stages into shared memory.
 struct TileMaps {  // 128-byte aligned (CUtensorMap)
@@ -224,6 +225,7 @@ struct SweepGrid {
   int nz, nx;
   int zoff;  // first row of the 64-row tiles (wide_tile_offset)
   int order;  // TileSplit::order
+  bool wide = false;  // a member's arrays are 4 GB or more: the tiles are one row of kWideTx columns a thread
 };
 
 // ---- launchers (kernels.cu). One launch covers the first `nshots` (<= K)

@@ -208,17 +208,30 @@ __device__ __forceinline__ bool outer_tile(const ShotSlot& S, int z0, int x0, in
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Fast and mid tiles lie wholly inside the grid: `base` is the byte offset of
-// the tile's first cell, `off` that of the thread's first cell from there and b
-// its index in a staged box. `special` marks the tiles that meet the bounding
+// A thread's own cells are at `base` + `off` bytes from an array's start: with
+// WIDE the tile's 64-bit offset (block-uniform) and the thread's from there, else
+// a 32-bit offset alone, for arrays of less than 4 GB. Without the additions to
+// every pointer F2 needs no spills: 16 shots of 352 x 832 27.0 -> 24.5 us, 608-row
+// windows of 24 shots 89.8 -> 84.8, four 1120 x 3152 shots 73.4 -> 68.2; F1 and C
+// 1 % less. B, whose offset then costs a spilled register, keeps the uniform base
+// (206.6 us on those windows; 213.0 without).
+#define SWEEP_ADDRESS(R_, WIDE_)                                               \
+  const size_t base =                                                          \
+      (WIDE_) ? static_cast<size_t>((static_cast<long long>(x0) * g.ldz + z0) * static_cast<long long>(sizeof(float))) \
+              : 0;                                                             \
+  const unsigned off =                                                         \
+      (((WIDE_) ? threadIdx.y : x0 + threadIdx.y) * static_cast<unsigned>(g.ldz) + ((WIDE_) ? 0 : z0) + \
+       (R_) * threadIdx.x) *                                                   \
+      static_cast<unsigned>(sizeof(float));
+
+// Fast and mid tiles lie wholly inside the grid; b is the index of the thread's
+// first cell in a staged box. `special` marks the tiles that meet the bounding
 // box of the shot's receivers and source.
-#define SWEEP_FAST(TZ_, BOXZ_, R_)                                             \
+#define SWEEP_FAST(TZ_, BOXZ_, R_, WIDE_)                                      \
   SWEEP_BODY_SLOT()                                                            \
   const bool special = tile_meets_shot_box(sh, z0, x0, (TZ_), TX);             \
   constexpr int N = (BOXZ_) * (TX + 4);                                        \
-  const size_t base = (static_cast<size_t>(x0) * g.ldz + z0) * sizeof(float);  \
-  const unsigned off =                                                         \
-      (threadIdx.y * static_cast<unsigned>(g.ldz) + (R_) * threadIdx.x) * static_cast<unsigned>(sizeof(float)); \
+  SWEEP_ADDRESS(R_, WIDE_)                                                     \
   const int b = (threadIdx.y + 2) * (BOXZ_) + (R_) * threadIdx.x + 4;          \
   const int z = z0 + (R_) * static_cast<int>(threadIdx.x), x = x0 + threadIdx.y; \
   SWEEP_SMEM()
@@ -249,11 +262,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Which of an edge thread's cells are in the stencil domain
 // (dom) and in the CPML along z (zc), and their address as in fast tiles (live
 // threads: even depths, so a pair lies in the padded column).
-#define SWEEP_EDGE_CELLS(R_)                                                     \
-  const size_t base =                                                          \
-      static_cast<size_t>((static_cast<long long>(x0) * g.ldz + z0) * static_cast<long long>(sizeof(float))); \
-  const unsigned off =                                                         \
-      (threadIdx.y * static_cast<unsigned>(g.ldz) + (R_) * threadIdx.x) * static_cast<unsigned>(sizeof(float)); \
+#define SWEEP_EDGE_CELLS(R_, WIDE_)                                            \
+  SWEEP_ADDRESS(R_, WIDE_)                                                     \
   bool dom[R_], zc[R_], any_dom = false, any_z = false;                        \
   _Pragma("unroll") for (int r = 0; r < (R_); ++r) {                           \
     dom[r] = in_box(z + r, x, g.zs0, g.zs1, g.xs0, g.xs1);                     \
@@ -441,12 +451,12 @@ __device__ __forceinline__ void cpml_fwd(const float4& q, float& mm, float& d) {
 // / 94.8; one 608 x 1600 shot F1 8.7 / 8.4, F2 7.6 / 7.1; four 1120 x 3152
 // shots F1 96.9 / 97.1, F2 80.7 / 78.1. (F2 with registers: 30.0, 97.6, 7.4,
 // 78.4.)
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_CELLS(R)
+  SWEEP_EDGE_CELLS(R, WIDE)
   const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_s);
   float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R], m1[R], m2[R];
   if (live) {
@@ -540,11 +550,11 @@ __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot,
 }
 
 // F2: el_velocity, isFor = true (el_velocity.cu:45-82). Staged: szz, sxx, sxz.
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_CELLS(R)
+  SWEEP_EDGE_CELLS(R, WIDE)
   constexpr int M = 32 * TX * R;  // floats between the thread's places in the shared arrays behind the staged ones
   float* mem = sm + 3 * N + R * (threadIdx.y * 32 + threadIdx.x);
   (void)sh;
@@ -761,7 +771,7 @@ template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_CELLS(R)
+  SWEEP_EDGE_CELLS(R, true)
   (void)sh;
   const bool xc = any_dom && (x < g.nPml || x > g.xpml_hi_s);
   // Where there is something to read along x and z: in the CPML, and where a psi coefficient may not be zero.
@@ -977,11 +987,11 @@ __device__ __forceinline__ void bwd_C_edge(const SweepPack<K>& P, int shot, int 
 
 // C of an outer tile (bwd_B_outer): of the forward fields only the ring's
 // velocities of step it - 1 are restored; only the adjoint velocities are staged.
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void bwd_C_outer(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
   SWEEP_EDGE(BOXZ, R)
-  SWEEP_EDGE_CELLS(R)
+  SWEEP_EDGE_CELLS(R, WIDE)
   (void)sh;
   (void)zc;
   (void)any_z;
@@ -1104,11 +1114,11 @@ __device__ __forceinline__ void bwd_C_outer(const SweepPack<K>& P, int shot, int
 // MID: the tile is a mid tile (no CPML cell; it may hold ring cells).
 // Own-cell operands and results move as float2 with two depths per thread.
 
-template <int TX, int K, int R, bool MID>
+template <int TX, int K, int R, bool MID, bool WIDE>
 __device__ __forceinline__ void fwd_stress_fast(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST(TZ, BOXZ, R)
+  SWEEP_FAST(TZ, BOXZ, R, WIDE)
   const uint64_t pol = media_policy();
   float lam[R], l2m[R], amu[R], szz[R], sxx[R], sxz[R];
   ldm<R>(m.lam, base, off, lam, pol);
@@ -1157,10 +1167,10 @@ __device__ __forceinline__ void fwd_stress_fast(const SweepPack<K>& P, int shot,
   sto<R>(f.sxx, base, off, sxx);
 }
 
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void fwd_velocity_fast(const SweepPack<K>& P, int shot, int z0, int x0, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST(TZ, BOXZ, R)
+  SWEEP_FAST(TZ, BOXZ, R, WIDE)
   (void)special;
   (void)z;
   (void)x;
@@ -1203,7 +1213,7 @@ __device__ __forceinline__ void fwd_velocity_fast(const SweepPack<K>& P, int sho
 template <int TX, int K, int R, bool MID>
 __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST(TZ, BOXZ, R)
+  SWEEP_FAST(TZ, BOXZ, R, true)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
   const uint64_t pol = media_policy();
@@ -1294,10 +1304,10 @@ __device__ __forceinline__ void bwd_B_fast(const SweepPack<K>& P, int shot, int 
 // within 2 cells of the CPML), the reverse velocity update and its imaging
 // sums only at cells of the reverse-time interior, and the ring's velocities
 // of step it-1 restored.
-template <int TX, int K, int R, bool MID>
+template <int TX, int K, int R, bool MID, bool WIDE>
 __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int TZ = 32 * R, BOXZ = TZ + 8;
-  SWEEP_FAST(TZ, BOXZ, R)
+  SWEEP_FAST(TZ, BOXZ, R, WIDE)
   const Grads& gr = S.gr;
   const int it = S.nSteps - 2 - j;
   const bool rev = it >= 1;
@@ -1400,27 +1410,27 @@ __device__ __forceinline__ void bwd_C_fast(const SweepPack<K>& P, int shot, int 
 // picked per workload by the autotuner.
 // flags: bit 0 saves the boundary ring, bit 1 is the timeout test hook
 // (stage_wait's `inject`).
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __global__ void FWD_BOUNDS k_fwd_stress(const __grid_constant__ SweepPack<K> P, int it, int flags, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R, 0)
   const bool inject = (flags & 2) != 0;
   if (fast)
-    fwd_stress_fast<TX, K, R, false>(P, shot, z0, x0, it, 0, inject, err);
+    fwd_stress_fast<TX, K, R, false, WIDE>(P, shot, z0, x0, it, 0, inject, err);
   else if (mid)
-    fwd_stress_fast<TX, K, R, true>(P, shot, z0, x0, it, flags & 1, inject, err);
+    fwd_stress_fast<TX, K, R, true, WIDE>(P, shot, z0, x0, it, flags & 1, inject, err);
   else
-    fwd_stress_edge<TX, K, R>(P, shot, z0, x0, it, flags & 1, inject, err);
+    fwd_stress_edge<TX, K, R, WIDE>(P, shot, z0, x0, it, flags & 1, inject, err);
 }
 
-template <int TX, int K, int R>
+template <int TX, int K, int R, bool WIDE>
 __global__ void FWD_BOUNDS k_fwd_velocity(const __grid_constant__ SweepPack<K> P, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R, kBackF2)
   // A mid tile of this sweep has nothing beyond the fast form: no CPML cell,
   // every cell in the stencil domain, and no ring or band work.
   if (fast || mid)
-    fwd_velocity_fast<TX, K, R>(P, shot, z0, x0, err);
+    fwd_velocity_fast<TX, K, R, WIDE>(P, shot, z0, x0, err);
   else
-    fwd_velocity_edge<TX, K, R>(P, shot, z0, x0, err);
+    fwd_velocity_edge<TX, K, R, WIDE>(P, shot, z0, x0, err);
 }
 
 // Backward sweeps: R depths per thread (tiles of 32 R rows), R in {1, 2};
@@ -1438,15 +1448,15 @@ __global__ void BWD_BOUNDS k_bwd_B(const __grid_constant__ SweepPack<K> P, int j
     bwd_B_edge<TX, K, R>(P, shot, z0, x0, j, err);
 }
 
-template <int TX, int K, int R, int NT>
+template <int TX, int K, int R, int NT, bool WIDE>
 __global__ void BWD_BOUNDS k_bwd_C(const __grid_constant__ SweepPack<K> P, int j, unsigned* err) {
   SWEEP_KERNEL_TILE(32 * R, kBackC)
   if (fast)
-    bwd_C_fast<TX, K, R, false>(P, shot, z0, x0, j, err);
+    bwd_C_fast<TX, K, R, false, WIDE>(P, shot, z0, x0, j, err);
   else if (mid)
-    bwd_C_fast<TX, K, R, true>(P, shot, z0, x0, j, err);
+    bwd_C_fast<TX, K, R, true, WIDE>(P, shot, z0, x0, j, err);
   else if (outer_tile(P.slots[shot], z0, x0, 32 * R, TX))
-    bwd_C_outer<TX, K, R>(P, shot, z0, x0, j, err);
+    bwd_C_outer<TX, K, R, WIDE>(P, shot, z0, x0, j, err);
   else
     bwd_C_edge<TX, K, R>(P, shot, z0, x0, j, err);
 }
@@ -1973,11 +1983,14 @@ template <int K>
 int launch_fwd_stress(cudaStream_t s, int tx, int rows, const SweepPack<K>& p, int nshots, const SweepGrid& gr, int it,
                       int flags, unsigned* err) {
   const int sv = flags & 3;
-  if (rows == 2)
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_stress<TX, K, 2>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
+  if (gr.wide)
+    launch_pdl(k_fwd_stress<kWideTx, K, 1, true>, sweep_grid(kWideTx, kTileZ, gr, nshots), dim3(32, kWideTx),
+               smem_bytes<kWideTx, kBoxZ>(2), s, p, it, sv, err);
+  else if (rows == 2)
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_stress<TX, K, 2, false>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
                                      smem_bytes<TX, kBoxZFwd>(2), s, p, it, sv, err))
   else
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_stress<TX, K, 1>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_stress<TX, K, 1, false>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
                                      smem_bytes<TX, kBoxZ>(2), s, p, it, sv, err))
   return 1;
 }
@@ -1985,11 +1998,14 @@ int launch_fwd_stress(cudaStream_t s, int tx, int rows, const SweepPack<K>& p, i
 template <int K>
 int launch_fwd_velocity(cudaStream_t s, int tx, int rows, const SweepPack<K>& p, int nshots, const SweepGrid& gr,
                         unsigned* err) {
-  if (rows == 2)
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 2>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
+  if (gr.wide)
+    launch_pdl(k_fwd_velocity<kWideTx, K, 1, true>, sweep_grid(kWideTx, kTileZ, gr, nshots), dim3(32, kWideTx),
+               smem_f2<kWideTx, 1>(3), s, p, err);
+  else if (rows == 2)
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 2, false>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
                                      smem_f2<TX, 2>(3), s, p, err))
   else
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 1>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_fwd_velocity<TX, K, 1, false>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
                                      smem_f2<TX, 1>(3), s, p, err))
   return 1;
 }
@@ -2012,14 +2028,17 @@ int launch_bwd_B(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>&
 template <int K>
 int launch_bwd_C(cudaStream_t s, int tx, int rows, int regs, const SweepPack<K>& p, int nshots,
                  const SweepGrid& gr, int j, unsigned* err) {
-  if (rows == 2)
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 2, 1024>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
+  if (gr.wide)
+    launch_pdl(k_bwd_C<kWideTx, K, 1, 2048, true>, sweep_grid(kWideTx, kTileZ, gr, nshots), dim3(32, kWideTx),
+               smem_bytes<kWideTx, kBoxZ>(5), s, p, j, err);
+  else if (rows == 2)
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 2, 1024, false>, sweep_grid(TX, kTileZFwd, gr, nshots), dim3(32, TX),
                                      smem_bytes<TX, kBoxZFwd>(5), s, p, j, err))
   else if (regs > 32)
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 1, 1536>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 1, 1536, false>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
                                      smem_bytes<TX, kBoxZ>(5), s, p, j, err))
   else
-    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 1, 2048>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
+    FWIGB_DISPATCH_TX(tx, launch_pdl(k_bwd_C<TX, K, 1, 2048, false>, sweep_grid(TX, kTileZ, gr, nshots), dim3(32, TX),
                                      smem_bytes<TX, kBoxZ>(5), s, p, j, err))
   return 1;
 }
