@@ -47,11 +47,11 @@ import __graft_entry__ as ge  # noqa: E402
 
 # Algorithmic bytes per grid cell and time step of each sweep (FP32 arrays read
 # or written once): forward stress 11 floats, forward velocity 9, backward B 24,
-# backward C 22; forward + adjoint = 264 B per cell-step.
+# backward C 21; forward + adjoint = 260 B per cell-step.
 SWEEP_NAMES = ["fwd_stress", "fwd_velocity", "bwd_B", "bwd_C"]
 SWEEP_KERNELS = ["k_fwd_stress", "k_fwd_velocity", "k_bwd_B", "k_bwd_C"]
-SWEEP_BYTES = [44, 36, 96, 88]
-FWD_ADJ_BYTES = 264
+SWEEP_BYTES = [44, 36, 96, 84]
+FWD_ADJ_BYTES = 260
 
 
 def peaks():

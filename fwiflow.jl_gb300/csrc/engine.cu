@@ -1149,16 +1149,16 @@ constexpr size_t kWideBytes = size_t{1} << 32;
 // (5 of F1 and F2, 13 of B and C) are larger than nearly half the L2, going back
 // over them finds their last part there; smaller ones are there anyway. ms a
 // pass over time, ahead / back (at 5 fields 57 MB are 2.9M cells, at 13 1.1M):
-//   F1 + F2  0.97M cells 8.0 / 8.0, 1.4M 4.18 / 4.43, 2.3M 7.92 / 7.85, 3.1M
-//            4.80 / 4.62, 3.5M (one shot) 5.36 / 5.13, 4.7M 14.68 / 14.25
-//   B + C    0.97M 13.6 / 13.8, 1.4M 10.1 / 9.3, 2.3M 15.6 / 14.6, 3.1M 10.5 /
-//            10.1, 3.5M 11.1 / 10.6, 4.7M 28.8 / 28.0
+//   F1 + F2  0.97M cells 6.6 / 6.6, 1.4M 3.43 / 3.42, 2.3M 5.89 / 5.82, 3.1M
+//            3.88 / 3.71, 3.5M (one shot) 4.93 / 4.50, 4.7M 12.40 / 11.69
+//   B + C    0.97M 12.0 / 12.2, 1.4M 9.5 / 8.8, 2.3M 14.6 / 13.5, 3.1M 9.8 /
+//            9.4, 3.5M 10.8 / 10.3, 4.7M 26.9 / 26.0
 // kByTile: the shots of a launch share the media (8 arrays of the model); where
 // these take more than a sixth of the L2, the shots of one tile follow each
 // other, so that they are read from memory once. ms a gradient, shot by shot /
-// tile by tile: model of 0.29M cells 42.1 / 43.9 (16 shots), 0.51M 36.3 / 36.6
-// (16) and 14.7 / 14.6 (6), 0.97M 107.8 / 104.7 (24), 1.4M 18.4 / 18.1 (3), 3.5M
-// 33.9 / 32.4 (4) and 17.6 / 17.1 (2).
+// tile by tile: model of 0.29M cells 37.7 / 39.3 (16 shots), 0.51M 33.5 / 34.2
+// (16) and 13.1 / 13.1 (6), 0.97M 102.0 / 99.0 (24), 1.4M 17.0 / 16.9 (3), 3.5M
+// 32.9 / 31.2 (4) and 16.9 / 16.4 (2).
 int block_order(const fwigb_ctx* ctx, const std::vector<ShotSlot>& slots) {
   constexpr size_t l2 = 126u << 20;
   size_t cells = 0;
@@ -1980,6 +1980,10 @@ int fwigb_sweep_time(fwigb_ctx* ctx, int kind, int reps, double* us_per_launch) 
   std::lock_guard<std::mutex> lk(ctx->mu);
   if (ctx->group_size < 1) {
     ctx->err = "no group has run yet";
+    return FWIGB_ERR_ARG;
+  }
+  if (kind >= 2 && ctx->store_stride == 0) {  // (no boundary ring to restore)
+    ctx->err = "the last run had no backward sweeps";
     return FWIGB_ERR_ARG;
   }
   cudaStream_t s = ctx->stream;

@@ -1,7 +1,7 @@
 // Marching kernels: a whole pass over time in one launch, for calls whose
 // grids are too small to fill the GPU in every sweep.
 //
-// A sweep of a small grid is all latency: 5-6 us a launch on a 96 x 84 grid as
+// A sweep of a small grid is all latency: 4 us a launch on a 96 x 84 grid as
 // on a 192 x 264 one (launch, cold parameter block, barrier set-up, staging
 // copy, one wave of tiles), four launches a step. Here each shot's columns are
 // cut into strips, one block each, and a block carries its strip through every
@@ -12,9 +12,8 @@
 // orders their writes before its reads, and their reads before its writes).
 // All blocks of a launch are resident together (a cooperative launch). The
 // hand-over costs 1.1 us of a sweep, the sweep itself 1-1.5 us at the smallest
-// sizes: a step of two 96 x 84 grids takes 9.4 us (20.4 with a launch per sweep),
-// of two 192 x 264 grids 13.3 us (24.5), of one 224 x 448 grid 11.9 us (22.1), of
-// two 352 x 832 grids 34.0 us (38.1).
+// sizes: a step of two 96 x 84 grids takes 9.2 us (16.1 with a launch per sweep),
+// of two 192 x 264 grids 13.4 us (18.0), of one 224 x 448 grid 11.9 us (13.7).
 //
 // A warp takes 64 depths of one column at a time, two adjacent ones a thread,
 // and reads its stencil samples from the fields themselves (L1 / L2): at these

@@ -56,3 +56,15 @@ def test_edge_tiles(name, gpu_lib, fw, orc, tmp_path):
             for a, k in zip(r[1:5], ("g_lambda", "g_mu", "g_den", "g_stf")):
                 assert rel(a, g[k]) < 1e-3, (width, rows, k, rel(a, g[k]))
             assert rel(ctx.illumination(), ill) < 1e-5
+
+
+def test_sweep_time_refuses_backward_sweeps_without_a_ring(gpu_lib, fw, tmp_path):
+    from fwiflow_gb300 import synthetic
+
+    w = synthetic.tiny(nSteps=20)
+    ctx = fw.FwiContext(w.write_files(str(tmp_path)), 0)
+    ctx.obs(*w.moduli(), w.stf, [0, 1], write_files=False)
+    assert ctx.sweep_time(0, 2) > 0
+    for kind in (2, 3):
+        with pytest.raises(Exception, match="backward"):
+            ctx.sweep_time(kind, 2)
