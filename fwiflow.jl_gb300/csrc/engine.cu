@@ -485,6 +485,7 @@ struct fwigb_ctx {
   bool model_set = false;
   DevBuf vp;                // the Vp of a fwigb_set_model_vp model and its mask (row-major doubles)
   bool vp_model = false, vp_masked = false;
+  bool vp_grad = false;     // the gradients are a run's under that model
   int last_calc = -1;
   long long launches = 0;
   int tx[4] = {8, 8, 8, 8};    // tile width per sweep (F1, F2, B, C)
@@ -741,7 +742,7 @@ int set_model(fwigb_ctx* ctx, const double* lam, const double* mu, const double*
   }
   CK(cudaSetDevice(ctx->device));
   clear_stale_error();
-  ctx->vp_model = false;
+  ctx->vp_model = ctx->vp_grad = false;
   const size_t nh = ctx->ncell, n = ctx->cells;
   double* st = ctx->stage.as<double>();
   CK(cudaMemcpyAsync(st, lam, nh * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -764,7 +765,7 @@ int set_model_vp(fwigb_ctx* ctx, const double* vp, const double* vp0, const doub
   }
   CK(cudaSetDevice(ctx->device));
   clear_stale_error();
-  ctx->vp_model = false;
+  ctx->vp_model = ctx->vp_grad = false;
   const size_t nh = ctx->ncell, n = ctx->cells;
   CK(ctx->vp.ensure(2 * nh * sizeof(double)));
   double* st = ctx->stage.as<double>();
@@ -1450,6 +1451,7 @@ int run(fwigb_ctx* ctx, int calc_id) {
   }
   CK(cudaSetDevice(ctx->device));
   clear_stale_error();
+  ctx->vp_grad = false;
   std::vector<std::vector<int>> groups;
   TRY_RC(plan_groups(ctx, adj, groups));
   cudaStream_t s = ctx->stream;
@@ -1712,6 +1714,7 @@ int run(fwigb_ctx* ctx, int calc_id) {
   CK(cudaGetLastError());
   ctx->launches = launches;
   ctx->last_calc = calc_id;
+  ctx->vp_grad = adj && ctx->vp_model;
   ctx->last_groups = static_cast<int>(groups.size());
   ctx->illum_valid = ctx->illum;
   if (adj && ctx->p.if_save_scratch) TRY_RC(write_scratch(ctx));
@@ -1734,22 +1737,26 @@ int kernel_times(fwigb_ctx* ctx, double* total_ms, long long* counts) {
   return FWIGB_OK;
 }
 
+// Whether every bounded wait of the runs since the last check ended. After one
+// that ran out the results are invalid, the Vp gradient's among them.
+int check_waits(fwigb_ctx* ctx) {
+  unsigned e = 0;
+  CK(cudaMemcpyAsync(&e, ctx->scal.as<char>() + 16, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  if (!e) return FWIGB_OK;
+  CK(cudaMemsetAsync(ctx->scal.as<char>() + 16, 0, sizeof(unsigned), ctx->stream));
+  ctx->vp_grad = false;
+  ctx->err = "a sweep gave up waiting for its staged tiles (bounded wait); results are invalid";
+  return FWIGB_ERR_TIMEOUT;
+}
+
 int fetch(fwigb_ctx* ctx, double* misfit, double* g_lam, double* g_mu, double* g_den, double* g_stf, float* gathers) {
   CK(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
   const Params& p = ctx->p;
   const size_t n = ctx->cells;
   const int nt_max = p.nSteps;
-  {
-    unsigned e = 0;
-    CK(cudaMemcpyAsync(&e, ctx->scal.as<char>() + 16, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (e) {
-      CK(cudaMemsetAsync(ctx->scal.as<char>() + 16, 0, sizeof(unsigned), s));
-      ctx->err = "a sweep gave up waiting for its staged tiles (bounded wait); results are invalid";
-      return FWIGB_ERR_TIMEOUT;
-    }
-  }
+  TRY_RC(check_waits(ctx));
   if (misfit) {
     double acc = 0.0;
     CK(cudaMemcpyAsync(&acc, ctx->scal.p, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1924,11 +1931,12 @@ int fwigb_set_model_vp(fwigb_ctx* ctx, const double* vp, const double* vp0, cons
 int fwigb_fetch_vp_gradient(fwigb_ctx* ctx, double* g_vp) {
   if (!ctx || !g_vp) return FWIGB_ERR_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  if (!ctx->vp_model || ctx->last_calc != 1) {
-    ctx->err = "the Vp gradient needs a Vp model (fwigb_set_model_vp) and a run with gradients";
+  CK(cudaSetDevice(ctx->device));
+  if (!ctx->vp_grad) {
+    ctx->err = "the Vp gradient needs a Vp model (fwigb_set_model_vp) and, after it, a run with gradients";
     return FWIGB_ERR_ARG;
   }
-  CK(cudaSetDevice(ctx->device));
+  TRY_RC(check_waits(ctx));
   const size_t n = ctx->cells;
   const float* g = ctx->grads.as<float>();
   double* st = ctx->stage.as<double>();

@@ -123,8 +123,9 @@ int fwigb_set_model(fwigb_ctx *ctx, const double *lambda, const double *mu, cons
 int fwigb_set_model_vp(fwigb_ctx *ctx, const double *vp, const double *vp0, const double *mask, double vmin,
                        double vmax);
 
-/* dJ/dVp [nz][nx] of the last run with gradients under that model, times the
- * model's mask (if any). */
+/* dJ/dVp [nz][nx] of the last run, which had gradients and was made under that
+ * model, times the model's mask (if any). FWIGB_ERR_ARG after a model or a run
+ * of another kind since, FWIGB_ERR_TIMEOUT as fwigb_fetch. */
 int fwigb_fetch_vp_gradient(fwigb_ctx *ctx, double *g_vp);
 
 /* Stages the shots of a call: source rows of stf, receivers, and (when
