@@ -24,6 +24,7 @@
 
 #include "fwiflow_gb300.h"
 #include "fwigb_kernels.h"
+#include "quotient.h"
 #include "json_lite.h"
 
 namespace fwigb {
@@ -645,7 +646,8 @@ Geo make_geo(const Params& p, int nx, const float* zprof, const float* xprof) {
 }
 
 // Floats of an axis' CPML profiles of length n: K, a, b and their half-point
-// values, and packed behind them (16-byte aligned) {K, a, b, 1 / K} of both.
+// values, and packed behind them (16-byte aligned) {K, a, b, 1 / K} of both, K
+// and 1 / K scaled as over() takes them.
 size_t cpml_floats(int n) { return (static_cast<size_t>(6) * n + 3) / 4 * 4 + 8 * static_cast<size_t>(n); }
 
 void cpml_axis(int N, int n, int nPml, float dh, float f0, float dt, float* p) {
@@ -654,7 +656,8 @@ void cpml_axis(int N, int n, int nPml, float dh, float f0, float dt, float* p) {
   for (int h = 0; h < 2; ++h)
     for (int i = 0; i < n; ++i, q += 4) {
       for (int k = 0; k < 3; ++k) q[k] = p[(3 * h + k) * n + i];
-      q[3] = 1.0f / q[0];
+      q[3] = 1.0f / q[0] / kQuotientScale;
+      q[0] *= kQuotientScale;
     }
 }
 

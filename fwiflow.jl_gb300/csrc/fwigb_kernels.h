@@ -133,7 +133,7 @@ struct MediaD {
 struct CpmlD {
   const float *K_z, *a_z, *b_z, *K_zh, *a_zh, *b_zh;  // length nz
   const float *K_x, *a_x, *b_x, *K_xh, *a_xh, *b_xh;  // length nx
-  const float4 *q_z, *q_zh, *q_x, *q_xh;              // the same as {K, a, b, 1 / K}
+  const float4 *q_z, *q_zh, *q_x, *q_xh;              // {K, a, b, 1 / K}, K and 1 / K scaled (over())
 };
 
 // Per-shot data for the sweeps.

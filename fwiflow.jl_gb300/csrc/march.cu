@@ -161,7 +161,7 @@ enum Field {
 };
 enum Medium { LAM = 0, L2M = 3, AMU = 4, BYA = 5, BYB = 6 };
 enum Sum { G_LAM, G_MU, G_TAU, G_VA, G_VB, G_ILLUM };
-enum Profile { K_, A_, B_, KH, AH, BH, RK, RKH };  // (the last two: 1 / K, 1 / K_half)
+enum Profile { K_, A_, B_, KH, AH, BH, RK, RKH };  // (the last two: 1 / K, 1 / K_half; K and 1 / K scaled, over())
 constexpr int kProfiles = 8;
 
 struct March {
@@ -222,10 +222,10 @@ __device__ __forceinline__ float px(const March& M, const Cells& c, int q) {
   return M.prof[kProfiles * M.nz + q * M.w + c.xl];
 }
 __device__ __forceinline__ float over_z(const March& M, const Cells& c, int r, float a, int h) {
-  return over(a, pz(M, c, r, h ? KH : K_), pz(M, c, r, h ? RKH : RK));
+  return over<false>(a, pz(M, c, r, h ? KH : K_), pz(M, c, r, h ? RKH : RK));
 }
 __device__ __forceinline__ float over_x(const March& M, const Cells& c, float a, int h) {
-  return over(a, px(M, c, h ? KH : K_), px(M, c, h ? RKH : RK));
+  return over<false>(a, px(M, c, h ? KH : K_), px(M, c, h ? RKH : RK));
 }
 // Differences at the cells. Only where one of them is in the stencil domain:
 // the pair's samples then lie in the array (two columns follow the domain's last).
@@ -649,12 +649,13 @@ __device__ __forceinline__ March set_up(const ShotSlot& S, const Strip& s, float
   unsigned* info = reinterpret_cast<unsigned*>(sm + (kProfiles * (M.nz + M.w) + 1) / 2 * 2);  // (8-byte aligned)
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
-    for (int i = threadIdx.x; i < M.nz; i += blockDim.x) sm[q * M.nz + i] = gz[q][i];
-    for (int i = threadIdx.x; i < M.w; i += blockDim.x) sx[q * M.w + i] = gx[q][s.xa + i];
+    const float scale = q % 3 == 0 ? kQuotientScale : 1.0f;
+    for (int i = threadIdx.x; i < M.nz; i += blockDim.x) sm[q * M.nz + i] = gz[q][i] * scale;
+    for (int i = threadIdx.x; i < M.w; i += blockDim.x) sx[q * M.w + i] = gx[q][s.xa + i] * scale;
   }
   for (int h = 0; h < 2; ++h) {
-    for (int i = threadIdx.x; i < M.nz; i += blockDim.x) sm[(RK + h) * M.nz + i] = 1.0f / gz[3 * h][i];
-    for (int i = threadIdx.x; i < M.w; i += blockDim.x) sx[(RK + h) * M.w + i] = 1.0f / gx[3 * h][s.xa + i];
+    for (int i = threadIdx.x; i < M.nz; i += blockDim.x) sm[(RK + h) * M.nz + i] = 1.0f / gz[3 * h][i] / kQuotientScale;
+    for (int i = threadIdx.x; i < M.w; i += blockDim.x) sx[(RK + h) * M.w + i] = 1.0f / gx[3 * h][s.xa + i] / kQuotientScale;
   }
   for (int i = threadIdx.x; i < M.w * M.depth; i += blockDim.x)
     info[i] = cell_info(S, i % M.depth, s.xa + i / M.depth);

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "fwigb_kernels.h"
+#include "quotient.h"
 
 namespace fwigb {
 
@@ -56,19 +57,6 @@ __device__ __forceinline__ void ring_save(const Geo& g, const StoreD& st, int it
   p[2 * g.ring_len] = sxx;
   p[3 * g.ring_len] = vz;
   p[4 * g.ring_len] = vx;
-}
-
-// a / K of the CPML formulas with r = 1 / K rounded: the quotient estimate a r
-// corrected by its residual, correctly rounded by Markstein's theorem (IBM J.
-// Res. Dev. 34, 1990) as the division is, without its range checks (K is in
-// [1, 2]; a / 1 is exact). The division's path for numerators near the smallest
-// floats is taken all the time in an absorbing layer, where the fields die out:
-// with it a gradient's sweeps on 608 x 1600 (500 steps) took 21.7 ms, so 18.8;
-// 16 shots of 352 x 832 (200 steps) 42.0, so 37.9; 608-row windows of 24 shots
-// 104.7, so 99.2; four shots of 1120 x 3152 (60 steps) 32.4, so 31.2.
-__device__ __forceinline__ float over(float a, float K, float r) {
-  const float q = a * r;
-  return fmaf(fmaf(-K, q, a), r, q);
 }
 
 __device__ __forceinline__ bool in_box(int z, int x, int z0, int z1, int x0, int x1) {
