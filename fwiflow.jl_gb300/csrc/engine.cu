@@ -475,6 +475,7 @@ struct fwigb_ctx {
   MarchPack march{};
   DevBuf march_flags;
   int last_groups = 0;
+  bool sums_in_stage = false;  // a group's imaging sums va and vb are in `stage` (plan_groups)
   // CUDA graph of a single-group call's whole launch sequence, replayed while
   // everything it was captured from is unchanged (graph_key).
   bool use_graphs = true;
@@ -1071,8 +1072,14 @@ int plan_groups(fwigb_ctx* ctx, bool adj, std::vector<std::vector<int>>& groups)
   int cap = static_cast<int>(std::min<size_t>(budget / std::max<size_t>(per_member, 1), 1u << 16));
   if (ctx->max_batch > 0) cap = std::min(cap, ctx->max_batch);
   cap = std::min(cap, static_cast<int>(ctx->plans.size()));
-  // A budget that holds one shot but for two of its five imaging sums is taken as one shot's.
-  if (cap < 1 && budget + 2 * ldz * nx_max * sizeof(float) >= per_member) cap = 1;
+  // A budget that holds one shot but for two of its imaging sums: these go to the
+  // staging buffer, which no run needs otherwise.
+  const size_t two = 2 * ldz * nx_max * sizeof(float);
+  ctx->sums_in_stage = cap < 1 && budget >= per_member - two && ctx->stage.bytes >= two;
+  if (ctx->sums_in_stage) {
+    cap = 1;
+    ctx->grads_stride -= 2 * ldz * nx_max;
+  }
   if (cap < 1) {
     ctx->err = "one shot's wavefields and boundary store do not fit in device memory";
     return FWIGB_ERR_OOM;
@@ -1137,12 +1144,14 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // 12-20 cells: 16k 9.2 / 16.1, 129k (16 shots) 14.7 / 22.9, 137k 16.7 / 19.3,
 // 170k (one) 16.2 / 16.7, 206k 20.7 / 20.3, 274k 24.1 / 22.6, 343k (five) 27.0
 // / 28.1, 380k (three) 29.1 / 26.6.
-// Fixed tile shapes and per-sweep timing ask for the sweeps themselves.
+// Fixed tile shapes and per-sweep timing ask for the sweeps themselves; marching
+// kernels take a shot's sums from one base.
 constexpr size_t kMarchCells = 150000;
 bool marches(const fwigb_ctx* ctx) {
   size_t cells = 0;
   for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
-  return ctx->autotune && !ctx->timing && ctx->plans.size() <= kPackShots && cells <= kMarchCells;
+  return ctx->autotune && !ctx->timing && !ctx->sums_in_stage && ctx->plans.size() <= kPackShots &&
+         cells <= kMarchCells;
 }
 
 // Arrays of this many bytes need 64-bit offsets in the sweeps.
@@ -1236,7 +1245,9 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
     sh.gstf = ctx->shot_gstf.as<float>(pl.gstf_off);
     sl.st = StoreD{ctx->store_stride ? ctx->g_store.as<float>(k * ctx->store_stride) : nullptr};
     float* gb = ctx->g_grads.as<float>(k * ctx->grads_stride);
-    sl.gr = Grads{gb, gb + n, gb + 2 * n, gb + 3 * n, gb + 4 * n, ctx->illum ? gb + 5 * n : nullptr};
+    float* vab = ctx->sums_in_stage ? ctx->stage.as<float>() : gb + 3 * n;
+    sl.gr = Grads{gb, gb + n, gb + 2 * n, vab, vab + n,
+                  ctx->illum ? gb + (ctx->sums_in_stage ? 3 : 5) * n : nullptr};
     sl.nSteps = pl.nSteps;
     sl.x_off = pl.x_off;
     for (int t = 0; t < 3; ++t) {
@@ -1515,6 +1526,10 @@ int run(fwigb_ctx* ctx, int calc_id) {
       }
       if (adj || ctx->illum)
         CK(cudaMemsetAsync(ctx->g_grads.p, 0, static_cast<size_t>(G) * ctx->grads_stride * sizeof(float), s));
+      if (adj && ctx->sums_in_stage) {
+        const size_t n = static_cast<size_t>(ctx->geo.ldz) * ctx->plans[mem[0]].nx;
+        CK(cudaMemsetAsync(ctx->stage.p, 0, 2 * n * sizeof(float), s));
+      }
       const int ntop = nst[0];
       unsigned* done = ctx->march_flags.as<unsigned>();
       const size_t flag_bytes = ctx->marching ? march_flag_bytes(ctx->march) : 0;

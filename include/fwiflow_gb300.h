@@ -154,8 +154,11 @@ long long fwigb_last_launch_count(const fwigb_ctx *ctx);
 
 /* Concurrent shots. The shots of a call run in groups, all members of a group
  * in the same launches (one per sweep and time step). A group holds at most
- * max_shots shots (0: no cap) and its state (wavefields, gradients, boundary
- * stores) at most mem_budget_bytes (0: 90% of the free device memory). Shots
+ * max_shots shots (0: no cap) and its state at most mem_budget_bytes (0: 90% of
+ * the free device memory): per shot 18 wavefields and 5 imaging sums (one array
+ * more with the illumination) on the widest sub-grid, and with gradients the
+ * boundary store of the longest record. A budget that holds one shot but for two
+ * of its sums still runs shot by shot. Shots
  * may carry their own record length ("nSteps") and aperture window
  * ("win_x0", "win_x1", interior columns) as extra keys of the survey file;
  * the reference's parser ignores those keys. */
