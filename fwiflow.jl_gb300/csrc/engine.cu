@@ -464,6 +464,9 @@ struct fwigb_ctx {
   // members), index (variant * 3 + tile slot) * npacks + pack. pack_nx[q] is
   // the widest member sub-grid of pack q.
   int group_size = 0, npacks = 0;
+  // The packs are those of a run that succeeded, and the buffers that they point
+  // into have not changed since.
+  bool packs_live = false;
   std::vector<SweepPack<1>> pack1;
   std::vector<SweepPack<kPackShots>> packs;
   std::vector<int> pack_nx;
@@ -813,6 +816,7 @@ int stage_shots(fwigb_ctx* ctx, const double* stf, int n_stf_rows, const int* sh
     return FWIGB_ERR_ARG;
   }
   CK(cudaSetDevice(ctx->device));
+  ctx->packs_live = false;
   const int nt_max = p.nSteps, nrm = ctx->nrec_max;
   ctx->plans.clear();
   size_t n_src = 0, n_rec = 0, n_blk = 0, n_data = 0, n_taper = 0, n_gstf = 0, n_cpmlx = 0, n_supd = 0;
@@ -1465,7 +1469,7 @@ int run(fwigb_ctx* ctx, int calc_id) {
   }
   CK(cudaSetDevice(ctx->device));
   clear_stale_error();
-  ctx->vp_grad = false;
+  ctx->vp_grad = ctx->packs_live = false;
   std::vector<std::vector<int>> groups;
   TRY_RC(plan_groups(ctx, adj, groups));
   cudaStream_t s = ctx->stream;
@@ -1730,6 +1734,7 @@ int run(fwigb_ctx* ctx, int calc_id) {
   }
 #undef TIMED
   CK(cudaGetLastError());
+  ctx->packs_live = true;
   ctx->launches = launches;
   ctx->last_calc = calc_id;
   ctx->vp_grad = adj && ctx->vp_model;
@@ -2004,11 +2009,11 @@ int fwigb_tile_config(const fwigb_ctx* ctx, int* tile_x) {
 int fwigb_sweep_time(fwigb_ctx* ctx, int kind, int reps, double* us_per_launch) {
   if (!ctx || !us_per_launch || kind < 0 || kind > 3 || reps < 1) return FWIGB_ERR_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
-  if (ctx->group_size < 1) {
-    ctx->err = "no group has run yet";
+  if (!ctx->packs_live) {
+    ctx->err = "no run has succeeded since the shots were staged";
     return FWIGB_ERR_ARG;
   }
-  if (kind >= 2 && ctx->store_stride == 0) {  // (no boundary ring to restore)
+  if (kind >= 2 && (ctx->store_stride == 0 || ctx->nSteps_max < 2)) {  // (no boundary ring to restore)
     ctx->err = "the last run had no backward sweeps";
     return FWIGB_ERR_ARG;
   }

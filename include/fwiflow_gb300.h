@@ -216,7 +216,9 @@ int fwigb_set_graphs(fwigb_ctx *ctx, int enable);
  * velocity, 2 backward B, 3 backward C) over the last run's (last) group, at
  * its tuned tile: `reps` back-to-back launches recorded in a CUDA graph and
  * timed with events around the graph (no per-launch event overhead). The
- * launches work on the live wavefields, which the next run resets. */
+ * launches work on the live wavefields, which the next run resets.
+ * FWIGB_ERR_ARG unless a run has succeeded since the shots were staged (for B
+ * and C one with gradients, of at least two steps). */
 int fwigb_sweep_time(fwigb_ctx *ctx, int kind, int reps, double *us_per_launch);
 
 /* Per-kernel timing of fwigb_run: when enabled, a CUDA event pair on the
