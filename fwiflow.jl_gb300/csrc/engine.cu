@@ -1769,7 +1769,7 @@ int check_waits(fwigb_ctx* ctx) {
   if (!e) return FWIGB_OK;
   CK(cudaMemsetAsync(ctx->scal.as<char>() + 16, 0, sizeof(unsigned), ctx->stream));
   ctx->vp_grad = false;
-  ctx->err = "a sweep gave up waiting for its staged tiles (bounded wait); results are invalid";
+  ctx->err = "a sweep gave up a bounded wait (for its staged tiles, or for a neighbouring strip); results are invalid";
   return FWIGB_ERR_TIMEOUT;
 }
 

@@ -49,9 +49,13 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
-// Waits until a neighbour's flag reaches `count`: bounded by kWaitLimitNs, and
-// given up as soon as another block has raised the error word.
-__device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned count, unsigned* err) {
+// The limit of the timeout test hook's wait (k_march_fwd).
+constexpr unsigned long long kInjectWaitNs = 20000000ull;
+
+// Waits until a neighbour's flag reaches `count`: at most `limit`, and given up
+// as soon as another block has raised the error word.
+__device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned count, unsigned* err,
+                                          unsigned long long limit = kWaitLimitNs) {
   unsigned long long t0 = 0;
   for (unsigned n = 0;; ++n) {
     if (ld_acquire(flag) >= count) return true;
@@ -59,7 +63,7 @@ __device__ __forceinline__ bool wait_flag(const unsigned* flag, unsigned count, 
       if (ld_relaxed(err) != 0) return false;
       const unsigned long long t = global_timer_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kWaitLimitNs) {
+      if (t - t0 > limit) {
         atomicOr(err, 1u);
         return false;
       }
@@ -666,8 +670,9 @@ __device__ __forceinline__ March set_up(const ShotSlot& S, const Strip& s, float
 }
 
 // One forward pass of every shot of the pack over its own record. flags: bit 0
-// saves the boundary ring, bit 1 is the timeout test hook (the first block
-// gives up its first wait and raises err; the others follow). B: blocks per SM.
+// saves the boundary ring, bit 1 is the timeout test hook (the first block ends
+// its first sweep with a wait for a count that nothing publishes, which runs out
+// after kInjectWaitNs and raises err; the others follow). B: blocks per SM.
 template <int B>
 __global__ void __launch_bounds__(kMarchThreads, B)
     k_march_fwd(const __grid_constant__ MarchPack P, int flags, unsigned* done, unsigned* err) {
@@ -686,7 +691,7 @@ __global__ void __launch_bounds__(kMarchThreads, B)
         f1_shear(M, it, flags & 1, z0, x);
     });
     if ((flags & 2) && it == 0 && blockIdx.x == 0) {
-      if (threadIdx.x == 0) atomicOr(err, 1u);
+      if (threadIdx.x == 0) wait_flag(s.flag, ~0u, err, kInjectWaitNs);
       return;
     }
     if (!strip_sync(s, 2 * it + 1, err)) return;

@@ -178,10 +178,11 @@ int fwigb_fetch_illumination(fwigb_ctx *ctx, double *illum);
 
 /* Test hook of the failure path (no counterpart in the reference, which has
  * no bounded waits): with enable != 0, the first forward sweep of every
- * following run waits, once its staged tiles have landed, for a barrier
- * phase that nothing completes; its bounded wait runs out, the run returns
- * FWIGB_ERR_TIMEOUT, and the context stays usable. No copy is in flight when
- * the wait gives up. Off by default. */
+ * following run ends in a wait that nothing completes: for a barrier phase, once
+ * its staged tiles have landed, or in a call that marches (one launch per pass)
+ * the first strip's for a count that no strip reaches. The bounded wait runs out,
+ * the run's results are refused with FWIGB_ERR_TIMEOUT, and the context stays
+ * usable. No copy is in flight when the wait gives up. Off by default. */
 int fwigb_test_inject_wait_timeout(fwigb_ctx *ctx, int enable);
 
 /* Tile widths (columns per thread block: 4, 8 or 16) of the four sweeps
