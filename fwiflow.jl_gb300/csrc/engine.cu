@@ -1761,14 +1761,14 @@ int kernel_times(fwigb_ctx* ctx, double* total_ms, long long* counts) {
 }
 
 // Whether every bounded wait of the runs since the last check ended. After one
-// that ran out the results are invalid, the Vp gradient's among them.
+// that ran out the results are invalid, the Vp gradient and the illumination too.
 int check_waits(fwigb_ctx* ctx) {
   unsigned e = 0;
   CK(cudaMemcpyAsync(&e, ctx->scal.as<char>() + 16, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (!e) return FWIGB_OK;
   CK(cudaMemsetAsync(ctx->scal.as<char>() + 16, 0, sizeof(unsigned), ctx->stream));
-  ctx->vp_grad = false;
+  ctx->vp_grad = ctx->illum_valid = false;
   ctx->err = "a sweep gave up a bounded wait (for its staged tiles, or for a neighbouring strip); results are invalid";
   return FWIGB_ERR_TIMEOUT;
 }
@@ -2146,6 +2146,7 @@ int fwigb_fetch_illumination(fwigb_ctx* ctx, double* illum) {
     ctx->err = "the last run did not accumulate the illumination (fwigb_set_illumination)";
     return FWIGB_ERR_ARG;
   }
+  if (const int rc = check_waits(ctx); rc != FWIGB_OK) return rc;
   cudaStream_t s = ctx->stream;
   double* st = ctx->stage.as<double>();
   launch_to_rowmajor(s, ctx->p.nz, ctx->p.nx, ctx->geo.ldz, ctx->grads.as<float>(3 * ctx->cells), st, 1.0);
