@@ -72,6 +72,7 @@ SIGNATURES = {
     "fwigb_misfit_gathers_noalloc": ([_V, _V, _V, ctypes.c_int, ctypes.c_int, ctypes.c_float, _D, _V], ctypes.c_int),
     "fwigb_noalloc_last_error": ([], ctypes.c_char_p),
     "fwigb_test_inject_wait_timeout": ([_V, ctypes.c_int], ctypes.c_int),
+    "fwigb_test_wide_offsets": ([_V, ctypes.c_int], ctypes.c_int),
     "fwigb_fetch_illumination": ([_V, _D], ctypes.c_int),
     "fwigb_cnn_conv3x3": ([_V, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _V, _V, _V, _V,
                            _V, _V, _V], ctypes.c_int),

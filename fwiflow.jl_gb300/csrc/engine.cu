@@ -478,6 +478,9 @@ struct fwigb_ctx {
   MarchPack march{};
   DevBuf march_flags;
   int last_groups = 0;
+  // Arrays of this many bytes need 64-bit offsets in the sweeps (0, of the test hook: all do).
+  static constexpr size_t kWideBytes = size_t{1} << 32;
+  size_t wide_bytes = kWideBytes;
   bool sums_in_stage = false;  // a group's imaging sums va and vb are in `stage` (plan_groups)
   // CUDA graph of a single-group call's whole launch sequence, replayed while
   // everything it was captured from is unchanged (graph_key).
@@ -1111,7 +1114,7 @@ int plan_groups(fwigb_ctx* ctx, bool adj, std::vector<std::vector<int>>& groups)
 // Returns the number of launches.
 int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int flags, unsigned* d_err) {
   cudaStream_t s = ctx->stream;
-  if (ctx->pack_grid[0].wide) {
+  if (ctx->pack_grid[0].wide && w != 2) {  // (B has 64-bit offsets in every shape)
     tx = kWideTx;
     rows = 1;
   }
@@ -1149,17 +1152,14 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // 170k (one) 16.2 / 16.7, 206k 20.7 / 20.3, 274k 24.1 / 22.6, 343k (five) 27.0
 // / 28.1, 380k (three) 29.1 / 26.6.
 // Fixed tile shapes and per-sweep timing ask for the sweeps themselves; marching
-// kernels take a shot's sums from one base.
+// kernels take a shot's sums from one base, and have no 64-bit offsets.
 constexpr size_t kMarchCells = 150000;
 bool marches(const fwigb_ctx* ctx) {
   size_t cells = 0;
   for (const ShotPlan& pl : ctx->plans) cells += static_cast<size_t>(ctx->p.nz) * pl.nx;
-  return ctx->autotune && !ctx->timing && !ctx->sums_in_stage && ctx->plans.size() <= kPackShots &&
-         cells <= kMarchCells;
+  return ctx->autotune && !ctx->timing && !ctx->sums_in_stage && ctx->wide_bytes > 0 &&
+         ctx->plans.size() <= kPackShots && cells <= kMarchCells;
 }
-
-// Arrays of this many bytes need 64-bit offsets in the sweeps.
-constexpr size_t kWideBytes = size_t{1} << 32;
 
 // Order of the sweeps' blocks (TileSplit::order).
 // kBackF2, kBackC: where the fields that a sweep shares with the one before it
@@ -1288,7 +1288,7 @@ int build_group(fwigb_ctx* ctx, const std::vector<int>& members, int& nx_max) {
     gr.zoff = zoff;
     gr.order = order;
     for (const ShotSlot& sl : slots)
-      gr.wide |= static_cast<size_t>(sl.g.ldz) * sl.g.nx * sizeof(float) >= kWideBytes;
+      gr.wide |= static_cast<size_t>(sl.g.ldz) * sl.g.nx * sizeof(float) >= ctx->wide_bytes;
   }
   auto split = [&](int w, int k) {
     const bool wide = w / 3 >= 4;
@@ -1346,6 +1346,12 @@ int autotune(fwigb_ctx* ctx, int nshots, int nx_max, bool adj) {
   for (int kind = ctx->tuned_fwd ? 2 : 0; kind < kinds_end; ++kind) {
     // (width, rows) candidates; the backward sweeps add one-row tiles at 40
     // registers (ctx->regs, read by launch_sweep, is set per candidate).
+    if (ctx->pack_grid[0].wide && kind != 2) {  // (one shape: launch_sweep)
+      ctx->tx[kind] = kWideTx;
+      ctx->rows[kind] = 1;
+      ctx->regs[kind] = 32;
+      continue;
+    }
     const int ncand = kind >= 2 ? 9 : 6;
     auto cand = [&](int q, int& tx, int& rows) {
       tx = kTileXs[q % 3];
@@ -1702,7 +1708,10 @@ int run(fwigb_ctx* ctx, int calc_id) {
         add_words(ctx->pack1.data(), ctx->pack1.size() * sizeof(SweepPack<1>));
       else
         add_words(ctx->packs.data(), ctx->packs.size() * sizeof(SweepPack<kPackShots>));
-      for (const SweepGrid& gr : ctx->pack_grid) key.push_back((static_cast<uint64_t>(gr.nz) << 32) | gr.nx);
+      for (const SweepGrid& gr : ctx->pack_grid) {
+        key.push_back((static_cast<uint64_t>(gr.nz) << 32) | gr.nx);
+        key.push_back(gr.wide);
+      }
       if (!ctx->graph_exec || key != ctx->graph_key) {
         if (ctx->graph_exec) {
           cudaGraphExecDestroy(ctx->graph_exec);
@@ -2129,6 +2138,13 @@ int fwigb_test_inject_wait_timeout(fwigb_ctx* ctx, int enable) {
   if (!ctx) return FWIGB_ERR_ARG;
   std::lock_guard<std::mutex> lk(ctx->mu);
   ctx->inject_timeout = enable != 0;
+  return FWIGB_OK;
+}
+
+int fwigb_test_wide_offsets(fwigb_ctx* ctx, int enable) {
+  if (!ctx) return FWIGB_ERR_ARG;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  ctx->wide_bytes = enable ? 0 : fwigb_ctx::kWideBytes;
   return FWIGB_OK;
 }
 

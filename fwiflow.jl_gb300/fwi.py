@@ -212,6 +212,10 @@ class FwiContext:
         status ERR_TIMEOUT; the context stays usable."""
         _lib.check(self._lib.fwigb_test_inject_wait_timeout(self._h, int(enable)), self._h)
 
+    def test_wide_offsets(self, enable: bool) -> None:
+        """Test hook: the sweeps' form for arrays of 4 GB and more at any size."""
+        _lib.check(self._lib.fwigb_test_wide_offsets(self._h, int(enable)), self._h)
+
     def set_illumination(self, enable: bool = True) -> None:
         """Accumulate the source illumination sum_t (vz^2 + vx^2) in the
         following runs (all their shots)."""

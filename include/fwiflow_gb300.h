@@ -185,6 +185,11 @@ int fwigb_fetch_illumination(fwigb_ctx *ctx, double *illum);
  * usable. No copy is in flight when the wait gives up. Off by default. */
 int fwigb_test_inject_wait_timeout(fwigb_ctx *ctx, int enable);
 
+/* Test hook: with enable != 0 the following runs take the form of the sweeps for
+ * arrays of 4 GB and more (64-bit offsets; F1, F2 and C in one-row tiles of 8
+ * columns, whatever tile shape is set) at any size. Off by default. */
+int fwigb_test_wide_offsets(fwigb_ctx *ctx, int enable);
+
 /* Tile widths (columns per thread block: 4, 8 or 16) of the four sweeps
  * (forward stress, forward velocity, backward B, backward C). By default an
  * autotuner times every width and 1 or 2 depths per thread on the context's
