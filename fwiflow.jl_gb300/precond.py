@@ -160,22 +160,25 @@ class CnnPreconditioner:
         if rc != 0:
             raise _lib.FwiError(rc, "CNN kernel launch failed")
 
+    def _plain(self, a, channels=()) -> bool:
+        """Whether `a` is an array of real numbers of the model's shape, which the image kernels take."""
+        return isinstance(a, np.ndarray) and a.shape == (*channels, self.Hz, self.Wx) and a.dtype.kind in "fiub" \
+            and a.dtype.itemsize <= 8
+
     def _upload(self, *arrays):
         """Model-shaped arrays as one device tensor (len(arrays), Hz, Wx) of doubles."""
         torch = _torch()
         out = torch.empty((len(arrays), self.Hz, self.Wx), dtype=torch.float64, device=self.dev)
         for k, a in enumerate(arrays):
             a = np.ascontiguousarray(a, dtype=np.float64)
-            if a.shape != (self.Hz, self.Wx) or not a.flags.writeable:  # (torch warns of read-only arrays)
-                a = np.array(np.broadcast_to(a, (self.Hz, self.Wx)))
+            if not a.flags.writeable:  # (torch warns of read-only arrays)
+                a = a.copy()
             out[k].copy_(torch.from_numpy(a))
         return out
 
     def _pack(self, chans, c_pad: int, out) -> None:
         """(C, nz, nx) arrays into the image tensor `out` (FP32 or BF16)."""
         torch = _torch()
-        if len(chans) > c_pad:
-            raise ValueError(f"{len(chans)} channels do not fit an image of {c_pad}")
         self._ck(self.lib.fwigb_cnn_pack_image(self._p(self._upload(*chans)), len(chans), self.Hz, self.Wx, c_pad,
                                                int(out.dtype == torch.bfloat16), self._p(out), self._s()))
 
@@ -183,13 +186,19 @@ class CnnPreconditioner:
         """(C, nz, nx) numpy -> device [npix][c_pad] in the kernels' layout."""
         torch = _torch()
         c = chans.shape[0]
-        if dtype in (torch.float32, torch.bfloat16) and 1 <= c <= c_pad <= 16:
+        if dtype in (torch.float32, torch.bfloat16) and 1 <= c <= c_pad <= 16 and self._plain(chans, (c,)):
             out = torch.empty((self.npix, c_pad), dtype=dtype, device=self.dev)
             self._pack(chans, c_pad, out)
             return out
         a = np.zeros((self.Wx, self.Hz, c_pad), dtype=np.float32)
         a[:, :, :c] = np.transpose(chans, (2, 1, 0))
         return torch.from_numpy(a.reshape(self.npix, c_pad)).to(device=self.dev, dtype=dtype)
+
+    def _stage_image(self, chans: np.ndarray, c_pad: int, out) -> None:
+        if 1 <= chans.shape[0] <= c_pad and self._plain(chans, chans.shape[:1]):
+            self._pack(chans, c_pad, out)
+        else:
+            out.copy_(self.to_image(chans, c_pad, out.dtype))
 
     def from_image(self, t, c: int) -> np.ndarray:
         """Device [npix][C] -> (c, nz, nx) float64 numpy."""
@@ -284,11 +293,16 @@ class CnnPreconditioner:
 
     # -- data
     def stage(self, feats: np.ndarray, target: Optional[np.ndarray] = None, mask: Optional[np.ndarray] = None):
-        self._pack(feats, 16, self.x0)
+        self._stage_image(feats, 16, self.x0)
         if target is not None:
-            self._pack(target, N_OUT, self.target)
+            self._stage_image(target, N_OUT, self.target)
         if mask is not None:
-            self._pack([mask], 1, self.mask)
+            if self._plain(mask):
+                self._pack([mask], 1, self.mask)
+            else:
+                torch = _torch()
+                flat = np.ascontiguousarray(mask.T.reshape(-1), dtype=np.float32)
+                self.mask.copy_(torch.from_numpy(flat).to(self.dev))
 
     def train(self, samples: Sequence[tuple], epochs: int, lr: float = 1e-3, seed: int = 0,
               log: Optional[List[float]] = None) -> List[float]:
@@ -327,6 +341,9 @@ class CnnPreconditioner:
         """Preconditioned lambda / mu / rho gradients (3, nz, nx): each
         gradient times exp of its predicted log-gain, zero outside the mask."""
         torch = _torch()
+        if not all(self._plain(v) for v in (g_lambda, g_mu, g_den, illum, mask)):
+            out = self.predict(features(g_lambda, g_mu, g_den, illum, mask))
+            return np.stack([g_lambda, g_mu, g_den]) * np.exp(np.clip(out, -30.0, 5.0)) * mask
         a = self._upload(g_lambda, g_mu, g_den, illum, mask)
         g, (e, m) = [self._p(v) for v in a[:3]], (self._p(v) for v in a[3:])
         scratch = torch.empty(self.lib.fwigb_cnn_feature_scratch(), dtype=torch.float64, device=self.dev)
