@@ -30,6 +30,7 @@ from typing import Callable, List, Optional
 
 import numpy as np
 
+from .fwi import FwiContext
 from .utils import velocity_to_moduli
 
 
@@ -96,8 +97,12 @@ class VpProblem:
         return float(np.linalg.norm(v[m] - self.vp_true[m]) / np.linalg.norm(self.vp_true[m]))
 
     def _set_model(self, vp) -> bool:
-        """The model moduli_of_vp(self.full(vp)); formed on the device (True) when the limits are numbers."""
-        on_device = np.isscalar(self.vmin) and np.isscalar(self.vmax)
+        """The model moduli_of_vp(self.full(vp)); formed on the device (True) when the limits are ordered numbers, and
+        neither `full` nor the context's models and gradients are somebody's own."""
+        ctx = type(self.ctx)
+        plain = type(self).full is VpProblem.full and all(
+            getattr(ctx, name, None) is getattr(FwiContext, name) for name in ("set_model", "run", "fetch"))
+        on_device = plain and np.isscalar(self.vmin) and np.isscalar(self.vmax) and bool(self.vmin <= self.vmax)
         if on_device:
             self.ctx.set_model_vp(vp, self.vp0, self.mask, self.vmin, self.vmax)
         else:
