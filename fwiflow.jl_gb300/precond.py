@@ -133,7 +133,7 @@ class CnnPreconditioner:
         self.out = torch.zeros((self.npix, 16), **f32)
         self.dz = [torch.zeros((self.npix, cop), **bf) for (_, _, _, cop) in self.LAYERS]
         self.ntiles = int(self.lib.fwigb_cnn_tile_count(Hz, Wx))
-        self.part = torch.zeros(self.ntiles * 9 * 32 * 32, **f32)
+        self.part = torch.zeros(int(self.lib.fwigb_cnn_wgrad_blocks(Hz, Wx)) * 9 * 32 * 32, **f32)
         self.chunk = 1024
         self.bpart = torch.zeros(((self.npix + self.chunk - 1) // self.chunk) * 32, **f32)
         self.lpart = torch.zeros((self.npix + 255) // 256, **f32)
