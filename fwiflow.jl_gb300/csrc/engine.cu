@@ -1150,7 +1150,10 @@ int launch_sweep(fwigb_ctx* ctx, int w, int tx, int rows, int a, int arg, int fl
 // 17.5 / 16.7, 287k (four) 22.1 / 18.5, 293k (one) 21.4 / 17.8; with one of
 // 12-20 cells: 16k 9.2 / 16.1, 129k (16 shots) 14.7 / 22.9, 137k 16.7 / 19.3,
 // 170k (one) 16.2 / 16.7, 206k 20.7 / 20.3, 274k 24.1 / 22.6, 343k (five) 27.0
-// / 28.1, 380k (three) 29.1 / 26.6.
+// / 28.1, 380k (three) 29.1 / 26.6. (The rule counts cells alone. Grids whose
+// strips are many rounds of a block's warps lose within it: four of 928 x 40 24.2 /
+// 18.8, one of 96 x 1520 20.2 / 17.9, of 736 x 200 19.2 / 16.9; four of 448 x 80
+// 18.2 / 19.0.)
 // Fixed tile shapes and per-sweep timing ask for the sweeps themselves; marching
 // kernels take a shot's sums from one base, and have no 64-bit offsets.
 constexpr size_t kMarchCells = 150000;

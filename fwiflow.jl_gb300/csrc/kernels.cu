@@ -168,13 +168,15 @@ __device__ __forceinline__ bool outer_tile(const ShotSlot& S, int z0, int x0, in
 // it holds the shot's source or a receiver.
 //
 // Work split. Block (32, TX): lane threadIdx.x covers R adjacent depths
-// (R = TZ / 32), threadIdx.y the column. The sweeps issue more integer than
-// floating-point instructions (F1: 27 FP32 and 57 integer of 164 per cell), so
-// the tile split comes with the parameters, and a thread's addresses are
-// pointers plus a byte offset in 32 bits (SWEEP_ADDRESS): with the shifted
-// 64-row tiles, a gradient's sweeps on 608 x 1600 (500 steps) 24.4 -> 23.1 ms,
-// two shots of 352 x 832 (400 steps) 15.9 -> 15.1 ms, four of 1120 x 3152 (60
-// steps) 35.4 -> 34.5 ms, 16 of 352 x 832 unchanged.
+// (R = TZ / 32), threadIdx.y the column. Index arithmetic takes about as many
+// instructions as the floating-point work (a cell of F1 on one 1120 x 3152 shot:
+// 26 integer and 29 FP32 of 148; 57 and 27 of 164 when a block worked its tile
+// split out and every address was 64 bits wide), so the tile split comes with the
+// parameters, and a thread's addresses are pointers plus a byte offset in 32 bits
+// (SWEEP_ADDRESS). The split and the shifted 64-row tiles together: a gradient's
+// sweeps on 608 x 1600 (500 steps) 24.4 -> 23.1 ms, two shots of 352 x 832 (400
+// steps) 15.9 -> 15.1 ms, four of 1120 x 3152 (60 steps) 35.4 -> 34.5 ms, 16 of
+// 352 x 832 unchanged.
 //
 // Programmatic dependent launch: a sweep lets the next sweep's blocks be
 // scheduled as soon as all of its own blocks have started, and waits
@@ -450,8 +452,7 @@ __device__ __forceinline__ void cpml_fwd(const float4& q, float& mm, float& d) {
 // 38.2, F2 32.0 / 29.0; 608-row windows of 24 shots F1 116.3 / 111.0, F2 102.9
 // / 94.8; one 608 x 1600 shot F1 8.7 / 8.4, F2 7.6 / 7.1; four 1120 x 3152
 // shots F1 96.9 / 97.1, F2 80.7 / 78.1. (F2 with registers: 30.0, 97.6, 7.4,
-// 78.4. With the quotients of over(), the block order and the offsets of
-// SWEEP_ADDRESS they now take 30.8 and 24.5, 101 and 85, 6.8 and 5.7, 83 and 68.)
+// 78.4.)
 template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
@@ -718,7 +719,7 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
   const bool zp = (z < g.nPml) || (z > g.zpml_hi);
   const bool xp = (x < g.nPml) || (x > g.xpml_hi_s);
   {
-    const float4 cx = __ldg(c.q_x + x), czh = __ldg(c.q_zh + z);  // {K, a, b, 1 / K}
+    const float4 cx = __ldg(c.q_x + x), czh = __ldg(c.q_zh + z);  // {K, a, b, 1 / K}, scaled for over()
     const float dszz_dx = -sdp(s_szz_a, b, BOXZ, g.rdx);
     const float dsxx_dx = -sdp(s_sxx_a, b, BOXZ, g.rdx);
     const float dsxz_dz = -sdm(s_sxz_a, b, 1, g.rdz);
@@ -767,8 +768,7 @@ __device__ __forceinline__ void bwd_B_edge(const SweepPack<K>& P, int shot, int 
 // registers for. us a sweep, edge body / this: 16 shots of 352 x 832 B 68.8 /
 // 66.1, C 71.5 / 67.9; 608-row windows of 24 shots B 224.1 / 220.2, C 226.1 /
 // 219.7; one 608 x 1600 shot B 13.5 / 13.1, C 13.8 / 12.6; four 1120 x 3152
-// shots B 202.4 / 203.8, C 185.9 / 183.9. (Now 63.0 and 65.7, 207 and 204, 11.3
-// and 11.1, 187 and 174.)
+// shots B 202.4 / 203.8, C 185.9 / 183.9.
 template <int TX, int K, int R>
 __device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int z0, int x0, int j, unsigned* err) {
   constexpr int BOXZ = 32 * R + 8;
@@ -831,7 +831,7 @@ __device__ __forceinline__ void bwd_B_outer(const SweepPack<K>& P, int shot, int
 #pragma unroll
       for (int r = 0; r < R; ++r) q1[r] = dom[r] ? gdp(f.m_dvx_dx, i + r, ldz, g.rdx) : 0.0f;
     }
-    const float4 cx = __ldg(c.q_x + x);  // {K, a, b, 1 / K}
+    const float4 cx = __ldg(c.q_x + x);  // {K, a, b, 1 / K}, scaled for over()
     const float bxh = xc ? __ldg(c.b_xh + x) : 0.0f;
 #pragma unroll
     for (int r = 0; r < R; ++r)

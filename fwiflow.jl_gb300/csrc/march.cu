@@ -12,21 +12,22 @@
 // orders their writes before its reads, and their reads before its writes).
 // All blocks of a launch are resident together (a cooperative launch). The
 // hand-over costs 1.1 us of a sweep, the sweep itself 1-1.5 us at the smallest
-// sizes: a step of two 96 x 84 grids takes 9.2 us (16.1 with a launch per sweep),
-// of two 192 x 264 grids 13.4 us (18.0), of one 224 x 448 grid 11.9 us (13.7).
+// sizes; marches() in engine.cu has the times against a launch per sweep.
 //
 // A warp takes 64 depths of one column at a time, two adjacent ones a thread,
 // and reads its stencil samples from the fields themselves (L1 / L2): at these
 // sizes the fields live in L2, and staging would add its own latency. Where a
 // block's work takes several rounds of its warps it is bound by the instructions
 // of its loads and their addresses (about 150 loads a cell of a step), which
-// paired loads halve: one depth a thread took 20.1 us a step for two 224 x 448
-// grids (now 17.8) and 25.6 us for one 352 x 832 (now 21.2).
+// paired loads halve.
 // With several rounds the forward pass runs two blocks of 512 threads on each
-// SM, so that one works while the other waits for its neighbours (352 x 832:
-// 3.6 us for F1 and F2; 4.2 with one block). The backward pass has more operands in flight: one block with
-// 128 registers a thread (two 352 x 832 grids: 11.3 us; 13.1 with two blocks of
-// 64 registers, 12.6 with one of 640 threads).
+// SM, so that one works while the other waits for its neighbours. us a step, two
+// blocks / one: two 192 x 264 grids 4.96 / 6.03, three 160 x 190 4.99 / 6.08, one
+// 224 x 448 4.88 / 5.65, sixteen 96 x 88 7.69 / 8.77; but one 320 x 324 6.52 /
+// 5.98 and one 352 x 334 6.65 / 5.99. The backward pass has more operands in
+// flight: one block with 128 registers a thread, against two of 64: the same
+// grids 8.82 / 9.42, 8.67 / 10.0, 7.24 / 9.76, 14.3 / 14.8, 8.53 / 9.30 and 8.65 /
+// 10.2, and two 96 x 84 ones 5.48 / 7.05.
 #include <algorithm>
 
 #include "fwigb_kernels.h"
@@ -795,8 +796,9 @@ bool march_plan(MarchPack& p, int sms) {
     const long long media = p.slots[k].m.aveMu - p.slots[k].m.l2m;
     if (g.ring_len >= 1 << 21 || 18ll * g.ldz * g.nx >= 1ll << 31 || 8 * media >= 1ll << 31) return false;
   }
-  // Two blocks per SM in the forward pass, unless one of more registers has a
-  // single round (a sweep of two 96 x 84 grids: 1.02 us; 1.05 with 64 registers).
+  // Two blocks per SM in the forward pass (the figures above), unless one of more
+  // registers has a single round (a sweep of two 96 x 84 grids: 1.02 us; 1.05 with
+  // 64 registers).
   p.fwd_blocks = split_shots(p, sms, 2, p.fwd) == 1 ? 1 : 2;
   return (p.fwd_blocks == 1 || split_shots(p, 2 * sms, 2, p.fwd)) && split_shots(p, sms, 3, p.bwd);
 }
