@@ -416,7 +416,7 @@ struct ShotPlan {
   size_t supd_off = 0;  // floats: source update block (supd_floats), when if_src_update
   std::vector<float> src_amp;  // tapered source wavelet (host; kept for the scratch outputs)
   size_t gstf_off = 0;  // floats: nSteps
-  size_t cpmlx_off = 0; // floats: 6 * nx (CPML x profiles of the sub-grid)
+  size_t cpmlx_off = 0; // floats: cpml_floats(nx) (CPML x profiles of the sub-grid)
   int rbz0 = 0, rbz1 = 0, rbx0 = 0, rbx1 = 0;  // receivers + source bounding box
 };
 

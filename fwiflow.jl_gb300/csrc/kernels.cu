@@ -428,10 +428,11 @@ __device__ __forceinline__ void psi_x(const float* a, const float* d, const bool
   }
 }
 
-// One CPML convolution (el_stress.cu:64-85): the memory value and the derivative.
+// One CPML convolution (el_stress.cu:64-85): the memory value and the derivative. CALL as in over().
+template <bool CALL = true>
 __device__ __forceinline__ void cpml_fwd(const float4& q, float& mm, float& d) {
   mm = q.z * mm + q.y * d;
-  d = over(d, q.x, q.w) + mm;
+  d = over<CALL>(d, q.x, q.w) + mm;
 }
 
 // ---------------------------------------------------------------------------
@@ -452,7 +453,9 @@ __device__ __forceinline__ void cpml_fwd(const float4& q, float& mm, float& d) {
 // 38.2, F2 32.0 / 29.0; 608-row windows of 24 shots F1 116.3 / 111.0, F2 102.9
 // / 94.8; one 608 x 1600 shot F1 8.7 / 8.4, F2 7.6 / 7.1; four 1120 x 3152
 // shots F1 96.9 / 97.1, F2 80.7 / 78.1. (F2 with registers: 30.0, 97.6, 7.4,
-// 78.4.)
+// 78.4.) F2 works the z terms off before it forms the x ones, and has large
+// quotients in place, or it spills: 16 shots of 352 x 832 26.2 us (27.8), eight
+// of 608 x 1600 41.7 (44.4), four of 1120 x 3152 71.2 (75.5).
 template <int TX, int K, int R, bool WIDE>
 __device__ __forceinline__ void fwd_stress_edge(const SweepPack<K>& P, int shot, int z0, int x0, int it, int save,
                                                 bool inject, unsigned* err) {
@@ -586,11 +589,9 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
   const float* s_szz = sm;
   const float* s_sxx = sm + N;
   const float* s_sxz = sm + 2 * N;
-  float dszz_dz[R], dsxz_dx[R], dsxz_dz[R], dsxx_dx[R];
+  float dszz_dz[R], dsxz_dz[R];
   dpz<R>(s_szz, b, g.rdz, dszz_dz);
-  dmx<R, BOXZ>(s_sxz, b, g.rdx, dsxz_dx);
   dmz<R>(s_sxz, b, g.rdz, dsxz_dz);
-  dpx<R, BOXZ>(s_sxx, b, g.rdx, dsxx_dx);
   if (any_z) {
     float m1[R], m2[R];
     own<R>(mem, 0, m1);
@@ -598,12 +599,15 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (zc[r]) {
-        cpml_fwd(__ldg(c.q_zh + z + r), m1[r], dszz_dz[r]);
-        cpml_fwd(__ldg(c.q_z + z + r), m2[r], dsxz_dz[r]);
+        cpml_fwd<false>(__ldg(c.q_zh + z + r), m1[r], dszz_dz[r]);
+        cpml_fwd<false>(__ldg(c.q_z + z + r), m2[r], dsxz_dz[r]);
       }
     sto<R>(f.m_dszz_dz, base, off, m1);
     sto<R>(f.m_dsxz_dz, base, off, m2);
   }
+  float dsxz_dx[R], dsxx_dx[R];
+  dmx<R, BOXZ>(s_sxz, b, g.rdx, dsxz_dx);
+  dpx<R, BOXZ>(s_sxx, b, g.rdx, dsxx_dx);
   if (xc) {
     float m1[R], m2[R];
     own<R>(mem + 2 * M, 0, m1);
@@ -611,8 +615,8 @@ __device__ __forceinline__ void fwd_velocity_edge(const SweepPack<K>& P, int sho
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (dom[r]) {
-        cpml_fwd(__ldg(c.q_x + x), m1[r], dsxz_dx[r]);
-        cpml_fwd(__ldg(c.q_xh + x), m2[r], dsxx_dx[r]);
+        cpml_fwd<false>(__ldg(c.q_x + x), m1[r], dsxz_dx[r]);
+        cpml_fwd<false>(__ldg(c.q_xh + x), m2[r], dsxx_dx[r]);
       }
     sto<R>(f.m_dsxz_dx, base, off, m1);
     sto<R>(f.m_dsxx_dx, base, off, m2);

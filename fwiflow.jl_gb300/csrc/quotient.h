@@ -51,7 +51,7 @@ FWIGB_QUOTIENT_CALL float call_over_large(float a, float K_scaled, float r_scale
 // steps 10.87 / 11.0 (10.84); marching, two 192 x 264 grids, 300 steps 4.15 / 4.06
 // (3.96). (With the division 37.9 became 42.0 ms on 16 such shots, 200 steps: its
 // path for numerators near the smallest floats is taken all the time in an
-// absorbing layer, where the fields die out.)
+// absorbing layer, where the fields die out.) F2 has them in place (fwd_velocity_edge).
 template <bool CALL = true>
 FWIGB_QUOTIENT float over(float a, float K_scaled, float r_scaled) {
   const float b = product(a, kQuotientScale), q = product(b, r_scaled);
